@@ -348,7 +348,7 @@ def exact(case, seed):
     if kind == "single":
         if case["op"] == "syrk":  # column-major upper triangle: row-major lower
             return torch.tril(psi.t() @ psi)
-        return 0.5 * (psi.t() @ _dense(st["b"], case["nn"])) + 0.25
+        return 0.5 * (psi.t() @ _dense(st["b"], case["nn"])) + 1e-3
     out = {"s": torch.tril(psi.t() @ psi), "hs": psi.t() @ _dense(st["hpsi"], nb)}
     if kind == "step":
         rot = psi @ st["q"]
