@@ -331,8 +331,9 @@ int configure(BatchPlan* P, Config c) {
     if ((st = P->d_probs.ensure(hp.size() * sizeof(Fp64Params)))) return st;
     if ((st = P->d_maps.ensure(hm.size() * sizeof(CUtensorMap)))) return st;
     if ((st = P->d_iters.ensure(hb.size() * sizeof(int64_t)))) return st;
-    if ((st = P->d_part.ensure((size_t)grid * BM * BN * sizeof(double)))) return st;
-    if ((st = P->d_flags.ensure((size_t)grid * sizeof(uint32_t)))) return st;
+    const size_t slots = (size_t)fixup_slots(grid, 1);
+    if ((st = P->d_part.ensure(slots * BM * BN * sizeof(double)))) return st;
+    if ((st = P->d_flags.ensure(slots * sizeof(uint32_t)))) return st;
     SKG_CUDA(cudaMemcpy(P->d_probs.ptr, hp.data(), hp.size() * sizeof(Fp64Params),
                         cudaMemcpyHostToDevice));
     SKG_CUDA(cudaMemcpy(P->d_maps.ptr, hm.data(), hm.size() * sizeof(CUtensorMap),
@@ -876,14 +877,15 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
   if (!R) return fail(SKGEMM_ERR_INVALID_ARG, "null group ring");
   int cap128 = 0, cap64 = 0, st;
   if ((st = grid_cap(R->dev, 128, &cap128)) || (st = grid_cap(R->dev, 64, &cap64))) return st;
-  const size_t part = std::max((size_t)cap128 * 128 * 128, (size_t)cap64 * 64 * 64) * 8;
-  const int grid = std::max(cap128, cap64);
+  const size_t part = std::max((size_t)fixup_slots(cap128, 1) * 128 * 128,
+                               (size_t)fixup_slots(cap64, 1) * 64 * 64) * 8;
+  const size_t nflags = (size_t)fixup_slots(std::max(cap128, cap64), 1);
   for (auto& sl : R->slots) {
     if ((st = sl.probs.ensure((size_t)max_problems * sizeof(Fp64Params)))) return st;
     if ((st = sl.maps.ensure((size_t)2 * max_problems * sizeof(CUtensorMap)))) return st;
     if ((st = sl.iters.ensure((size_t)(max_problems + 1) * sizeof(int64_t)))) return st;
     if ((st = sl.part.ensure(part))) return st;
-    if ((st = sl.flags.ensure((size_t)grid * sizeof(uint32_t)))) return st;
+    if ((st = sl.flags.ensure(nflags * sizeof(uint32_t)))) return st;
     if (!sl.err.ptr) {
       if ((st = sl.err.ensure(sizeof(uint32_t)))) return st;
       SKG_CUDA(cudaMemset(sl.err.ptr, 0, sizeof(uint32_t)));

@@ -64,23 +64,26 @@ void DeviceBuffer::release() {
   bytes = 0;
 }
 
-int StreamWorkspace::ensure(int slots) {
-  if ((size_t)slots <= partial_slots && err) return SKGEMM_OK;
+int StreamWorkspace::ensure(size_t slots, size_t nflags) {
+  if (slots <= partial_slots && nflags <= num_flags && err) return SKGEMM_OK;
+  slots = std::max(slots, partial_slots);
+  nflags = std::max(nflags, num_flags);
   if (partials) cudaFree(partials);
   if (flags) cudaFree(flags);
   partials = nullptr;
   flags = nullptr;
-  partial_slots = 0;
-  SKG_CUDA(cudaMalloc(&partials, (size_t)slots * kBM * kBN * sizeof(double)));
+  partial_slots = num_flags = 0;
+  SKG_CUDA(cudaMalloc(&partials, slots * kBM * kBN * sizeof(double)));
   if (debug_fill_enabled())
-    SKG_CUDA(cudaMemset(partials, 0xFF, (size_t)slots * kBM * kBN * sizeof(double)));
-  SKG_CUDA(cudaMalloc(&flags, (size_t)slots * sizeof(uint32_t)));
-  SKG_CUDA(cudaMemset(flags, 0, (size_t)slots * sizeof(uint32_t)));
+    SKG_CUDA(cudaMemset(partials, 0xFF, slots * kBM * kBN * sizeof(double)));
+  SKG_CUDA(cudaMalloc(&flags, nflags * sizeof(uint32_t)));
+  SKG_CUDA(cudaMemset(flags, 0, nflags * sizeof(uint32_t)));
   if (!err) {
     SKG_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
     SKG_CUDA(cudaMemset(err, 0, sizeof(uint32_t)));
   }
   partial_slots = slots;
+  num_flags = nflags;
   epoch = 0;
   return SKGEMM_OK;
 }
@@ -121,11 +124,12 @@ DeviceState* current_device(int* status) {
   return dev;
 }
 
-StreamWorkspace* stream_workspace(DeviceState* dev, cudaStream_t s, int slots, int* status) {
+StreamWorkspace* stream_workspace(DeviceState* dev, cudaStream_t s, size_t slots, int* status,
+                                  size_t nflags) {
   std::lock_guard<std::mutex> lk(dev->mu);
   StreamWorkspace*& ws = dev->ws[s];
   if (!ws) ws = new StreamWorkspace();
-  *status = ws->ensure(slots);
+  *status = ws->ensure(slots, nflags ? nflags : slots);
   if (*status == SKGEMM_OK)
     *status = debug_poison(ws->partials, ws->partial_slots * kBM * kBN * sizeof(double), s);
   return *status == SKGEMM_OK ? ws : nullptr;

@@ -145,9 +145,21 @@ int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
   if ((int64_t)sc.num_tiles * sc.ipt > ((int64_t)1 << 40))
     return fail(SKGEMM_ERR_INVALID_ARG, "problem too large");
 
-  StreamWorkspace* ws = ws_override ? ws_override : stream_workspace(dev, s, sc.grid, &st);
+  // Slots in units of 128 x 128 partial tiles (a 64 x 64 slot is a quarter).
+  auto big_slots = [&](int spread) {
+    const int64_t n = fixup_slots(sc.grid, spread);
+    return (size_t)(tile == 128 ? n : (n + 3) / 4);
+  };
+  int spread = 1;
+  StreamWorkspace* ws = ws_override ? ws_override
+                                    : stream_workspace(dev, s, big_slots(1), &st,
+                                                       (size_t)fixup_slots(sc.grid, 1));
   if (!ws) return st;
-  if ((int)ws->partial_slots < sc.grid)
+  if (ws_override && (ws->partial_slots < big_slots(1) ||
+                      ws->num_flags < (size_t)fixup_slots(sc.grid, 1)))
+    spread = 0;
+  if (ws->partial_slots < big_slots(spread) ||
+      ws->num_flags < (size_t)fixup_slots(sc.grid, spread))
     return fail(SKGEMM_ERR_INVALID_ARG, "workspace has fewer partial slots than the grid");
 
   CUtensorMap mapA, mapB;
@@ -163,7 +175,7 @@ int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
   p.num_tiles = sc.num_tiles;
   p.iters_per_tile = sc.ipt;
   p.total_iters = sc.total;
-  p.grid = sc.grid;
+  p.split = make_split(sc.total, sc.grid);
   p.a_kind = prob.a.kind;
   p.b_kind = prob.b.kind;
   p.tile_order = prob.tile_order;
@@ -177,6 +189,7 @@ int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
   p.flags = ws->flags;
   p.epoch = ++ws->epoch;
   if (p.epoch == 0) p.epoch = ++ws->epoch;  // 0 is the value of a fresh flag
+  p.spread = spread;
   p.err = ws->err;
 
   cudaLaunchConfig_t cfg = {};
@@ -228,7 +241,7 @@ template <class TS>
 int grouped_launch(const Fp64Group& g, cudaStream_t s) {
   // Flags start at zero for every launch (a stream-ordered memset, captured
   // together with the kernel when the pair is recorded into a graph).
-  SKG_CUDA(cudaMemsetAsync(g.flags, 0, (size_t)g.grid * sizeof(uint32_t), s));
+  SKG_CUDA(cudaMemsetAsync(g.flags, 0, (size_t)fixup_slots(g.grid, 1) * sizeof(uint32_t), s));
   fp64_grouped_kernel<TS><<<g.grid, kThreads, TS::kSmem, s>>>(g);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
@@ -242,8 +255,10 @@ int fp64_group_occupancy(DeviceState* dev, int tile, int* blocks_per_sm) {
   return fail(SKGEMM_ERR_INVALID_ARG, "tile must be 128 or 64");
 }
 
-int launch_fp64_group(int tile, const Fp64Group& g, cudaStream_t s) {
-  if (g.grid <= 0 || g.total_iters <= 0) return SKGEMM_OK;
+int launch_fp64_group(int tile, const Fp64Group& group, cudaStream_t s) {
+  if (group.grid <= 0 || group.total_iters <= 0) return SKGEMM_OK;
+  Fp64Group g = group;
+  g.split = make_split(g.total_iters, g.grid);
   if (tile == 128) return grouped_launch<Tile128>(g, s);
   if (tile == 64) return grouped_launch<Tile64>(g, s);
   return fail(SKGEMM_ERR_INVALID_ARG, "tile must be 128 or 64");

@@ -15,10 +15,12 @@
 // Work decomposition (Stream-K): the MAC-loop iterations of all tiles
 // (tiles * ceil(K/BK)) are split evenly over the persistent CTAs. A CTA whose
 // range starts inside a tile stores its partial accumulator to a workspace slot
-// and publishes a flag; the CTA that owns the tile's k = 0 segment waits (with
-// a time budget) for those flags, adds the partials in ascending-k order and
-// runs the epilogue. The reduction order is a pure function of the schedule,
-// so results are bitwise reproducible run to run.
+// and publishes a flag. A tile split over two CTAs is finished by the CTA that
+// owns its k = 0 segment: it waits (with a time budget) for the flag, adds the
+// partial and runs the epilogue. A tile split over more is finished by all the
+// CTAs whose range ends in it (shared_fixup below), each a slice of the
+// elements. The reduction order is a pure function of the schedule, so results
+// are bitwise reproducible run to run.
 //
 // The same body serves one problem (fp64_streamk_kernel, BM = BN = 128, or
 // fp64_streamk_kernel64, BM = BN = 64) and a
@@ -131,8 +133,7 @@ struct SingleSched {
   const Fp64Params& p;
   const CUtensorMap* mA;
   const CUtensorMap* mB;
-  __device__ __forceinline__ int64_t total() const { return p.total_iters; }
-  __device__ __forceinline__ int grid() const { return p.grid; }
+  __device__ __forceinline__ const IterSplit& split() const { return p.split; }
   __device__ __forceinline__ const Fp64Params& prob(int) const { return p; }
   __device__ __forceinline__ const CUtensorMap* map_a(int) const { return mA; }
   __device__ __forceinline__ const CUtensorMap* map_b(int) const { return mB; }
@@ -142,13 +143,13 @@ struct SingleSched {
   __device__ __forceinline__ uint32_t* flags() const { return p.flags; }
   __device__ __forceinline__ uint32_t* err() const { return p.err; }
   __device__ __forceinline__ uint32_t pub() const { return p.epoch; }
+  __device__ __forceinline__ bool spread() const { return p.spread != 0; }
 };
 
 // A group of problems: descriptors and tensor maps in global memory.
 struct GroupSched {
   const Fp64Group& g;
-  __device__ __forceinline__ int64_t total() const { return g.total_iters; }
-  __device__ __forceinline__ int grid() const { return g.grid; }
+  __device__ __forceinline__ const IterSplit& split() const { return g.split; }
   __device__ __forceinline__ const Fp64Params& prob(int i) const { return g.probs[i]; }
   __device__ __forceinline__ const CUtensorMap* map_a(int i) const { return g.maps + 2 * i; }
   __device__ __forceinline__ const CUtensorMap* map_b(int i) const { return g.maps + 2 * i + 1; }
@@ -170,6 +171,7 @@ struct GroupSched {
   __device__ __forceinline__ uint32_t* flags() const { return g.flags; }
   __device__ __forceinline__ uint32_t* err() const { return g.err; }
   __device__ __forceinline__ uint32_t pub() const { return 1u; }
+  __device__ __forceinline__ bool spread() const { return true; }
 };
 
 // Where iteration `it` (< it_end) falls: problem, tile, k-block range of this
@@ -190,6 +192,127 @@ __device__ __forceinline__ Seg locate_seg(const Sched& S, int64_t it, int64_t it
   sg.ke = (int)((int64_t)ipt < sg.kb + (it_end - it) ? (int64_t)ipt : sg.kb + (it_end - it));
   tile_coords(q, sg.tile, sg.tm, sg.tn);
   return sg;
+}
+
+// One output element (m, n) of the finished sum v.
+__device__ __forceinline__ void store_one(const Fp64Params& p, int64_t m, int64_t n, double v) {
+  if (m >= p.M || n >= p.N) return;
+  if (p.out_kind == kOutRowMajor) {
+    p.D[m * p.ldd + n] = p.alpha * v + p.gamma;
+  } else if (p.out_kind == kOutSyrkUpper) {
+    if (m > n) return;
+    double* c = p.D + m + n * p.ldd;
+    double r = p.alpha * v;
+    if (!p.beta_zero) r += p.gamma * (*c);
+    *c = r;
+  } else {  // kOutBand16
+    p.D[(n >> 4) * (p.M * 16) + m * 16 + (n & 15)] = v;
+  }
+}
+
+// Parts from which a tile's fix-up is shared. Fewer are added by the owner
+// alone, which needs no exchange of its own part: with 2 / 3 / 4 as the line a
+// 10000 x 32 rotation (3 parts) takes 14.7 / 10.7 / 10.7 us (10.6 with the
+// owner) and a dense 1000^3 product (4 parts) 87.7 / 88.3 / 85.0 us (82.2);
+// with 5 both stay, and the tiles cut into more parts are faster shared.
+constexpr int kSharedParts = 5;
+
+// CTAs of the tile [tile_begin, tile_end) in iterations: first .. last hold a
+// part of it, first .. red_last finish it (their ranges end in it).
+struct FixupSpan {
+  int first, last, red_last;
+};
+
+template <class Sched>
+__device__ __forceinline__ FixupSpan fixup_span(const Sched& S, int64_t tile_begin,
+                                                int64_t tile_end) {
+  const IterSplit& sp = S.split();
+  FixupSpan f;
+  f.first = sp.cta_of(tile_begin);
+  f.last = sp.cta_of(tile_end - 1);
+  f.red_last = sp.begin(f.last + 1) <= tile_end ? f.last : f.last - 1;
+  return f;
+}
+
+// Shared fix-up of a tile split over more than two CTAs. All parts are in
+// workspace slots (the owner's in slot grid + first); CTA `cta` of first ..
+// red_last sums its slice of the tile's elements over the parts and stores
+// them. Added by the owner alone, the parts are a serial chain of
+// last - first reads of a whole tile by one SM: a 10000 x 32 SYRK (295 parts
+// of 32 KB) took 334 us and a 13824 x 128 GEMM (147 of 128 KB) 445 us, now 21
+// and 29 us. Here every SM reads one tile's worth.
+// Slices of fewer than 256 elements are summed by several threads an element,
+// each over a contiguous run of parts, and the runs added in order. The CTAs
+// of a tile finish together (equal ranges), so nobody waits long; all CTAs
+// are co-resident. A flag that does not arrive within the budget is recorded
+// in the error word.
+template <class TS, bool AKM, class Sched>
+__device__ __noinline__ void shared_fixup(const Sched& S, const Fp64Params& q, FixupSpan f,
+                                          int cta, int tm, int tn, uint32_t pubval, double* red) {
+  constexpr int kSlot = TS::BM * TS::BN;
+  constexpr int NJ = TS::NJ;
+  const int tid = threadIdx.x;  // 0 .. kConsumerThreads - 1
+  const int n = f.last - f.first + 1, nred = f.red_last - f.first + 1;
+  for (int j = tid; j < n; j += kConsumerThreads)
+    fixup_flag_wait(S.flags() + (j == 0 ? S.split().grid + f.first : f.first + j), pubval, S.err(),
+                    kFixupBudgetNs);
+  asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+  const int idx = cta - f.first;
+  const int e0 = (int)((int64_t)idx * kSlot / nred), e1 = (int)((int64_t)(idx + 1) * kSlot / nred);
+  const int ne = e1 - e0;
+  // part(j): slot of the j-th part in ascending k.
+  const double* own = S.workspace() + ((int64_t)S.split().grid + f.first) * kSlot;
+  const double* others = S.workspace() + (int64_t)f.first * kSlot;
+  const int64_t mb = (int64_t)tm * TS::BM, nbase = (int64_t)tn * TS::BN;
+  auto finish = [&](int e, double v) {
+    // Slot element e = reg * 256 + thread: the accumulator layout.
+    const int reg = e / kConsumerThreads, th = e % kConsumerThreads;
+    const int r = reg & 3, j = (reg >> 2) % NJ, i = (reg >> 2) / NJ;
+    const int w = th >> 5, l = th & 31, g = l >> 2, t = l & 3;
+    const int row = (w >> 2) * (TS::BM / 2) + i * 16 +
+                    (AKM ? 4 * (g & 1) + (g >> 1) + 8 * (r >> 1) : 2 * g + (r >> 1));
+    const int col = (w & 3) * (TS::BN / 4) + (j >> 1) * 16 + 4 * t + (j & 1) + 2 * (r & 1);
+    store_one(q, mb + row, nbase + col, v);
+  };
+  const int P = ne > 0 ? min(kConsumerThreads / ne, n) : 0;
+  if (P <= 1) {
+    // Eight elements a thread at a time: the loads of one part are in flight
+    // together (the sums are bound by their latency).
+    constexpr int U = 8;
+    for (int eb = e0 + tid; eb < e1; eb += U * kConsumerThreads) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = eb + u * kConsumerThreads;
+        v[u] = e < e1 ? __ldcg(own + e) : 0.0;
+      }
+#pragma unroll 2
+      for (int j = 1; j < n; ++j) {
+        const double* part = others + (int64_t)j * kSlot + eb;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (eb + u * kConsumerThreads < e1) v[u] += __ldcg(part + u * kConsumerThreads);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (eb + u * kConsumerThreads < e1) finish(eb + u * kConsumerThreads, v[u]);
+    }
+    return;
+  }
+  const int grp = tid / ne, e = e0 + tid % ne;
+  if (grp < P) {
+    const int j0 = (int)((int64_t)grp * n / P), j1 = (int)((int64_t)(grp + 1) * n / P);
+    double v = j0 == 0 ? __ldcg(own + e) : __ldcg(others + (int64_t)j0 * kSlot + e);
+#pragma unroll 8
+    for (int j = j0 + 1; j < j1; ++j) v += __ldcg(others + (int64_t)j * kSlot + e);
+    red[grp * ne + tid % ne] = v;
+  }
+  asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+  if (tid < ne) {
+    double v = red[tid];
+    for (int p = 1; p < P; ++p) v += red[p * ne + tid];
+    finish(e0 + tid, v);
+  }
 }
 
 template <class TS, bool AKM = false, class Sched>
@@ -215,8 +338,8 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   }
   __syncthreads();
 
-  const int64_t it_begin = (int64_t)cta * S.total() / S.grid();
-  const int64_t it_end = (int64_t)(cta + 1) * S.total() / S.grid();
+  const int64_t it_begin = S.split().begin(cta);
+  const int64_t it_end = S.split().begin(cta + 1);
 
   if (warp == kConsumerWarps) {
     // ------------------------------------------------------------ producer
@@ -279,6 +402,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   const uint32_t offk0 = qg * 128 + ((t ^ qg) << 4);
   const uint32_t smem_base = smem_u32(smem);
   __shared__ int fixup_ok;
+  __shared__ double fixup_red[kConsumerThreads];
 
   double acc[MI][NJ][4];
 #pragma unroll
@@ -363,9 +487,16 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     const bool complete = owner && (sg.ke == q.iters_per_tile);
     const int ctid = threadIdx.x;  // 0..255
     constexpr int kSlot = TS::BM * TS::BN;
-    if (!owner) {
+    FixupSpan f = {cta, cta, cta};
+    if (!complete) {
+      const int64_t tb = S.begin(sg.pid) + (int64_t)sg.tile * q.iters_per_tile;
+      f = fixup_span(S, tb, tb + q.iters_per_tile);
+    }
+    const bool shared = S.spread() && f.last - f.first + 1 >= kSharedParts;
+    if (!owner || shared) {
       // Publish this CTA's partial tile (layout [reg][thread], coalesced).
-      double* slot = S.workspace() + (int64_t)cta * kSlot;
+      const int slot_id = owner ? S.split().grid + cta : cta;
+      double* slot = S.workspace() + (int64_t)slot_id * kSlot;
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -375,17 +506,16 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
             __stcg(slot + ((i * NJ + j) * 4 + r) * kConsumerThreads + ctid, acc[i][j][r]);
       __threadfence();
       asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
-      if (ctid == 0) st_release_gpu(S.flags() + cta, pubval);
+      if (ctid == 0) st_release_gpu(S.flags() + slot_id, pubval);
+      if (shared && cta <= f.red_last)
+        shared_fixup<TS, AKM>(S, q, f, cta, sg.tm, sg.tn, pubval, fixup_red);
     } else {
       if (!complete) {
         // Add the partials of the later CTAs that cover the rest of this tile,
         // in ascending k order. A flag that does not arrive within the budget
         // is recorded in the error word and its partial is skipped; the CTA
         // keeps consuming its pipeline so no copy is left in flight.
-        const int64_t tile_end = S.begin(sg.pid) + (int64_t)(sg.tile + 1) * q.iters_per_tile;
-        for (int c2 = cta + 1; c2 < S.grid(); ++c2) {
-          const int64_t s2 = (int64_t)c2 * S.total() / S.grid();
-          if (s2 >= tile_end) break;
+        for (int c2 = cta + 1; c2 <= f.last; ++c2) {
           if (ctid == 0)
             fixup_ok = fixup_flag_wait(S.flags() + c2, pubval, S.err(), kFixupBudgetNs) ? 1 : 0;
           asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));

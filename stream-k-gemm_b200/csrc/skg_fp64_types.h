@@ -60,13 +60,48 @@ enum OutKind : int { kOutRowMajor = 0, kOutSyrkUpper = 1, kOutBand16 = 2 };
 
 enum TileOrder : int { kTilesAll = 0, kTilesUpper = 1 };
 
+// The even split of `total` iterations over `grid` CTAs: CTA c covers
+// [begin(c), begin(c + 1)), begin(c) = floor(c total / grid), held as quotient
+// and remainder so that the kernels divide 32-bit numbers only.
+struct IterSplit {
+  int64_t q;     // total / grid
+  int r;         // total % grid
+  int grid;
+  double inv;    // ~ grid / total, to guess the CTA of an iteration
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  int64_t begin(int c) const {
+    return (int64_t)c * q + (uint32_t)c * (uint32_t)r / (uint32_t)grid;
+  }
+  // The CTA whose range holds iteration i (0 <= i < total).
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  int cta_of(int64_t i) const {
+    int c = (int)((double)i * inv);
+    c = c < grid - 1 ? c : grid - 1;
+    while (begin(c) > i) --c;
+    while (begin(c + 1) <= i) ++c;
+    return c;
+  }
+};
+
+inline IterSplit make_split(int64_t total, int grid) {
+  IterSplit s;
+  s.grid = grid > 0 ? grid : 1;
+  s.q = total / s.grid;
+  s.r = (int)(total % s.grid);
+  s.inv = total > 0 ? (double)s.grid / (double)total : 0.0;
+  return s;
+}
+
 struct Fp64Params {
   int64_t M, N, K;
   int tiles_m, tiles_n;
   int num_tiles;
   int iters_per_tile;  // ceil(K / BK)
   int64_t total_iters;
-  int grid;
   int a_kind, b_kind;
   int tile_order;
   int out_kind;
@@ -75,11 +110,18 @@ struct Fp64Params {
   double alpha;
   double gamma;  // GEMM: added scalar; SYRK: beta
   int beta_zero;
-  double* workspace;  // grid * BM*BN doubles (partial tiles)
-  uint32_t* flags;    // grid flags
+  double* workspace;  // partial tiles: BM*BN doubles per slot, slots(spread, grid)
+  uint32_t* flags;    // one per slot
   uint32_t epoch;     // value a published flag carries for this launch
+  IterSplit split;    // the launch's CTA ranges (single-problem launches)
+  int spread;         // shared fix-up (2 slots per CTA); 0: the owner adds the partials
   uint32_t* err;      // device error word
 };
+
+// Partial-tile slots (and flags) of a launch of `grid` CTAs. A CTA publishes
+// its first segment's partial in slot `cta`; with the shared fix-up the owner
+// of a tile publishes its own part too, in slot grid + cta.
+inline int64_t fixup_slots(int grid, int spread) { return (int64_t)grid * (spread ? 2 : 1); }
 
 // Grouped launch: many independent problems in one persistent Stream-K
 // launch. Their MAC-loop iterations are concatenated (problem p owns
@@ -97,8 +139,9 @@ struct Fp64Group {
   int num_problems;
   int64_t total_iters;
   int grid;
-  double* workspace;  // grid * BM*BN doubles
-  uint32_t* flags;    // grid flags, zero at launch
+  IterSplit split;    // make_split(total_iters, grid)
+  double* workspace;  // 2 * grid slots of BM*BN doubles (shared fix-up)
+  uint32_t* flags;    // 2 * grid flags, zero at launch
   uint32_t* err;
 };
 

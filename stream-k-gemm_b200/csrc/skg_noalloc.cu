@@ -69,7 +69,7 @@ int noalloc_setup(DeviceState* dev, NoAllocDevice& d) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(no-alloc scratch)");
   unsigned char* b = static_cast<unsigned char*>(base);
   d.ws.partials = reinterpret_cast<double*>(b);
-  d.ws.partial_slots = kNoAllocSlots;
+  d.ws.partial_slots = d.ws.num_flags = kNoAllocSlots;
   d.ws.flags = reinterpret_cast<uint32_t*>(b + kNoAllocPartialBytes);
   d.ws.err = reinterpret_cast<uint32_t*>(b + kNoAllocPartialBytes + kNoAllocFlagBytes);
   d.ws.epoch = 0;  // the array starts zeroed: first epoch used is 1

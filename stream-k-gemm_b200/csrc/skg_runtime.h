@@ -58,11 +58,12 @@ struct DeviceBuffer {
 // epoch the flags of the next launch will carry, and the device error word.
 struct StreamWorkspace {
   double* partials = nullptr;
-  size_t partial_slots = 0;
+  size_t partial_slots = 0;  // 128 x 128-tile slots held
+  size_t num_flags = 0;
   uint32_t* flags = nullptr;
   uint32_t* err = nullptr;  // device error word
   uint32_t epoch = 0;
-  int ensure(int slots);
+  int ensure(size_t slots, size_t nflags);
 };
 
 struct DeviceState {
@@ -85,7 +86,9 @@ struct DeviceState {
 // Current device's state (initialises on first use). Returns nullptr and
 // records an error when no sm_100 device is usable.
 DeviceState* current_device(int* status);
-StreamWorkspace* stream_workspace(DeviceState* dev, cudaStream_t s, int slots, int* status);
+// `slots` 128 x 128 partial tiles and `nflags` flags (0: as many as slots).
+StreamWorkspace* stream_workspace(DeviceState* dev, cudaStream_t s, size_t slots, int* status,
+                                  size_t nflags = 0);
 
 // Encodes a tiled TMA descriptor through the driver entry point.
 int encode_tiled(CUtensorMap* map, int rank, const void* base, const uint64_t* dims,
