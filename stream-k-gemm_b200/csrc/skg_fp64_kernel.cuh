@@ -247,7 +247,7 @@ __device__ __forceinline__ FixupSpan fixup_span(const Sched& S, int64_t tile_beg
 // are co-resident. A flag that does not arrive within the budget is recorded
 // in the error word.
 template <class TS, bool AKM, class Sched>
-__device__ __noinline__ void shared_fixup(const Sched& S, const Fp64Params& q, FixupSpan f,
+__device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q, FixupSpan f,
                                           int cta, int tm, int tn, uint32_t pubval, double* red) {
   constexpr int kSlot = TS::BM * TS::BN;
   constexpr int NJ = TS::NJ;
@@ -418,6 +418,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   int hint = S.locate(it_begin < it_end ? it_begin : 0, 0);
   const uint32_t pubval = S.pub();
 
+  bool published = false;  // the last segment's partial sum went to a slot
   for (int64_t it = it_begin; it < it_end;) {
     const Seg sg = locate_seg(S, it, it_end, hint);
     hint = sg.pid;
@@ -433,6 +434,11 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
       b_chunk[qq] = b32 ? (uint32_t)((c & 1) * (TS::BN / 32) + (c >> 1)) : (uint32_t)c;
     }
 
+    // Three iterations a trip (half the ring), so that the loop's own work
+    // spreads over 48 k: GEMM 512 x 512 x 110592 1.670 -> 1.617 ms, SYRK 0.933
+    // -> 0.921, rotation 110592 x 512 1.710 -> 1.680 (two, four, six a trip:
+    // 1.617, 1.617, 1.616 / 0.930, 0.923, 0.923 / 1.685, 1.680, 1.681).
+#pragma unroll 3
     for (int k = sg.kb; k < sg.ke && !aborted; ++k) {
       if (!mbar_wait(&full_bar[stage], phase, S.err())) {
         aborted = true;
@@ -445,6 +451,14 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
       for (int s = 0; s < kBK / 8; ++s) {
         const uint32_t ks = s * 8 * 128;  // k8 step = 8 rows of 128 B
         double2 a_lo[MI], a_hi[MI], b_lo[NQ], b_hi[NQ];
+        auto load_b = [&]() {
+#pragma unroll
+          for (int qq = 0; qq < NQ; ++qq) {
+            b_lo[qq] = lds128(sb + b_chunk[qq] * kChunkBytes + ks + off_r0);
+            b_hi[qq] = lds128(sb + b_chunk[qq] * kChunkBytes + ks + off_r1);
+          }
+        };
+        if constexpr (AKM) load_b();
 #pragma unroll
         for (int i = 0; i < MI; ++i) {
           if constexpr (AKM) {
@@ -457,19 +471,26 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
             a_hi[i] = lds128(sa + i * kChunkBytes + ks + off_r1);
           }
         }
-#pragma unroll
-        for (int qq = 0; qq < NQ; ++qq) {
-          b_lo[qq] = lds128(sb + b_chunk[qq] * kChunkBytes + ks + off_r0);
-          b_hi[qq] = lds128(sb + b_chunk[qq] * kChunkBytes + ks + off_r1);
-        }
+        if constexpr (!AKM) load_b();
+        // The column direction turns at each row of MMAs (a neighbour shares
+        // A or B) where that measured faster: GEMM 512 x 512 x 110592 on
+        // 128 x 128 tiles 1.618 against 1.628 ms, the K-major rotation of
+        // 13824 x 512 0.233 against 0.242 ms; no gain on 64 x 64 packed tiles.
+        constexpr bool kTurn = TS::BM == 128 || AKM;
 #pragma unroll
         for (int i = 0; i < MI; ++i) {
 #pragma unroll
-          for (int qq = 0; qq < NQ; ++qq) {
-            dmma_16x8x8(acc[i][2 * qq], a_lo[i].x, a_lo[i].y, a_hi[i].x, a_hi[i].y, b_lo[qq].x,
-                        b_hi[qq].x);
+          for (int j = 0; j < NQ; ++j) {
+            const bool back = kTurn && (i & 1);
+            const int qq = back ? NQ - 1 - j : j;
+            auto even = [&]() {
+              dmma_16x8x8(acc[i][2 * qq], a_lo[i].x, a_lo[i].y, a_hi[i].x, a_hi[i].y, b_lo[qq].x,
+                          b_hi[qq].x);
+            };
+            if (!back) even();
             dmma_16x8x8(acc[i][2 * qq + 1], a_lo[i].x, a_lo[i].y, a_hi[i].x, a_hi[i].y,
                         b_lo[qq].y, b_hi[qq].y);
+            if (back) even();
           }
         }
       }
@@ -487,12 +508,11 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     const bool complete = owner && (sg.ke == q.iters_per_tile);
     const int ctid = threadIdx.x;  // 0..255
     constexpr int kSlot = TS::BM * TS::BN;
-    FixupSpan f = {cta, cta, cta};
-    if (!complete) {
-      const int64_t tb = S.begin(sg.pid) + (int64_t)sg.tile * q.iters_per_tile;
-      f = fixup_span(S, tb, tb + q.iters_per_tile);
-    }
-    const bool shared = S.spread() && f.last - f.first + 1 >= kSharedParts;
+    const int64_t tile_end = it - sg.kb + q.iters_per_tile;
+    // An owner without the whole tile is in its last segment. It adds the
+    // other parts itself if they are few.
+    const bool shared = owner && !complete && S.spread() && cta + kSharedParts <= S.split().grid &&
+                        S.split().begin(cta + kSharedParts - 1) < tile_end;
     if (!owner || shared) {
       // Publish this CTA's partial tile (layout [reg][thread], coalesced).
       const int slot_id = owner ? S.split().grid + cta : cta;
@@ -507,15 +527,16 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
       __threadfence();
       asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
       if (ctid == 0) st_release_gpu(S.flags() + slot_id, pubval);
-      if (shared && cta <= f.red_last)
-        shared_fixup<TS, AKM>(S, q, f, cta, sg.tm, sg.tn, pubval, fixup_red);
+      published = true;
     } else {
+      published = false;
       if (!complete) {
         // Add the partials of the later CTAs that cover the rest of this tile,
         // in ascending k order. A flag that does not arrive within the budget
         // is recorded in the error word and its partial is skipped; the CTA
         // keeps consuming its pipeline so no copy is left in flight.
-        for (int c2 = cta + 1; c2 <= f.last; ++c2) {
+        for (int c2 = cta + 1; c2 < S.split().grid; ++c2) {
+          if (S.split().begin(c2) >= tile_end) break;
           if (ctid == 0)
             fixup_ok = fixup_flag_wait(S.flags() + c2, pubval, S.err(), kFixupBudgetNs) ? 1 : 0;
           asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
@@ -560,6 +581,15 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
     it += sg.ke - sg.kb;
+  }
+  // The tile this CTA's range ends in, if its part of it went to a slot.
+  if (published && S.spread() && !aborted) {
+    const Seg sg = locate_seg(S, it_end - 1, it_end, 0);
+    const Fp64Params& q = S.prob(sg.pid);
+    const int64_t tb = S.begin(sg.pid) + (int64_t)sg.tile * q.iters_per_tile;
+    const FixupSpan f = fixup_span(S, tb, tb + q.iters_per_tile);
+    if (f.last - f.first + 1 >= kSharedParts)
+      shared_fixup<TS, AKM>(S, q, f, cta, sg.tm, sg.tn, pubval, fixup_red);
   }
 }
 
