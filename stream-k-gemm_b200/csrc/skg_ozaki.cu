@@ -330,7 +330,11 @@ __global__ void row_exponents_kernel(int64_t R, int64_t Rpad, int C, const doubl
 // r + 16 h took twice the L1 store wavefronts); the stage is 128B-swizzled so
 // that the two k-rows a half-warp reads fall on disjoint banks. BF16 (64-byte
 // rows): lane r + 16 h, unswizzled stage. No CTA-wide barrier. Row exponents
-// mu[row] are read from the exponent pass.
+// mu[row] are read from the exponent pass. Only the operand's own 16-row
+// groups are converted: the plane's padding rows (Rpad is a multiple of 128 or
+// 256) keep whatever they hold, since a row of residues only reaches the
+// product's row or column of that index, and those past R are never read back.
+// 42875 x 333 (Rpad = 512): one operand 0.101 -> 0.070 ms.
 constexpr int kConvStages = 3;
 constexpr int kConvWarps = 8;
 constexpr int kConvTile = 16 * 32;  // doubles per warp tile
@@ -423,7 +427,7 @@ __device__ __forceinline__ void convert_stage_i8(const double* stage, int r, int
 // ((k % 16) / 2) ^ (R % 8), half k % 2.
 template <int T, int L, bool BF, bool KM = false>
 __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
-    const __grid_constant__ CUtensorMap map, int64_t KP, int64_t Rpad,
+    const __grid_constant__ CUtensorMap map, int64_t KP, int64_t R, int64_t Rpad,
     const int* __restrict__ mu, uint8_t* __restrict__ res, uint32_t* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -431,7 +435,7 @@ __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kConvWarps * kConvStages * kConvTile * 8) +
                   warp * kConvStages;
   const int64_t KB = KP / 32;
-  const int64_t ntiles = (Rpad / 16) * KB;
+  const int64_t ntiles = ((R + 15) / 16) * KB;
   // Warp gw takes tiles gw, gw + nw, gw + 2 nw, ...: at any moment the
   // machine converts one contiguous window of tiles, so the stores of all
   // warps land in a narrow band of each residue plane (page-local writes)
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(kShortThreads, 3) convert_short_kernel(
   double* sc = red + 256;                         // s1 [16], s2 [16]
   uint64_t* bar = reinterpret_cast<uint64_t*>(sc + 32);
   const int KB = (int)(KP / 32);
-  const int64_t G = Rpad / 16;
+  const int64_t G = (R + 15) / 16;  // the operand's own groups (see the conversion kernel)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
@@ -716,15 +720,16 @@ __device__ __forceinline__ double pow2i(int e) {  // 2^e, e in [-1022, 1023]
 // C[i + j*ldd] = alpha*v + beta*C (beta_zero: no read).
 __global__ void __launch_bounds__(256) crt_partials_kernel(
     int M, int N, int L, const int32_t* __restrict__ partials, int T,
-    const int* __restrict__ tile_index, int tiles_n, const int* __restrict__ mod_slot_off,
+    const int* __restrict__ tile_index, int tiles_n, int bn, const int* __restrict__ mod_slot_off,
     const int* __restrict__ mod_slots, const int* __restrict__ mu, const int* __restrict__ nu,
     int mode, double* __restrict__ D, int64_t ldd, double alpha, double gamma, int beta_zero) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)M * N) return;
   const int i = (int)(idx / N), j = (int)(idx % N);
   if (mode == 1 && i > j) return;
-  const int t = tile_index[(i / kI8BM) * tiles_n + j / kI8BN];
-  const int64_t off = (int64_t)(i % kI8BM) * kI8BN + (j % kI8BN);
+  const int tn = j / bn;
+  const int t = tile_index[(i / kI8BM) * tiles_n + tn];
+  const int64_t off = (int64_t)(i % kI8BM) * kI8BN + (j - tn * bn);
   uint32_t r[kI8MaxModuli];
 #pragma unroll
   for (int l = 0; l < kI8MaxModuli; ++l) {
@@ -823,13 +828,14 @@ int launch_crt_band(int64_t Nd, int64_t nb, const uint8_t* res, const int* mu, c
 // Exact INT8 GEMM output: C[i*ldc + j] = sum over slots of the partial slabs.
 __global__ void __launch_bounds__(256) sum_partials_kernel(
     int M, int N, const int32_t* __restrict__ partials, int T, const int* __restrict__ tile_index,
-    int tiles_n, const int* __restrict__ mod_slot_off, const int* __restrict__ mod_slots,
+    int tiles_n, int bn, const int* __restrict__ mod_slot_off, const int* __restrict__ mod_slots,
     int32_t* __restrict__ C, int64_t ldc) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)M * N) return;
   const int i = (int)(idx / N), j = (int)(idx % N);
-  const int t = tile_index[(i / kI8BM) * tiles_n + j / kI8BN];
-  const int64_t off = (int64_t)(i % kI8BM) * kI8BN + (j % kI8BN);
+  const int tn = j / bn;
+  const int t = tile_index[(i / kI8BM) * tiles_n + tn];
+  const int64_t off = (int64_t)(i % kI8BM) * kI8BN + (j - tn * bn);
   int64_t s = 0;
   for (int q = mod_slot_off[0]; q < mod_slot_off[1]; ++q)
     s += partials[((int64_t)mod_slots[q] * T + t) * (kI8BM * kI8BN) + off];
@@ -840,6 +846,7 @@ __global__ void __launch_bounds__(256) sum_partials_kernel(
 struct LanePlan {
   int T = 0, T1 = 0, Q = 0, slots = 0, L = 0, KB = 0, tiles_m = 0, tiles_n = 0;
   int T2 = 0;              // CTA-pair plans: pair tiles (0: one-CTA plan)
+  int bn = kI8BN;          // columns of a tile
   int4* pairs = nullptr;   // [T2] {tm_lo, tn, t_lo, t_hi}
   // tiles | lane_seg_off | segs | tile_index | mod_slot_off | mod_slots | tile_index2
   DeviceBuffer buf;
@@ -975,6 +982,9 @@ int get_lane_plan(DeviceState* dev, int M, int N, int KB, int L, bool syrk, int 
   pl->KB = KB;
   pl->tiles_m = (M + kI8BM - 1) / kI8BM;
   pl->tiles_n = (N + kI8BN - 1) / kI8BN;
+  // Pair plans cut N evenly, in multiples of 32 (the tiles' number stays).
+  if (units > 0) pl->bn = ((N + pl->tiles_n - 1) / pl->tiles_n + 31) / 32 * 32;
+  const int bn = pl->bn;
   std::vector<int2> tiles;
   std::vector<int4> pairs;
   std::vector<int> tile_index(pl->tiles_m * pl->tiles_n, -1), tile_index2;
@@ -985,7 +995,7 @@ int get_lane_plan(DeviceState* dev, int M, int N, int KB, int L, bool syrk, int 
     if (units == 0) {  // one-CTA plan: row-major tile order
       for (int tm = 0; tm < pl->tiles_m; ++tm)
         for (int tn = 0; tn < pl->tiles_n; ++tn) {
-          if (upper && tm * kI8BM > tn * kI8BN + kI8BN - 1) continue;  // strictly lower
+          if (upper && tm * kI8BM > tn * bn + bn - 1) continue;  // strictly lower
           index[tm * pl->tiles_n + tn] = (int)tiles.size();
           tiles.push_back(make_int2(tm, tn));
         }
@@ -997,7 +1007,7 @@ int get_lane_plan(DeviceState* dev, int M, int N, int KB, int L, bool syrk, int 
         bool need = false;
         for (int h = 0; h < span; ++h) {
           const int tm = tm2 + h;
-          if (tm < pl->tiles_m && !(upper && tm * kI8BM > tn * kI8BN + kI8BN - 1)) need = true;
+          if (tm < pl->tiles_m && !(upper && tm * kI8BM > tn * bn + bn - 1)) need = true;
         }
         if (!need) continue;
         int t[2] = {-1, -1};
@@ -1199,8 +1209,8 @@ int launch_lanes(DeviceState* dev, const LanePlan* pl, const void* resA, int64_t
   const bool pair_k = pl->T2 > 0;
   CUtensorMap mA, mB, mB2;
   if ((st = make_res_map(&mA, resA, KPb, RA, p.L, kI8BM))) return st;
-  if ((st = make_res_map(&mB, resB, KPb, RB, p.L, pair_k ? 128 : kI8BN))) return st;
-  if (resB2 && (st = make_res_map(&mB2, resB2, KPb, RB, p.L, pair_k ? 128 : kI8BN))) return st;
+  if ((st = make_res_map(&mB, resB, KPb, RB, p.L, pair_k ? pl->bn / 2 : kI8BN))) return st;
+  if (resB2 && (st = make_res_map(&mB2, resB2, KPb, RB, p.L, pair_k ? pl->bn / 2 : kI8BN))) return st;
   p.T = pl->T;
   p.T1 = pl->T1;
   p.Q = pl->Q;
@@ -1209,6 +1219,7 @@ int launch_lanes(DeviceState* dev, const LanePlan* pl, const void* resA, int64_t
   p.segs = pl->segs;
   p.T2 = pl->T2;
   p.pairs = pl->pairs;
+  p.bn = pl->bn;
   if (!pair_k)
     return launch_i8(dev, mA, mB, p, std::min(dev->num_sms, pl->T * pl->Q), s, bf,
                      resB2 ? &mB2 : nullptr);
@@ -1282,7 +1293,7 @@ void report(skgemm_options_t* opts, int L, int gamma_bits, int64_t K) {
   }
 
 template <int T, int L, bool BF, bool KM = false>
-int launch_convert(DeviceState* dev, const CUtensorMap& map, int64_t KP, int64_t Rpad,
+int launch_convert(DeviceState* dev, const CUtensorMap& map, int64_t KP, int64_t R, int64_t Rpad,
                    const int* mu, uint8_t* res, uint32_t* err, cudaStream_t s) {
   static int occ[64] = {0};
   if (!occ[dev->device]) {
@@ -1293,14 +1304,14 @@ int launch_convert(DeviceState* dev, const CUtensorMap& map, int64_t KP, int64_t
                                                            256, kConvSmem));
     occ[dev->device] = n > 0 ? n : 1;
   }
-  const int64_t ntiles = (Rpad / 16) * (KP / 32);
+  const int64_t ntiles = ((R + 15) / 16) * (KP / 32);
   const int64_t blocks = std::min<int64_t>((ntiles + kConvWarps - 1) / kConvWarps,
                                            (int64_t)dev->num_sms * occ[dev->device]);
   // (every warp of the grid gets at least one tile only if ntiles >= warps;
   // warps without a tile return at once)
   KernelTimer kt_(s, "convert_tma_kernel");
-  convert_tma_kernel<T, L, BF, KM><<<(unsigned)blocks, 256, kConvSmem, s>>>(map, KP, Rpad, mu,
-                                                                            res, err);
+  convert_tma_kernel<T, L, BF, KM><<<(unsigned)blocks, 256, kConvSmem, s>>>(map, KP, R, Rpad,
+                                                                            mu, res, err);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
 }
@@ -1318,7 +1329,7 @@ int launch_short_L(DeviceState* dev, const CUtensorMap& map, int64_t R, int64_t 
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kShortSmem));
     attr_done[dev->device] = true;
   }
-  const int64_t G = Rpad / 16;
+  const int64_t G = (R + 15) / 16;
   const int64_t grid = std::min<int64_t>(G, 3 * (int64_t)dev->num_sms);  // three CTAs per SM
   KernelTimer kt_(s, "convert_short_kernel");
   convert_short_kernel<L, KM, BF><<<(unsigned)grid, kShortThreads, kShortSmem, s>>>(map, R, K, KP, Rpad,
@@ -1377,9 +1388,9 @@ int prep_convert(DeviceState* dev, int64_t R, int64_t K, int64_t KP, int64_t Rpa
                            CU_TENSOR_MAP_SWIZZLE_128B)))
       return st;
     if (bf) {
-      SKG_DISPATCH_L(L, (launch_convert<16, LL, true, true>(dev, map, KP, Rpad, mp, rp, err, s)))
+      SKG_DISPATCH_L(L, (launch_convert<16, LL, true, true>(dev, map, KP, R, Rpad, mp, rp, err, s)))
     }
-    SKG_DISPATCH_L(L, (launch_convert<16, LL, false, true>(dev, map, KP, Rpad, mp, rp, err, s)))
+    SKG_DISPATCH_L(L, (launch_convert<16, LL, false, true>(dev, map, KP, R, Rpad, mp, rp, err, s)))
   }
   // [P_in][K][T] doubles; boxes of 16 rows x 32 k (zero fill past K / P_in).
   const int64_t P_in = (R + T - 1) / T;
@@ -1391,9 +1402,9 @@ int prep_convert(DeviceState* dev, int64_t R, int64_t K, int64_t KP, int64_t Rpa
                          bf ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B)))
     return st;
   if (bf) {
-    SKG_DISPATCH_L(L, (launch_convert<T, LL, true>(dev, map, KP, Rpad, mp, rp, err, s)))
+    SKG_DISPATCH_L(L, (launch_convert<T, LL, true>(dev, map, KP, R, Rpad, mp, rp, err, s)))
   }
-  SKG_DISPATCH_L(L, (launch_convert<T, LL, false>(dev, map, KP, Rpad, mp, rp, err, s)))
+  SKG_DISPATCH_L(L, (launch_convert<T, LL, false>(dev, map, KP, R, Rpad, mp, rp, err, s)))
 }
 
 template <int T>
@@ -1448,7 +1459,7 @@ template <int L, bool BF>
 int launch_local_L(int64_t R, int64_t K, int64_t KP, int64_t Rpad, const double* src,
                    int64_t panel_stride, int64_t ks, uint8_t* res, int* mu, cudaStream_t s) {
   KernelTimer kt_(s, "convert_local_kernel");
-  convert_local_kernel<L, BF><<<(unsigned)(Rpad / 16), 256, 0, s>>>(R, K, KP, Rpad, src,
+  convert_local_kernel<L, BF><<<(unsigned)((R + 15) / 16), 256, 0, s>>>(R, K, KP, Rpad, src,
                                                                     panel_stride, ks, res, mu);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
@@ -1503,7 +1514,7 @@ int lanes_product(DeviceState* dev, OzakiStream* os, StreamWorkspace* ws, int64_
   const int64_t n = M * N;
   KernelTimer kt_(s, "crt_partials_kernel");
   crt_partials_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-      (int)M, (int)N, L, (const int32_t*)part.ptr, pl->T, pl->tile_index, pl->tiles_n,
+      (int)M, (int)N, L, (const int32_t*)part.ptr, pl->T, pl->tile_index, pl->tiles_n, pl->bn,
       pl->mod_slot_off, pl->mod_slots, (const int*)os->mu_a.ptr, (const int*)muB->ptr,
       syrk ? 1 : 0, D, ldd, alpha, gamma, (syrk && gamma == 0.0) ? 1 : 0);
   SKG_CUDA(cudaGetLastError());
@@ -1548,7 +1559,7 @@ int pair_product(DeviceState* dev, OzakiStream* os, StreamWorkspace* ws, int64_t
   {
     KernelTimer kt_(os->aux, "crt_partials_kernel");
     crt_partials_kernel<<<blocks, 256, 0, os->aux>>>(
-        (int)M, (int)M, L, (const int32_t*)part.ptr, pl->T, pl->tile_index, pl->tiles_n,
+        (int)M, (int)M, L, (const int32_t*)part.ptr, pl->T, pl->tile_index, pl->tiles_n, pl->bn,
         pl->mod_slot_off, pl->mod_slots, (const int*)os->mu_a.ptr, (const int*)os->mu_a.ptr, 1, S,
         lds, alpha_s, beta_s, beta_s == 0.0 ? 1 : 0);
   }
@@ -1557,7 +1568,7 @@ int pair_product(DeviceState* dev, OzakiStream* os, StreamWorkspace* ws, int64_t
   if (e1 != cudaSuccess) return cuda_fail(e1, "crt_partials_kernel");
   KernelTimer kt_(s, "crt_partials_kernel");
   crt_partials_kernel<<<blocks, 256, 0, s>>>(
-      (int)M, (int)M, L, (const int32_t*)part.ptr, pl->T, pl->tile_index2, pl->tiles_n,
+      (int)M, (int)M, L, (const int32_t*)part.ptr, pl->T, pl->tile_index2, pl->tiles_n, pl->bn,
       pl->mod_slot_off, pl->mod_slots, (const int*)os->mu_a.ptr, (const int*)os->mu_b.ptr, 0, Hs,
       ldh, alpha_h, gamma_h, 0);
   SKG_CUDA(cudaGetLastError());
@@ -2091,7 +2102,7 @@ int igemm_s8(int64_t M, int64_t N, int64_t K, const int8_t* A, int64_t lda, cons
   const int64_t n = M * N;
   KernelTimer kt_(s, "sum_partials_kernel");
   sum_partials_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-      (int)M, (int)N, (const int32_t*)os->partials.ptr, pl->T, pl->tile_index, pl->tiles_n,
+      (int)M, (int)N, (const int32_t*)os->partials.ptr, pl->T, pl->tile_index, pl->tiles_n, pl->bn,
       pl->mod_slot_off, pl->mod_slots, C, ldc);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
