@@ -70,30 +70,47 @@ double issued_macs(const Fp64Problem& prob, int tile) {
   return tiles * tile * tile * (double)((prob.K + kBK - 1) / kBK * kBK);
 }
 
-// Tile of a single-problem launch: 64 x 64 when it issues fewer MACs than
-// 128 x 128 (triangles, ragged edges) or when the output has so many
-// 128 x 128 tiles (>= 4 per SM) that two CTAs per SM pay off; 128 x 128
-// otherwise. Measured on B200 with 110592 x 512 operands: SYRK 0.95 ms on
-// 64 x 64 vs 1.08 ms on 128 x 128, rotation 1.72 vs 1.77 ms, GEMM
-// (M = N = 512, 16 tiles) 1.68 vs 1.67 ms.
+// Tile of a single-problem launch, by the MACs it issues (padding included) and
+// how much work a CTA gets. Measured on B200 (us on 128 / 64 / 32 tiles):
+//  * 32 x 32 where it saves enough padding: its operand traffic (half a byte a
+//    MAC) holds it to 0.8 of the 64 x 64 rate. SYRK / GEMM 110592 x 96: 117 /
+//    91 / 62, 118 / 116 / 88; SYRK 110592 x 224: 323 / 269 / 218; not GEMM
+//    110592 x 128 (0 saved): 119 / 117 / 132. Dense operands take more, smaller
+//    loads a tile (2000^3: 494 / 531 / 696) and need 0.7.
+//  * 32 x 32 where the output has fewer 64 x 64 iterations than eight a CTA and
+//    a short reduction, so that latency counts: GEMM 1008 x 128: 23 / 14 / 12,
+//    rotation 1008 x 256: 21 / 16 / 15.
+//  * 64 x 64 where it issues fewer MACs than 128 x 128 (triangles, edges) or
+//    the output has >= 4 tiles of 128 x 128 per SM, so that two CTAs per SM
+//    pay off: SYRK 110592 x 512 1018 / 925.
+//  * 64 x 64 too where a CTA would get few 128 x 128 iterations (the last part
+//    and the fix-up of a tile are a quarter as long): under 200 with packed
+//    operands (GEMM 10000 x 512 (67): 162 / 158, 110592 x 128 (47): 119 / 117;
+//    equal at 187-221), under 60 with a dense one (1000^3 (27): 81 / 76,
+//    rotation 32768 x 256 (55): 155 / 137; 1500^3 (91): 218 / 228).
 int single_tile(DeviceState* dev, const Fp64Problem& prob) {
-  const double i64 = issued_macs(prob, 64), i128 = issued_macs(prob, 128);
-  if (i64 < i128) return 64;
-  const double t128 = i128 / (128.0 * 128.0 * (double)((prob.K + kBK - 1) / kBK * kBK));
-  return (i64 == i128 && t128 >= 4.0 * dev->num_sms) ? 64 : 128;
+  const double i32 = issued_macs(prob, 32), i64 = issued_macs(prob, 64),
+               i128 = issued_macs(prob, 128);
+  const bool dense_a = prob.a.kind == kOpDense, dense = dense_a || prob.b.kind == kOpDense;
+  if (i32 < (dense_a ? 0.7 : 0.8) * i64) return 32;
+  const double ipt = (double)((prob.K + kBK - 1) / kBK);
+  const double it64 = i64 / (64.0 * 64.0 * kBK), it128 = i128 / (128.0 * 128.0 * kBK);
+  if (!dense_a && ipt <= 128 && it64 < 16.0 * dev->num_sms) return 32;
+  if (i64 < i128 || it128 / ipt >= 4.0 * dev->num_sms) return 64;
+  return it128 < (dense ? 60.0 : 200.0) * dev->num_sms ? 64 : 128;
 }
 
 // CTAs per SM of the single-problem kernel of `tile` and A layout (its
 // shared-memory attribute set once per device).
 template <class TS>
 int single_setup(int device, const void* kernel, bool akm, int* per_sm) {
-  static int occ[2][2][64] = {};
-  int& o = occ[TS::BM == 64 ? 1 : 0][akm ? 1 : 0][device];
+  static int occ[2][64] = {};  // per tile shape: one array per instantiation
+  int& o = occ[akm ? 1 : 0][device];
   if (!o) {
     SKG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TS::kSmem));
     int n = 0;
-    SKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, TS::kSmem));
+    SKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, TS::kThreads, TS::kSmem));
     if (n < 1) return fail(SKGEMM_ERR_CUDA, "FP64 kernel does not fit on an SM");
     o = std::min(n, TS::kMinBlocks);
   }
@@ -129,26 +146,41 @@ int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
     return fail(SKGEMM_ERR_UNSUPPORTED, "K == 0 is handled by the caller");
   }
   if (tile == 0) tile = single_tile(dev, prob);
-  if (tile != 128 && tile != 64) return fail(SKGEMM_ERR_INVALID_ARG, "tile must be 128 or 64");
+
+  if (tile != 128 && tile != 64 && tile != 32)
+    return fail(SKGEMM_ERR_INVALID_ARG, "tile must be 128, 64 or 32");
   const bool akm = prob.a.kind == kOpBandK;
   if (prob.b.kind == kOpBandK || (akm && prob.b.kind == kOpPacked32))
     return fail(SKGEMM_ERR_INVALID_ARG, "operand layouts not supported together");
-  const void* kernel = tile == 64 ? (akm ? (const void*)fp64_streamk_kernel64_ak
-                                         : (const void*)fp64_streamk_kernel64)
-                                  : (akm ? (const void*)fp64_streamk_kernel_ak
-                                         : (const void*)fp64_streamk_kernel);
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, Fp64Params);
+  struct Variant {
+    Kernel kernel;
+    const char* name;
+  };
+  static const Variant variants[3][2] = {
+      {{fp64_streamk_kernel, "fp64_streamk_kernel"},
+       {fp64_streamk_kernel_ak, "fp64_streamk_kernel_ak"}},
+      {{fp64_streamk_kernel64, "fp64_streamk_kernel64"},
+       {fp64_streamk_kernel64_ak, "fp64_streamk_kernel64_ak"}},
+      {{fp64_streamk_kernel32, "fp64_streamk_kernel32"},
+       {fp64_streamk_kernel32_ak, "fp64_streamk_kernel32_ak"}}};
+  const Variant& var = variants[tile == 128 ? 0 : (tile == 64 ? 1 : 2)][akm ? 1 : 0];
+  const void* kernel = (const void*)var.kernel;
   int per_sm = 1, st = SKGEMM_OK;
-  if ((st = tile == 64 ? single_setup<Tile64>(dev->device, kernel, akm, &per_sm)
-                       : single_setup<Tile128>(dev->device, kernel, akm, &per_sm)))
+  if ((st = tile == 128  ? single_setup<Tile128>(dev->device, kernel, akm, &per_sm)
+            : tile == 64 ? single_setup<Tile64>(dev->device, kernel, akm, &per_sm)
+                         : single_setup<Tile32>(dev->device, kernel, akm, &per_sm)))
     return st;
   Schedule sc = make_schedule(dev, prob, tile, per_sm);
   if ((int64_t)sc.num_tiles * sc.ipt > ((int64_t)1 << 40))
     return fail(SKGEMM_ERR_INVALID_ARG, "problem too large");
 
-  // Slots in units of 128 x 128 partial tiles (a 64 x 64 slot is a quarter).
+  // Slots in units of 128 x 128 partial tiles (a 64 x 64 slot is a quarter, a
+  // 32 x 32 slot a sixteenth).
   auto big_slots = [&](int spread) {
     const int64_t n = fixup_slots(sc.grid, spread);
-    return (size_t)(tile == 128 ? n : (n + 3) / 4);
+    const int64_t per = (128 / tile) * (128 / tile);
+    return (size_t)((n + per - 1) / per);
   };
   int spread = 1;
   StreamWorkspace* ws = ws_override ? ws_override
@@ -194,22 +226,16 @@ int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(sc.grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = tile == 64 ? Tile64::kSmem : Tile128::kSmem;
+  cfg.blockDim = dim3(tile == 32 ? Tile32::kThreads : Tile64::kThreads);
+  cfg.dynamicSmemBytes = tile == 128 ? Tile128::kSmem : tile == 64 ? Tile64::kSmem : Tile32::kSmem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  KernelTimer kt_(s, tile == 64 ? (akm ? "fp64_streamk_kernel64_ak" : "fp64_streamk_kernel64")
-                                 : (akm ? "fp64_streamk_kernel_ak" : "fp64_streamk_kernel"));
-  if (tile == 64)
-    SKG_CUDA(cudaLaunchKernelEx(&cfg, akm ? fp64_streamk_kernel64_ak : fp64_streamk_kernel64,
-                                mapA, mapB, p));
-  else
-    SKG_CUDA(cudaLaunchKernelEx(&cfg, akm ? fp64_streamk_kernel_ak : fp64_streamk_kernel, mapA,
-                                mapB, p));
+  KernelTimer kt_(s, var.name);
+  SKG_CUDA(cudaLaunchKernelEx(&cfg, var.kernel, mapA, mapB, p));
   return SKGEMM_OK;
 }
 
@@ -229,7 +255,7 @@ int grouped_setup(int device, int* blocks_per_sm) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, TS::kSmem));
     int n = 0;
     SKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp64_grouped_kernel<TS>,
-                                                           kThreads, TS::kSmem));
+                                                           TS::kThreads, TS::kSmem));
     if (n < 1) return fail(SKGEMM_ERR_UNSUPPORTED, "grouped kernel does not fit on an SM");
     occ[device] = n;
   }
@@ -242,7 +268,7 @@ int grouped_launch(const Fp64Group& g, cudaStream_t s) {
   // Flags start at zero for every launch (a stream-ordered memset, captured
   // together with the kernel when the pair is recorded into a graph).
   SKG_CUDA(cudaMemsetAsync(g.flags, 0, (size_t)fixup_slots(g.grid, 1) * sizeof(uint32_t), s));
-  fp64_grouped_kernel<TS><<<g.grid, kThreads, TS::kSmem, s>>>(g);
+  fp64_grouped_kernel<TS><<<g.grid, TS::kThreads, TS::kSmem, s>>>(g);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
 }

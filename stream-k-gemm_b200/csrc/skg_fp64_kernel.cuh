@@ -251,12 +251,12 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
                                           int cta, int tm, int tn, uint32_t pubval, double* red) {
   constexpr int kSlot = TS::BM * TS::BN;
   constexpr int NJ = TS::NJ;
-  const int tid = threadIdx.x;  // 0 .. kConsumerThreads - 1
+  const int tid = threadIdx.x;  // 0 .. TS::kCons - 1
   const int n = f.last - f.first + 1, nred = f.red_last - f.first + 1;
-  for (int j = tid; j < n; j += kConsumerThreads)
+  for (int j = tid; j < n; j += TS::kCons)
     fixup_flag_wait(S.flags() + (j == 0 ? S.split().grid + f.first : f.first + j), pubval, S.err(),
                     kFixupBudgetNs);
-  asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons) : "memory");
   const int idx = cta - f.first;
   const int e0 = (int)((int64_t)idx * kSlot / nred), e1 = (int)((int64_t)(idx + 1) * kSlot / nred);
   const int ne = e1 - e0;
@@ -266,24 +266,24 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
   const int64_t mb = (int64_t)tm * TS::BM, nbase = (int64_t)tn * TS::BN;
   auto finish = [&](int e, double v) {
     // Slot element e = reg * 256 + thread: the accumulator layout.
-    const int reg = e / kConsumerThreads, th = e % kConsumerThreads;
+    const int reg = e / TS::kCons, th = e % TS::kCons;
     const int r = reg & 3, j = (reg >> 2) % NJ, i = (reg >> 2) / NJ;
     const int w = th >> 5, l = th & 31, g = l >> 2, t = l & 3;
-    const int row = (w >> 2) * (TS::BM / 2) + i * 16 +
+    const int row = (w / TS::WN) * (TS::BM / TS::WM) + i * 16 +
                     (AKM ? 4 * (g & 1) + (g >> 1) + 8 * (r >> 1) : 2 * g + (r >> 1));
-    const int col = (w & 3) * (TS::BN / 4) + (j >> 1) * 16 + 4 * t + (j & 1) + 2 * (r & 1);
+    const int col = (w % TS::WN) * (TS::BN / TS::WN) + (j >> 1) * 16 + 4 * t + (j & 1) + 2 * (r & 1);
     store_one(q, mb + row, nbase + col, v);
   };
-  const int P = ne > 0 ? min(kConsumerThreads / ne, n) : 0;
+  const int P = ne > 0 ? min(TS::kCons / ne, n) : 0;
   if (P <= 1) {
     // Eight elements a thread at a time: the loads of one part are in flight
     // together (the sums are bound by their latency).
     constexpr int U = 8;
-    for (int eb = e0 + tid; eb < e1; eb += U * kConsumerThreads) {
+    for (int eb = e0 + tid; eb < e1; eb += U * TS::kCons) {
       double v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int e = eb + u * kConsumerThreads;
+        const int e = eb + u * TS::kCons;
         v[u] = e < e1 ? __ldcg(own + e) : 0.0;
       }
 #pragma unroll 2
@@ -291,11 +291,11 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
         const double* part = others + (int64_t)j * kSlot + eb;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (eb + u * kConsumerThreads < e1) v[u] += __ldcg(part + u * kConsumerThreads);
+          if (eb + u * TS::kCons < e1) v[u] += __ldcg(part + u * TS::kCons);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (eb + u * kConsumerThreads < e1) finish(eb + u * kConsumerThreads, v[u]);
+        if (eb + u * TS::kCons < e1) finish(eb + u * TS::kCons, v[u]);
     }
     return;
   }
@@ -307,7 +307,7 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
     for (int j = j0 + 1; j < j1; ++j) v += __ldcg(others + (int64_t)j * kSlot + e);
     red[grp * ne + tid % ne] = v;
   }
-  asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons) : "memory");
   if (tid < ne) {
     double v = red[tid];
     for (int p = 1; p < P; ++p) v += red[p * ne + tid];
@@ -331,7 +331,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], kConsumerWarps);
+      mbar_init(&empty_bar[s], TS::kWarps);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -341,7 +341,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   const int64_t it_begin = S.split().begin(cta);
   const int64_t it_end = S.split().begin(cta + 1);
 
-  if (warp == kConsumerWarps) {
+  if (warp == TS::kWarps) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
       int stage = 0;
@@ -381,8 +381,8 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
 
   // -------------------------------------------------------------- consumers
   constexpr int MI = TS::MI, NJ = TS::NJ, NQ = TS::NQ;
-  const int wm = warp >> 2;  // 0..1 : rows wm*BM/2 ..
-  const int wn = warp & 3;   // 0..3 : cols wn*BN/4 ..
+  const int wm = warp / TS::WN;  // rows wm*BM/WM ..
+  const int wn = warp % TS::WN;  // cols wn*BN/WN ..
   const int g = lane >> 2;
   const int t = lane & 3;
   // Byte offsets inside a chunk of the two k-rows this lane reads per k8 step.
@@ -402,7 +402,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   const uint32_t offk0 = qg * 128 + ((t ^ qg) << 4);
   const uint32_t smem_base = smem_u32(smem);
   __shared__ int fixup_ok;
-  __shared__ double fixup_red[kConsumerThreads];
+  __shared__ double fixup_red[TS::kCons];
 
   double acc[MI][NJ][4];
 #pragma unroll
@@ -523,9 +523,9 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int r = 0; r < 4; ++r)
-            __stcg(slot + ((i * NJ + j) * 4 + r) * kConsumerThreads + ctid, acc[i][j][r]);
+            __stcg(slot + ((i * NJ + j) * 4 + r) * TS::kCons + ctid, acc[i][j][r]);
       __threadfence();
-      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
+      asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons));
       if (ctid == 0) st_release_gpu(S.flags() + slot_id, pubval);
       published = true;
     } else {
@@ -539,9 +539,9 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
           if (S.split().begin(c2) >= tile_end) break;
           if (ctid == 0)
             fixup_ok = fixup_flag_wait(S.flags() + c2, pubval, S.err(), kFixupBudgetNs) ? 1 : 0;
-          asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
+          asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons));
           const bool have = fixup_ok != 0;
-          asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads));
+          asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons));
           if (!have) continue;
           const double* slot = S.workspace() + (int64_t)c2 * kSlot;
 #pragma unroll
@@ -550,13 +550,13 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
             for (int j = 0; j < NJ; ++j)
 #pragma unroll
               for (int r = 0; r < 4; ++r)
-                acc[i][j][r] += __ldcg(slot + ((i * NJ + j) * 4 + r) * kConsumerThreads + ctid);
+                acc[i][j][r] += __ldcg(slot + ((i * NJ + j) * 4 + r) * TS::kCons + ctid);
         }
       }
       // Final epilogue for tile (tm, tn).
-      const int64_t mbase = (int64_t)sg.tm * TS::BM + wm * (TS::BM / 2);
-      const int64_t nbase = (int64_t)sg.tn * TS::BN + wn * (TS::BN / 4);
-      const bool syrk_skip = (q.out_kind == kOutSyrkUpper) && (mbase > nbase + TS::BN / 4 - 1);
+      const int64_t mbase = (int64_t)sg.tm * TS::BM + wm * (TS::BM / TS::WM);
+      const int64_t nbase = (int64_t)sg.tn * TS::BN + wn * (TS::BN / TS::WN);
+      const bool syrk_skip = (q.out_kind == kOutSyrkUpper) && (mbase > nbase + TS::BN / TS::WN - 1);
       if (!syrk_skip) {
 #pragma unroll
         for (int i = 0; i < MI; ++i) {
@@ -593,7 +593,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Tile128::kThreads, 1)
     fp64_streamk_kernel(const __grid_constant__ CUtensorMap mapA,
                         const __grid_constant__ CUtensorMap mapB,
                         const __grid_constant__ Fp64Params p) {
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // One problem on 64 x 64 tiles, two CTAs per SM.
-__global__ void __launch_bounds__(kThreads, Tile64::kMinBlocks)
+__global__ void __launch_bounds__(Tile64::kThreads, Tile64::kMinBlocks)
     fp64_streamk_kernel64(const __grid_constant__ CUtensorMap mapA,
                           const __grid_constant__ CUtensorMap mapB,
                           const __grid_constant__ Fp64Params p) {
@@ -610,9 +610,18 @@ __global__ void __launch_bounds__(kThreads, Tile64::kMinBlocks)
   streamk_body<Tile64>(S);
 }
 
-// The same two kernels on a K-major A (kOpBandK: the rotation reading
+// One problem on 32 x 32 tiles, four CTAs of four MMA warps per SM.
+__global__ void __launch_bounds__(Tile32::kThreads, Tile32::kMinBlocks)
+    fp64_streamk_kernel32(const __grid_constant__ CUtensorMap mapA,
+                          const __grid_constant__ CUtensorMap mapB,
+                          const __grid_constant__ Fp64Params p) {
+  const SingleSched S{p, &mapA, &mapB};
+  streamk_body<Tile32>(S);
+}
+
+// The same kernels on a K-major A (kOpBandK: the rotation reading
 // band-packed Psi, the band -> grid transposition folded into the loads).
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Tile128::kThreads, 1)
     fp64_streamk_kernel_ak(const __grid_constant__ CUtensorMap mapA,
                            const __grid_constant__ CUtensorMap mapB,
                            const __grid_constant__ Fp64Params p) {
@@ -620,7 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   streamk_body<Tile128, true>(S);
 }
 
-__global__ void __launch_bounds__(kThreads, Tile64::kMinBlocks)
+__global__ void __launch_bounds__(Tile64::kThreads, Tile64::kMinBlocks)
     fp64_streamk_kernel64_ak(const __grid_constant__ CUtensorMap mapA,
                              const __grid_constant__ CUtensorMap mapB,
                              const __grid_constant__ Fp64Params p) {
@@ -628,8 +637,16 @@ __global__ void __launch_bounds__(kThreads, Tile64::kMinBlocks)
   streamk_body<Tile64, true>(S);
 }
 
+__global__ void __launch_bounds__(Tile32::kThreads, Tile32::kMinBlocks)
+    fp64_streamk_kernel32_ak(const __grid_constant__ CUtensorMap mapA,
+                             const __grid_constant__ CUtensorMap mapB,
+                             const __grid_constant__ Fp64Params p) {
+  const SingleSched S{p, &mapA, &mapB};
+  streamk_body<Tile32, true>(S);
+}
+
 template <class TS>
-__global__ void __launch_bounds__(kThreads, TS::kMinBlocks)
+__global__ void __launch_bounds__(TS::kThreads, TS::kMinBlocks)
     fp64_grouped_kernel(const __grid_constant__ Fp64Group g) {
   const GroupSched S{g};
   streamk_body<TS>(S);

@@ -11,37 +11,38 @@ constexpr int kBM = 128;
 constexpr int kBN = 128;
 constexpr int kBK = 16;
 constexpr int kStages = 6;
-constexpr int kConsumerWarps = 8;
-constexpr int kConsumerThreads = kConsumerWarps * 32;
-constexpr int kThreads = kConsumerThreads + 32;  // + one producer warp
 constexpr int kChunkBytes = kBK * 16 * 8;           // [BK][16] doubles = 2 KB
 constexpr int kTileABytes = (kBM / 16) * kChunkBytes;  // 16 KB
 constexpr int kTileBBytes = (kBN / 16) * kChunkBytes;  // 16 KB
 constexpr int kStageBytes = kTileABytes + kTileBBytes;
-constexpr int kAccPerThread = 64;  // warp tile 64x32 -> 64 doubles per lane
 constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
 
-// Output-tile shape of one kernel instantiation. Eight consumer warps in a
-// 2 x 4 grid: a warp owns (BM/2) x (BN/4) outputs = MI m16 blocks x NJ n8
-// blocks, fed by MI A chunks and NQ = NJ/2 B chunks of 16 columns.
-template <int BM_, int BN_>
+// Output-tile shape of one kernel instantiation: WM x WN consumer warps, each
+// owning (BM/WM) x (BN/WN) outputs = MI m16 blocks x NJ n8 blocks, fed by MI A
+// chunks and NQ = NJ/2 B chunks of 16 columns; one more warp issues the loads.
+template <int BM_, int BN_, int WM_, int WN_>
 struct TileShape {
   static constexpr int BM = BM_;
   static constexpr int BN = BN_;
-  static constexpr int MI = BM / 32;
-  static constexpr int NJ = BN / 32;
+  static constexpr int WM = WM_;
+  static constexpr int WN = WN_;
+  static constexpr int kWarps = WM * WN;        // consumer warps
+  static constexpr int kCons = kWarps * 32;     // consumer threads
+  static constexpr int kThreads = kCons + 32;   // + one producer warp
+  static constexpr int MI = BM / (16 * WM);
+  static constexpr int NJ = BN / (8 * WN);
   static constexpr int NQ = NJ / 2;
   static constexpr int kABytes = (BM / 16) * kChunkBytes;
   static constexpr int kBBytes = (BN / 16) * kChunkBytes;
   static constexpr int kStage = kABytes + kBBytes;
   static constexpr int kSmem = kStages * kStage + 1024 /*align*/ + 256 /*barriers*/;
-  static constexpr int kAcc = MI * NJ * 4;  // doubles per consumer thread
   // CTAs per SM the launch bounds ask for: one 197 KB ring for 128 x 128,
-  // two 97 KB rings for 64 x 64.
-  static constexpr int kMinBlocks = BM * BN >= 128 * 128 ? 1 : 2;
+  // two 97 KB rings for 64 x 64, four 49 KB rings for 32 x 32.
+  static constexpr int kMinBlocks = BM >= 128 ? 1 : (BM >= 64 ? 2 : 4);
 };
-using Tile128 = TileShape<128, 128>;
-using Tile64 = TileShape<64, 64>;
+using Tile128 = TileShape<128, 128, 2, 4>;
+using Tile64 = TileShape<64, 64, 2, 4>;
+using Tile32 = TileShape<32, 32, 2, 2>;
 static_assert(Tile128::kStage == kStageBytes && Tile128::kSmem == kSmemBytes, "tile constants");
 
 enum OperandKind : int {

@@ -117,7 +117,7 @@ struct Fp64Problem {
 
 // Enqueues the native FP64 Stream-K kernel on `s`. `ws_override` (optional)
 // supplies caller-owned partial slots/flags/err instead of the stream cache.
-// `tile` 128 or 64 fixes the output tile; 0 lets the cost model choose.
+// `tile` 128, 64 or 32 fixes the output tile; 0 lets the cost model choose.
 int launch_fp64(DeviceState* dev, const Fp64Problem& prob, cudaStream_t s,
                 StreamWorkspace* ws_override = nullptr, int tile = 0);
 // Number of Stream-K partial slots the 128 x 128-tile launch of `prob` uses

@@ -1,6 +1,6 @@
 """Stream-K tiles cut into many parts: the fix-up shared by the CTAs that end in
-a tile (five parts or more) and the owner's own (fewer), on both tile shapes,
-every output layout and the grouped launch. One 64 x 64 tile over the whole
+a tile (five parts or more) and the owner's own (fewer), on the three tile shapes
+that the sizes choose, every output layout and the grouped launch. One 64 x 64 tile over the whole
 machine, parts of one iteration, uneven splits and tiles that end on a range
 boundary. Bar: the repository's 1e-13 relative Frobenius error against Dot2."""
 import numpy as np
@@ -20,7 +20,8 @@ def dev(x):
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4736), (32, 32, 10000), (64, 64, 300), (64, 64, 4736),
                                    (65, 40, 1185), (128, 128, 2368), (128, 128, 13824),
-                                   (200, 136, 3000), (500, 300, 900), (1000, 1000, 200)])
+                                   (200, 136, 3000), (500, 300, 900), (1000, 1000, 200),
+                                   (33, 31, 17), (96, 70, 20000), (257, 129, 1000)])
 def test_gemm_parts(cuda, M, N, K):
     A, B = gaussian((M, K), M + K), gaussian((K, N), N + 3 * K)
     a, b = dev(oracle.pack(A, 16)), dev(oracle.pack(np.ascontiguousarray(B.T), 32))
@@ -34,7 +35,8 @@ def test_gemm_parts(cuda, M, N, K):
     assert oracle.rel_frobenius(out[0], oracle.dot2_matmul(A, B, 1.5, 0.25)) <= 1e-13
 
 
-@pytest.mark.parametrize("M,K", [(16, 5000), (64, 777), (100, 4736), (130, 12000), (512, 600)])
+@pytest.mark.parametrize("M,K", [(16, 5000), (64, 777), (100, 4736), (130, 12000), (512, 600),
+                                 (31, 40), (70, 9000), (33, 16)])
 def test_syrk_parts(cuda, M, K):
     A, C = gaussian((M, K), M * 7 + K), gaussian((M, M), M)
     c = dev(C.T)  # column-major
@@ -48,7 +50,8 @@ def test_syrk_parts(cuda, M, K):
     assert np.array_equal(got[il], C[il])
 
 
-@pytest.mark.parametrize("Nd,nb", [(64, 64), (16, 512), (128, 1024), (208, 336)])
+@pytest.mark.parametrize("Nd,nb", [(64, 64), (16, 512), (128, 1024), (208, 336), (4096, 32),
+                                   (1008, 96), (16, 16)])
 def test_rotation_parts(cuda, Nd, nb):
     psi, Q = gaussian((Nd, nb), Nd + nb), gaussian((nb, nb), nb)
     want = oracle.band_pack(oracle.dot2_matmul(psi, Q)).ravel()
