@@ -533,7 +533,9 @@ int skgemm_serve_run(skgemm_serve_request_t* reqs, int n, skgemm_serve_options_t
 int skgemm_serve_simulate(skgemm_serve_request_t* reqs, int n, skgemm_serve_options_t* opts);
 
 /* Releases the per-stream scratch the library keeps for `stream` (Stream-K
- * partial slots, Ozaki residue buffers); synchronises the stream first. */
+ * partial slots, Ozaki residue buffers); synchronises the stream first. The
+ * default stream (NULL) also gives back the pinned slots (up to 16 MB) through
+ * which the host-pointer calls copy pageable memory. */
 int skgemm_stream_release(void* stream);
 
 #ifdef __cplusplus

@@ -13,6 +13,7 @@
 #include "skg_batch.h"
 #include "skg_common.cuh"
 #include "skg_fp64_types.h"
+#include "skg_hostcopy.h"
 #include "skg_ozaki.h"
 #include "skg_runtime.h"
 
@@ -364,20 +365,35 @@ int run_host(int nin, const HostIO* in, void* out_host, size_t out_bytes, bool o
   if (!dev->host_stream) SKG_CUDA(cudaStreamCreateWithFlags(&dev->host_stream, cudaStreamNonBlocking));
   cudaStream_t s = dev->host_stream;
   void* dptr[4] = {nullptr, nullptr, nullptr, nullptr};
-  for (int i = 0; i < nin; ++i) {
-    if ((st = dev->stage[i].ensure(in[i].bytes ? in[i].bytes : 16)) != SKGEMM_OK) return st;
-    dptr[i] = dev->stage[i].ptr;
-    if (in[i].bytes) SKG_CUDA(cudaMemcpyAsync(dptr[i], in[i].src, in[i].bytes, cudaMemcpyHostToDevice, s));
+  {
+    HostCopy up(dev, cudaMemcpyHostToDevice, s);
+    for (int i = 0; i < nin; ++i) {
+      if ((st = dev->stage[i].ensure(in[i].bytes ? in[i].bytes : 16)) != SKGEMM_OK) return st;
+      dptr[i] = dev->stage[i].ptr;
+      up.add(0, dptr[i], in[i].bytes, in[i].src, in[i].bytes, in[i].bytes, 1);
+    }
+    if ((st = dev->stage[3].ensure(out_bytes ? out_bytes : 16)) != SKGEMM_OK) return st;
+    dptr[3] = dev->stage[3].ptr;
+    if (out_is_input) up.add(0, dptr[3], out_bytes, out_host, out_bytes, out_bytes, 1);
+    if ((st = up.start()) == SKGEMM_OK) st = up.finish();
+    if (st != SKGEMM_OK) {
+      cudaStreamSynchronize(s);
+      return st;
+    }
   }
-  if ((st = dev->stage[3].ensure(out_bytes ? out_bytes : 16)) != SKGEMM_OK) return st;
-  dptr[3] = dev->stage[3].ptr;
-  if (out_is_input && out_bytes)
-    SKG_CUDA(cudaMemcpyAsync(dptr[3], out_host, out_bytes, cudaMemcpyHostToDevice, s));
   if ((st = body(dptr, s)) != SKGEMM_OK) {
     cudaStreamSynchronize(s);
     return st;
   }
-  if (out_bytes) SKG_CUDA(cudaMemcpyAsync(out_host, dptr[3], out_bytes, cudaMemcpyDeviceToHost, s));
+  {
+    HostCopy down(dev, cudaMemcpyDeviceToHost, s);
+    down.add(0, out_host, out_bytes, dptr[3], out_bytes, out_bytes, 1);
+    if ((st = down.start()) == SKGEMM_OK) st = down.finish();
+    if (st != SKGEMM_OK) {
+      cudaStreamSynchronize(s);
+      return st;
+    }
+  }
   StreamWorkspace* ws = nullptr;
   {
     std::lock_guard<std::mutex> lk2(dev->mu);
@@ -434,6 +450,10 @@ SKG_EXPORT int skgemm_stream_release(void* stream) {
       delete ws;
       dev->ws.erase(it);
     }
+  }
+  if (s == nullptr) {  // the host-pointer calls' pinned slots go with the default stream's
+    std::lock_guard<std::mutex> lk(dev->host_mu);
+    host_slots_release(dev);
   }
   return ozaki_release_stream(dev, s);
 }
@@ -616,11 +636,11 @@ int host_chunks(int64_t K) {
   return (int)std::min<int64_t>(kHostChunks, std::max<int64_t>(1, K / kHostChunkK));
 }
 
-cudaError_t upload_packed_chunk(double* dst, const double* src, int T, int64_t R, int64_t K,
-                                int64_t k0, int64_t kc, cudaStream_t s) {
+void add_packed_chunk(HostCopy& up, int g, double* dst, const double* src, int T, int64_t R,
+                      int64_t K, int64_t k0, int64_t kc) {
   const int64_t panels = (R + T - 1) / T;
-  return cudaMemcpy2DAsync(dst, (size_t)kc * T * 8, src + k0 * T, (size_t)K * T * 8,
-                           (size_t)kc * T * 8, (size_t)panels, cudaMemcpyHostToDevice, s);
+  up.add(g, dst, (size_t)kc * T * 8, src + k0 * T, (size_t)K * T * 8, (size_t)kc * T * 8,
+         (size_t)panels);
 }
 
 struct HostPipe {
@@ -679,19 +699,24 @@ SKG_EXPORT int skgemm_dgemm_packed(int64_t M, int64_t N, int64_t K, const double
     double* dA = (double*)dev->stage[0].ptr;
     double* dB = (double*)dev->stage[1].ptr;
     double* dD = (double*)dev->stage[3].ptr;
+    HostCopy up(dev, cudaMemcpyHostToDevice, hp.si);
+    auto k_of = [&](int c) { return K * c / C; };
+    for (int c = 0; c < C; ++c) {
+      add_packed_chunk(up, c, dA + PA * 16 * k_of(c), Ap, 16, M, K, k_of(c), k_of(c + 1) - k_of(c));
+      add_packed_chunk(up, c, dB + PB * 32 * k_of(c), Bp, 32, N, K, k_of(c), k_of(c + 1) - k_of(c));
+    }
+    st = up.start();
     for (int c = 0; c < C && st == SKGEMM_OK; ++c) {
-      const int64_t k0 = K * c / C, kc = K * (c + 1) / C - k0;
-      double* a = dA + PA * 16 * k0;
-      double* b = dB + PB * 32 * k0;
-      cudaError_t e = upload_packed_chunk(a, Ap, 16, M, K, k0, kc, hp.si);
-      if (e == cudaSuccess) e = upload_packed_chunk(b, Bp, 32, N, K, k0, kc, hp.si);
-      if (e == cudaSuccess) e = cudaEventRecord(hp.ev[c], hp.si);
+      if ((st = up.wait_group(c))) break;
+      cudaError_t e = cudaEventRecord(hp.ev[c], hp.si);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(hp.sc, hp.ev[c], 0);
       if (e != cudaSuccess) {
         st = cuda_fail(e, "GEMM chunk upload");
         break;
       }
-      st = skgemm_dgemm_packed_dev(M, N, kc, a, b, dD + (size_t)c * M * N, N, alpha, 0.0, hp.sc);
+      st = skgemm_dgemm_packed_dev(M, N, k_of(c + 1) - k_of(c), dA + PA * 16 * k_of(c),
+                                   dB + PB * 32 * k_of(c), dD + (size_t)c * M * N, N, alpha, 0.0,
+                                   hp.sc);
     }
     if (!st) st = launch_sum_parts(dD, C, M * N, gamma, dD, hp.sc);
     if (!st) {
@@ -815,17 +840,21 @@ SKG_EXPORT int skgemm_dsyrk_packed(int64_t K, int64_t M, const double* Ap, doubl
     // returns as the caller passed it.
     cudaError_t e = cudaMemcpyAsync(dC, C, (size_t)M * M * 8, cudaMemcpyHostToDevice, hp.si);
     if (e != cudaSuccess) return hp.finish(cuda_fail(e, "SYRK upload"));
+    HostCopy up(dev, cudaMemcpyHostToDevice, hp.si);
+    auto k_of = [&](int c) { return K * c / nch; };
+    for (int c = 0; c < nch; ++c)
+      add_packed_chunk(up, c, dA + PA * 16 * k_of(c), Ap, 16, M, K, k_of(c), k_of(c + 1) - k_of(c));
+    st = up.start();
     for (int c = 0; c < nch && st == SKGEMM_OK; ++c) {
-      const int64_t k0 = K * c / nch, kc = K * (c + 1) / nch - k0;
-      double* a = dA + PA * 16 * k0;
-      e = upload_packed_chunk(a, Ap, 16, M, K, k0, kc, hp.si);
-      if (e == cudaSuccess) e = cudaEventRecord(hp.ev[c], hp.si);
+      if ((st = up.wait_group(c))) break;
+      e = cudaEventRecord(hp.ev[c], hp.si);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(hp.sc, hp.ev[c], 0);
       if (e != cudaSuccess) {
         st = cuda_fail(e, "SYRK chunk upload");
         break;
       }
-      st = skgemm_dsyrk_packed_dev(kc, M, a, dC, M, alpha, c == 0 ? beta : 1.0, hp.sc);
+      st = skgemm_dsyrk_packed_dev(k_of(c + 1) - k_of(c), M, dA + PA * 16 * k_of(c), dC, M, alpha,
+                                   c == 0 ? beta : 1.0, hp.sc);
     }
     if (!st) {
       e = cudaMemcpyAsync(C, dC, (size_t)M * M * 8, cudaMemcpyDeviceToHost, hp.sc);
@@ -961,29 +990,40 @@ static int host_rot(int64_t Nd, int64_t nb, const double* A, const double* Q, do
   const int C = (int)std::min<int64_t>(8, panels);
   std::vector<cudaEvent_t> ev(2 * C, nullptr);
   for (auto& e : ev) SKG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  SKG_CUDA(cudaMemcpyAsync(dQ, Q, (size_t)nb * nb * 8, cudaMemcpyHostToDevice, si));
-  for (int c = 0; c < C && st == SKGEMM_OK; ++c) {
-    const int64_t p0 = panels * c / C, p1 = panels * (c + 1) / C;
-    const int64_t g0 = p0 * 16, rows = (p1 - p0) * 16;
-    const size_t off = (size_t)g0 * nb;  // doubles: grid-packed rows and the chunk's output block
-    cudaError_t e = cudaMemcpyAsync(dA + off, A + off, (size_t)rows * nb * 8,
-                                    cudaMemcpyHostToDevice, si);
-    if (e == cudaSuccess) e = cudaEventRecord(ev[2 * c], si);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(sc, ev[2 * c], 0);
-    if (e != cudaSuccess) {
-      st = cuda_fail(e, "rotation upload");
-      break;
+  {
+    HostCopy up(dev, cudaMemcpyHostToDevice, si), down(dev, cudaMemcpyDeviceToHost, so);
+    auto g_of = [&](int c) { return panels * c / C * 16; };  // first grid point of chunk c
+    up.add(0, dQ, (size_t)nb * nb * 8, Q, (size_t)nb * nb * 8, (size_t)nb * nb * 8, 1);
+    for (int c = 0; c < C; ++c) {
+      const int64_t g0 = g_of(c), rows = g_of(c + 1) - g0;
+      const size_t off = (size_t)g0 * nb;  // doubles: grid-packed rows and the output block
+      const size_t n = (size_t)rows * nb * 8, seg = (size_t)rows * 16 * 8;
+      up.add(c, dA + off, n, A + off, n, n, 1);
+      // Band b of the chunk (rows x 16 doubles at dD + off + b rows 16) goes to
+      // D + b Nd 16 + g0 16.
+      down.add(c, D + g0 * 16, (size_t)Nd * 16 * 8, dD + off, seg, seg, (size_t)(nb / 16));
     }
-    if ((st = skgemm_drot_dev_opt(rows, nb, dA + off, dQ, dD + off, opts, sc)) != SKGEMM_OK)
-      break;
-    e = cudaEventRecord(ev[2 * c + 1], sc);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(so, ev[2 * c + 1], 0);
-    // Band b of the chunk (rows x 16 doubles at dD + off + b rows 16) goes to
-    // D + b Nd 16 + g0 16.
-    if (e == cudaSuccess)
-      e = cudaMemcpy2DAsync(D + g0 * 16, (size_t)Nd * 16 * 8, dD + off, (size_t)rows * 16 * 8,
-                            (size_t)rows * 16 * 8, (size_t)(nb / 16), cudaMemcpyDeviceToHost, so);
-    if (e != cudaSuccess) st = cuda_fail(e, "rotation download");
+    if ((st = up.start()) == SKGEMM_OK) st = down.start(true);
+    for (int c = 0; c < C && st == SKGEMM_OK; ++c) {
+      const size_t off = (size_t)g_of(c) * nb;
+      if ((st = up.wait_group(c))) break;
+      cudaError_t e = cudaEventRecord(ev[2 * c], si);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(sc, ev[2 * c], 0);
+      if (e != cudaSuccess) {
+        st = cuda_fail(e, "rotation upload");
+        break;
+      }
+      if ((st = skgemm_drot_dev_opt(g_of(c + 1) - g_of(c), nb, dA + off, dQ, dD + off, opts, sc)) !=
+          SKGEMM_OK)
+        break;
+      e = cudaEventRecord(ev[2 * c + 1], sc);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(so, ev[2 * c + 1], 0);
+      if (e != cudaSuccess)
+        st = cuda_fail(e, "rotation download");
+      else
+        st = down.open(c);
+    }
+    if (st == SKGEMM_OK) st = down.finish();
   }
   cudaStreamSynchronize(si);
   cudaStreamSynchronize(sc);
