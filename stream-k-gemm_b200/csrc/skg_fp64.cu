@@ -1,6 +1,7 @@
 // Host launcher of the native FP64 Stream-K kernel: operand descriptors ->
 // TMA tensor maps, Stream-K schedule, cooperative persistent launch.
 #include <algorithm>
+#include <cmath>
 
 #include "skg_fp64_kernel.cuh"
 #include "skg_runtime.h"
@@ -51,6 +52,28 @@ struct Schedule {
   int grid;
 };
 
+// Persistent CTAs of a single-problem launch: every resident CTA, fewer where that
+// cuts tiles into more parts than their sum pays for. Measured (us, grid at full
+// occupancy / here):
+//  * half of the resident CTAs where a tile is in many parts and a CTA's share
+//    short: SYRK 10000 x 96 on 32 x 32 tiles 24 / 15, GEMM 32768 x 96 37 / 31,
+//    rotation 1008 x 256 15 / 13; SYRK 10000 x 128 on 64 x 64 22 / 21, GEMM 23 /
+//    19; equal from about 230 (32 x 32) and 60 iterations a CTA (64 x 64), where
+//    the multiplications want all of them. 64 x 64 tiles in fewer than eight
+//    parts are not cut evenly enough by half (dense 1000^3 72 / 80).
+//  * at most sqrt(14 iterations) parts a tile: an iteration costs about as much
+//    as the sums of 14 parts in the fix-up. SYRK 10000 x 32 17 / 11 (94 parts
+//    instead of 592), 32768 x 32 25 / 14.
+int schedule_grid(DeviceState* dev, const Schedule& sc, int tile, int per_sm) {
+  const int64_t full = (int64_t)dev->num_sms * per_sm;
+  int64_t g = std::min(full, sc.total);
+  if ((tile == 32 && sc.num_tiles < full && sc.total < 230 * full) ||
+      (tile == 64 && 8 * (int64_t)sc.num_tiles <= full && sc.total < 60 * full))
+    g = std::min(g, full / 2);
+  const int64_t parts = (int64_t)std::ceil(std::sqrt(14.0 * sc.ipt));
+  return (int)std::max<int64_t>(1, std::min(g, sc.num_tiles * parts));
+}
+
 Schedule make_schedule(DeviceState* dev, const Fp64Problem& prob, int tile, int per_sm) {
   Schedule sc;
   sc.tiles_m = (int)((prob.M + tile - 1) / tile);
@@ -59,7 +82,7 @@ Schedule make_schedule(DeviceState* dev, const Fp64Problem& prob, int tile, int 
                                                 : sc.tiles_m * sc.tiles_n;
   sc.ipt = (int)((prob.K + kBK - 1) / kBK);
   sc.total = (int64_t)sc.num_tiles * sc.ipt;
-  sc.grid = (int)std::min<int64_t>((int64_t)dev->num_sms * per_sm, sc.total);
+  sc.grid = schedule_grid(dev, sc, tile, per_sm);
   return sc;
 }
 
