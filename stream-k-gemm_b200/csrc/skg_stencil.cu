@@ -30,50 +30,91 @@ struct StencilCoef {
   double c0;
 };
 
-// CTA = one 4-band slab (bands 4 q ..
-// 4 q + 3: one 32-byte sector per point) of a 16 x 16 column tile, marching
-// k through [k0, k1). A producer warp streams, by TMA, one stage per k step
-// into a ring of kStRing shared-memory stages, kStRing - 1 steps ahead:
-//   the tile's plane k with its x / y halo, 28 x 28 points x 4 bands;
-//   the tile's 16 x 16 points of plane k + 6 (the z queue's new entry);
-//   A[g] of the tile's 16 x 16 points of plane k: one 2-D box when ni is
-//   even (A viewed as [nj nk][ni]: 16-byte row strides), else one 18-double
-//   box per row from an even index, in a 256-byte slot.
+// Tile = one 8-band slab (bands 8 q .. 8 q + 7: 64 bytes per point) of 16 x 8
+// columns. One CTA per SM takes whole tiles, nk planes each, and then an even
+// share of the planes that are left (StWork). A producer warp streams one stage
+// per plane k into a ring of kStRing shared-memory stages, on through the tiles:
+//   the tile's plane k with its x / y halo, 28 x 20 points x 8 bands, by TMA;
+//   the tile's 16 x 8 points of plane k + 6 (the z queue's new entry), by TMA;
+//   A[g] of the tile's points of plane k, by 8-byte asynchronous copies (a row
+//   of A starts at any multiple of 8 bytes).
+// A piece begins with kStFills stages that hold planes k0 - 6 .. k0 + 5 for the
+// queues, so that they too are loaded while the piece before is computed.
 // Consumer thread = two columns (i, j) and (i, j + 1) and a band pair: a
-// quarter-warp reads 4 consecutive points (128 contiguous bytes); the 14
+// quarter-warp reads 2 consecutive points (128 contiguous bytes); the 14
 // staged values j - 6 .. j + 7 serve the y neighbours of both columns; the
 // 12 z neighbours come from the columns' 13-slot register queues (slot of
 // plane k + d at step u of a 13-step period: (u + d + 6) mod 13). No global
 // load waits inside the k loop. Same arithmetic in the same order as the
 // reference kernels: the output equals theirs bit for bit. Every wait is
 // bounded; on expiry the CTA records the error and skips the remaining waits.
+//
+// Bound by the shared-memory pipe: 20 16-byte loads per column and band pair
+// and the stage itself are 1.7 kcycles of it per plane (335 us of 48^3 x 512's
+// 351 us). TMA moves one box row per 1.3 cycles whatever its length, so the
+// 32-byte rows of a 4-band slab on 16 x 16 columns took 297 us without any
+// arithmetic against 225 us for these 64-byte rows (400 us and 351 us in all).
+// Whole launches, one CTA per tile with its queues loaded at its start, 4-band
+// slabs -> this: 48^3 x 512 400 -> 351 us, 33 x 35 x 41 x 512 362 -> 243 us,
+// 56^3 x 318 475 -> 394 us, 48^3 x 72 86 -> 60 us, 24^3 x 24 31 -> 15 us.
+// Five stages took 353 us.
 constexpr int kStI = 16;                 // columns per CTA along x
-constexpr int kStJ = 16;                 // columns per CTA along y
-constexpr int kSlab = 4;                 // bands per CTA
+constexpr int kStJ = 8;                  // columns per CTA along y
+constexpr int kSlab = 8;                 // bands per CTA
+constexpr int kBP = kSlab / 2;           // band pairs
 constexpr int kStHI = kStI + 2 * kFDn;   // staged points along x
 constexpr int kStHJ = kStJ + 2 * kFDn;   // staged points along y
-constexpr int kStARow = 18;              // doubles per A box (from an even index)
-constexpr int kStAPitch = 32;            // doubles between staged A rows (TMA
-                                         // destinations are 128-byte aligned)
 constexpr int kStPlane = kStHI * kStHJ * kSlab;  // doubles: halo plane
 constexpr int kStCenter = kStI * kStJ * kSlab;   // doubles: plane k + 6
-constexpr int kStStage = kStPlane + kStCenter + kStJ * kStAPitch;  // doubles per stage
+constexpr int kStA = kStI * kStJ;                // doubles: A of plane k
+constexpr int kStStage = kStPlane + kStCenter + kStA;  // doubles per stage
 constexpr int kStRing = 4;
-constexpr int kStConsumerWarps = kStJ / 2;
+constexpr int kStConsumerWarps = kStI * kStJ * kSlab / 128;  // 4 outputs a thread
 constexpr int kStThreads = (kStConsumerWarps + 1) * 32;
-constexpr int kStTxBytes2d = (kStPlane + kStCenter + kStJ * kStI) * 8;
-constexpr int kStTxBytesRows = (kStPlane + kStCenter + kStJ * kStARow) * 8;
+constexpr int kStFill = 4;               // planes of a queue-filling stage
+constexpr int kStFills = 2 * kFDn / kStFill;
+constexpr int kStTxBytes = (kStPlane + kStCenter) * 8;
+constexpr int kStMinSteps = 8;           // planes a CTA should have at least: each piece
+                                         // costs 12 planes' queue entries on top
 constexpr int kStSmem = kStRing * kStStage * 8 + 2 * kStRing * 8 + 16 + 128;
 static_assert((kStPlane * 8) % 128 == 0 && (kStCenter * 8) % 128 == 0, "stage alignment");
-static_assert((kStStage * 8) % 128 == 0 && (kStAPitch * 8) % 128 == 0, "stage alignment");
-static_assert((kStARow * 8) % 16 == 0 && kStARow <= kStAPitch, "A box");
+static_assert((kStStage * 8) % 128 == 0 && (2 * kFDn) % kStFill == 0, "stage layout");
+static_assert(kStFill * kStCenter <= kStStage, "queue-filling stage");
 static_assert(kStSmem <= 232448, "stencil stages exceed 227 KB of shared memory");
+
+// Arrives at a barrier once all this thread's asynchronous copies have landed.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// The work of one CTA: tiles c, c + G, .. of the full waves, then its share of
+// the remaining tiles' planes, cut evenly over all G CTAs (a share is shorter
+// than a tile's nk planes: at most two pieces).
+struct StWork {
+  int waves, first, ka, len;  // whole tiles; the share's first tile, first plane and planes
+};
+// Piece n: its tile and planes [k0, k1); false when there is none.
+__device__ __forceinline__ bool st_piece(const volatile StWork* w, int n, int nk, int* tile, int* k0,
+                                         int* k1) {
+  const int m = n - w->waves;
+  if (m < 0) {
+    *tile = blockIdx.x + n * gridDim.x;
+    *k0 = 0;
+    *k1 = nk;
+    return true;
+  }
+  const int end = w->ka + w->len - m * nk;  // the share's end, from this tile's plane 0
+  *tile = w->first + m;
+  *k0 = m == 0 ? w->ka : 0;
+  *k1 = min(nk, end);
+  return w->len > 0 && end > 0;
+}
 
 template <int OT>
 __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
     const __grid_constant__ CUtensorMap mapP, const __grid_constant__ CUtensorMap mapC,
-    const __grid_constant__ CUtensorMap mapA, bool a2d, int ni, int nj, int nk, int nb, int kc,
-    const double* __restrict__ ext, const __grid_constant__ StencilCoef cf,
+    const __grid_constant__ CUtensorMap mapF, int ni, int nj, int nk, int nb, int tiles,
+    const double* __restrict__ A, const __grid_constant__ StencilCoef cf,
     double* __restrict__ out, uint32_t* __restrict__ err) {
   extern __shared__ uint8_t sraw[];
   double* stages =
@@ -82,19 +123,21 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
   uint64_t* empty = full + kStRing;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kStRing);
   const int itiles = (ni + kStI - 1) / kStI;
-  const int i0 = (int)(blockIdx.x % itiles) * kStI, j0 = (int)(blockIdx.x / itiles) * kStJ;
-  const int q = blockIdx.y;  // slab: bands 4 q .. 4 q + 3
-  const int t = q / (16 / kSlab), sl = q % (16 / kSlab);
-  const int k0 = blockIdx.z * kc;
-  const int k1 = min(nk, k0 + kc);
-  if (q * kSlab >= nb || k0 >= k1) return;
-  const int nsteps = k1 - k0;
-  const int64_t nix = ni + 2 * kFDn, njx = nj + 2 * kFDn, nkx = nk + 2 * kFDn;
+  const int64_t nkx = nk + 2 * kFDn;
   const int64_t plane_pts = (int64_t)ni * nj;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cols = itiles * ((nj + kStJ - 1) / kStJ);
+  __shared__ StWork work;
   if (threadIdx.x == 0) {
+    const int G = gridDim.x, full_tiles = tiles / G * G;
+    const int64_t rest = (int64_t)(tiles - full_tiles) * nk;
+    const int lo = (int)(blockIdx.x * rest / G), hi = (int)((blockIdx.x + 1) * rest / G);
+    work.waves = tiles / G;
+    work.first = full_tiles + lo / nk;
+    work.ka = lo % nk;
+    work.len = hi - lo;
     for (int b = 0; b < kStRing; ++b) {
-      mbar_init(&full[b], 1);
+      mbar_init(&full[b], 33);  // the TMA loads and 32 lanes' copies of A
       mbar_init(&empty[b], kStConsumerWarps);
     }
     *abort_flag = 0;
@@ -102,131 +145,155 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
   }
   __syncthreads();
 
+  int tile, k0, k1;
   if (warp == kStConsumerWarps) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
       tma_prefetch_desc(&mapP);
       tma_prefetch_desc(&mapC);
-      tma_prefetch_desc(&mapA);
-      int issued = 0;
-      for (int u = 0; u < nsteps; ++u) {
-        const int b = u % kStRing;
-        if (u >= kStRing) {
-          if (*abort_flag || !mbar_wait(&empty[b], ((u / kStRing) - 1) & 1, err)) {
-            *abort_flag = 1;
-            break;
-          }
-        }
-        const int k = k0 + u;
-        double* st = stages + b * kStStage;
-        mbar_arrive_expect_tx(&full[b], a2d ? kStTxBytes2d : kStTxBytesRows);
-        tma_load_4d(st, &mapP, &full[b], sl * kSlab, i0, j0, (int)(t * nkx + k + kFDn));
-        tma_load_4d(st + kStPlane, &mapC, &full[b], sl * kSlab, i0 + kFDn, j0 + kFDn,
-                    (int)(t * nkx + k + 2 * kFDn));
-        if (a2d) {
-          tma_load_2d(st + kStPlane + kStCenter, &mapA, &full[b], i0, j0 + k * nj);
-        } else {
-          for (int jj = 0; jj < kStJ; ++jj) {
-            const int64_t g = (int64_t)i0 + (int64_t)(j0 + jj) * ni + (int64_t)k * plane_pts;
-            tma_load_1d(st + kStPlane + kStCenter + jj * kStAPitch, &mapA, &full[b],
-                        (int)(g & ~1LL));
-          }
-        }
-        ++issued;
-      }
-      // The CTA leaves only after its last loads have landed (immediate on
-      // the normal path: the consumers waited for every one of them).
-      for (int u = issued - 1; u >= 0 && u >= issued - kStRing; --u)
-        mbar_wait(&full[u % kStRing], (u / kStRing) & 1, err);
+      tma_prefetch_desc(&mapF);
     }
+    uint32_t it = 0;
+    bool ok = true;
+    for (int n = 0; ok && st_piece(&work, n, nk, &tile, &k0, &k1); ++n) {
+      const int col = tile % cols, q = tile / cols;
+      const int i0 = col % itiles * kStI, j0 = col / itiles * kStJ;
+      const int t = q / (16 / kSlab), b0 = q % (16 / kSlab) * kSlab;
+      const int jl = lane / kStI, i = i0 + lane % kStI;
+      const double* Ak = A + i + (int64_t)(j0 + jl) * ni + k0 * plane_pts;
+      for (int u = -kStFills; u < k1 - k0; ++u, ++it) {
+        const uint32_t b = it % kStRing;
+        if (it >= kStRing && (*abort_flag || !mbar_wait(&empty[b], (it / kStRing - 1) & 1, err)))
+          ok = false;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          *abort_flag = 1;
+          break;
+        }
+        double* st = stages + b * kStStage;
+        if (u < 0) {  // planes k0 - 6 .. k0 + 5 for the queues, kStFill a stage
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&full[b], kStFill * kStCenter * 8);
+            tma_load_4d(st, &mapF, &full[b], b0, i0 + kFDn, j0 + kFDn,
+                        (int)(t * nkx + k0 + (u + kStFills) * kStFill));
+          }
+        } else {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&full[b], kStTxBytes);
+            tma_load_4d(st, &mapP, &full[b], b0, i0, j0, (int)(t * nkx + k0 + u + kFDn));
+            tma_load_4d(st + kStPlane, &mapC, &full[b], b0, i0 + kFDn, j0 + kFDn,
+                        (int)(t * nkx + k0 + u + 2 * kFDn));
+          }
+          double* As = st + kStPlane + kStCenter + lane;
+#pragma unroll
+          for (int m = 0; m < kStJ; m += 32 / kStI)
+            if (i < ni && j0 + jl + m < nj) cp_async8(As + m * kStI, Ak + (int64_t)m * ni, 8);
+          Ak += plane_pts;
+        }
+        cp_async_arrive(&full[b]);
+      }
+    }
+    // The CTA leaves only after its last loads have landed (immediate on
+    // the normal path: the consumers waited for every one of them).
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (uint32_t v = it > kStRing ? it - kStRing : 0; v < it; ++v)
+      mbar_wait(&full[v % kStRing], (v / kStRing) & 1, err);
     return;
   }
 
   // -------------------------------------------------------------- consumers
-  const int bp = lane & 1;
-  const int il = lane >> 1;
-  const int jA = 2 * warp;  // tile rows jA, jA + 1
-  const int i = i0 + il, j = j0 + jA;
-  const int b = q * kSlab + 2 * bp;
-  const bool actA = i < ni && j < nj && b < nb;
-  const bool actB = i < ni && j + 1 < nj && b < nb;
-  const int64_t sk = nix * njx * 8;  // z stride in lane pairs
-  const int64_t K = plane_pts * nk;
-  const double2* baseA =
-      reinterpret_cast<const double2*>(ext) +
-      ((int64_t)t * nix * njx * nkx + (i + kFDn) + (int64_t)(j + kFDn) * nix) * 8 + sl * 2 + bp;
-  const double2* baseB = baseA + nix * 8;
-  double2 zqA[kZq], zqB[kZq];
-#pragma unroll
-  for (int d = -kFDn; d < kFDn; ++d) {  // prologue: planes k0 - 6 .. k0 + 5
-    zqA[d + kFDn] = actA ? __ldg(baseA + (int64_t)(k0 + d + kFDn) * sk) : make_double2(0.0, 0.0);
-    zqB[d + kFDn] = actB ? __ldg(baseB + (int64_t)(k0 + d + kFDn) * sk) : make_double2(0.0, 0.0);
-  }
+  const int bp = lane % kBP;
+  const int il = warp % (kStI * kBP / 32) * (32 / kBP) + lane / kBP;
+  const int jA = warp / (kStI * kBP / 32) * 2;  // tile rows jA, jA + 1
   // Lane pair (il, row) offsets in a stage, in double2 units.
-  const int pA = ((jA + kFDn) * kStHI + il + kFDn) * 2 + bp;  // halo plane, row jA
-  const int yA = (jA * kStHI + il + kFDn) * 2 + bp;            // halo plane, row jA - 6
-  const int cA = ((jA * kStI) + il) * 2 + bp;                   // center box, row jA
-  for (int kb = k0; kb < k1; kb += kZq) {
+  const int pA = ((jA + kFDn) * kStHI + il + kFDn) * kBP + bp;  // halo plane, row jA
+  const int yA = (jA * kStHI + il + kFDn) * kBP + bp;            // halo plane, row jA - 6
+  const int cA = (jA * kStI + il) * kBP + bp;                     // center box, row jA
+  const int64_t K = plane_pts * nk;
+  uint32_t buf = 0, ph = 0;
+  for (int n = 0; st_piece(&work, n, nk, &tile, &k0, &k1); ++n) {
+    const int col = tile % cols, q = tile / cols;
+    const int i = col % itiles * kStI + il, j = col / itiles * kStJ + jA;
+    const int b = q * kSlab + 2 * bp;
+    const bool actA = i < ni && j < nj && b < nb;
+    const bool actB = i < ni && j + 1 < nj && b < nb;
+    double2 zqA[kZq], zqB[kZq];
 #pragma unroll
-    for (int u = 0; u < kZq; ++u) {
-      const int k = kb + u;
-      if (k >= k1) break;
-      const int step = k - k0, buf = step % kStRing;
-      if (!*abort_flag && !mbar_wait(&full[buf], (step / kStRing) & 1, err)) *abort_flag = 1;
-      const double* st = stages + buf * kStStage;
-      const double2* P = reinterpret_cast<const double2*>(st);
-      const double2* C = reinterpret_cast<const double2*>(st + kStPlane);
-      const double* As = st + kStPlane + kStCenter;
-      zqA[(u + 2 * kFDn) % kZq] = C[cA];
-      zqB[(u + 2 * kFDn) % kZq] = C[cA + kStI * 2];
-      if (actA) {
-        const int64_t g = (int64_t)i + (int64_t)j * ni + (int64_t)k * plane_pts;
-        const int64_t gr = g - il;  // row start
-        const int64_t grB = gr + ni;
-        const double aA = (a2d ? As[jA * kStI + il] : As[jA * kStAPitch + (int)(gr & 1) + il]) +
-                          cf.c0;
-        const double aB = (a2d ? As[(jA + 1) * kStI + il]
-                               : As[(jA + 1) * kStAPitch + (int)(grB & 1) + il]) + cf.c0;
-        double2 Y[2 * kFDn + 2];  // rows jA - 6 .. jA + 7
+    for (int f = 0; f < kStFills; ++f) {  // planes k0 - 6 .. k0 + 5
+      if (!*abort_flag && !mbar_wait(&full[buf], ph, err)) *abort_flag = 1;
+      const double2* C = reinterpret_cast<const double2*>(stages + buf * kStStage);
 #pragma unroll
-        for (int d = 0; d < 2 * kFDn + 2; ++d) Y[d] = P[yA + d * kStHI * 2];
-        const double2 ca = zqA[(u + kFDn) % kZq], cb = zqB[(u + kFDn) % kZq];
-        double a0 = ca.x * aA, a1 = ca.y * aA;
-        double b0 = cb.x * aB, b1 = cb.y * aB;
-#pragma unroll
-        for (int r = 1; r <= kFDn; ++r) {
-          const double2 xpA = P[pA + 2 * r], xmA = P[pA - 2 * r];
-          const double2 xpB = P[pA + 2 * kStHI + 2 * r], xmB = P[pA + 2 * kStHI - 2 * r];
-          a0 = fma(xpA.x + xmA.x, cf.cx[r], a0);
-          a1 = fma(xpA.y + xmA.y, cf.cx[r], a1);
-          b0 = fma(xpB.x + xmB.x, cf.cx[r], b0);
-          b1 = fma(xpB.y + xmB.y, cf.cx[r], b1);
-          a0 = fma(Y[kFDn + r].x + Y[kFDn - r].x, cf.cy[r], a0);
-          a1 = fma(Y[kFDn + r].y + Y[kFDn - r].y, cf.cy[r], a1);
-          b0 = fma(Y[kFDn + 1 + r].x + Y[kFDn + 1 - r].x, cf.cy[r], b0);
-          b1 = fma(Y[kFDn + 1 + r].y + Y[kFDn + 1 - r].y, cf.cy[r], b1);
-          const double2 zpA = zqA[(u + kFDn + r) % kZq], zmA = zqA[(u + kFDn - r + kZq) % kZq];
-          const double2 zpB = zqB[(u + kFDn + r) % kZq], zmB = zqB[(u + kFDn - r + kZq) % kZq];
-          a0 = fma(zpA.x + zmA.x, cf.cz[r], a0);
-          a1 = fma(zpA.y + zmA.y, cf.cz[r], a1);
-          b0 = fma(zpB.x + zmB.x, cf.cz[r], b0);
-          b1 = fma(zpB.y + zmB.y, cf.cz[r], b1);
-        }
-        double* o = out + ((int64_t)(b / OT) * K + g) * OT + b % OT;
-        if (b + 1 < nb)
-          *reinterpret_cast<double2*>(o) = make_double2(a0, a1);
-        else
-          o[0] = a0;  // lane b + 1 is padding: left untouched
-        if (actB) {
-          double* o2 = o + (int64_t)ni * OT;
-          if (b + 1 < nb)
-            *reinterpret_cast<double2*>(o2) = make_double2(b0, b1);
-          else
-            o2[0] = b0;
-        }
+      for (int d = 0; d < kStFill; ++d) {
+        zqA[f * kStFill + d] = C[d * (kStCenter / 2) + cA];
+        zqB[f * kStFill + d] = C[d * (kStCenter / 2) + cA + kStI * kBP];
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[buf]);
+      if (++buf == kStRing) {
+        buf = 0;
+        ph ^= 1;
+      }
+    }
+    double* o = out + ((int64_t)(b / OT) * K + i + (int64_t)j * ni + k0 * plane_pts) * OT + b % OT;
+    for (int kb = k0; kb < k1; kb += kZq) {
+#pragma unroll
+      for (int u = 0; u < kZq; ++u) {
+        if (kb + u >= k1) break;
+          if (!*abort_flag && !mbar_wait(&full[buf], ph, err)) *abort_flag = 1;
+        const double* st = stages + buf * kStStage;
+        const double2* P = reinterpret_cast<const double2*>(st);
+        const double2* C = reinterpret_cast<const double2*>(st + kStPlane);
+        const double* As = st + kStPlane + kStCenter + jA * kStI + il;
+        zqA[(u + 2 * kFDn) % kZq] = C[cA];
+        zqB[(u + 2 * kFDn) % kZq] = C[cA + kStI * kBP];
+        if (actA) {
+          const double aA = As[0] + cf.c0;
+          const double aB = As[kStI] + cf.c0;
+          double2 Y[2 * kFDn + 2];  // rows jA - 6 .. jA + 7
+#pragma unroll
+          for (int d = 0; d < 2 * kFDn + 2; ++d) Y[d] = P[yA + d * kStHI * kBP];
+          const double2 ca = zqA[(u + kFDn) % kZq], cb = zqB[(u + kFDn) % kZq];
+          double a0 = ca.x * aA, a1 = ca.y * aA;
+          double b0 = cb.x * aB, b1 = cb.y * aB;
+#pragma unroll
+          for (int r = 1; r <= kFDn; ++r) {
+            const double2 xpA = P[pA + kBP * r], xmA = P[pA - kBP * r];
+            const double2 xpB = P[pA + kBP * (kStHI + r)], xmB = P[pA + kBP * (kStHI - r)];
+            a0 = fma(xpA.x + xmA.x, cf.cx[r], a0);
+            a1 = fma(xpA.y + xmA.y, cf.cx[r], a1);
+            b0 = fma(xpB.x + xmB.x, cf.cx[r], b0);
+            b1 = fma(xpB.y + xmB.y, cf.cx[r], b1);
+            a0 = fma(Y[kFDn + r].x + Y[kFDn - r].x, cf.cy[r], a0);
+            a1 = fma(Y[kFDn + r].y + Y[kFDn - r].y, cf.cy[r], a1);
+            b0 = fma(Y[kFDn + 1 + r].x + Y[kFDn + 1 - r].x, cf.cy[r], b0);
+            b1 = fma(Y[kFDn + 1 + r].y + Y[kFDn + 1 - r].y, cf.cy[r], b1);
+            const double2 zpA = zqA[(u + kFDn + r) % kZq], zmA = zqA[(u + kFDn - r + kZq) % kZq];
+            const double2 zpB = zqB[(u + kFDn + r) % kZq], zmB = zqB[(u + kFDn - r + kZq) % kZq];
+            a0 = fma(zpA.x + zmA.x, cf.cz[r], a0);
+            a1 = fma(zpA.y + zmA.y, cf.cz[r], a1);
+            b0 = fma(zpB.x + zmB.x, cf.cz[r], b0);
+            b1 = fma(zpB.y + zmB.y, cf.cz[r], b1);
+          }
+          if (b + 1 < nb)
+            *reinterpret_cast<double2*>(o) = make_double2(a0, a1);
+          else
+            o[0] = a0;  // lane b + 1 is padding: left untouched
+          if (actB) {
+            double* o2 = o + (int64_t)ni * OT;
+            if (b + 1 < nb)
+              *reinterpret_cast<double2*>(o2) = make_double2(b0, b1);
+            else
+              o2[0] = b0;
+          }
+        }
+        o += plane_pts * OT;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[buf]);
+        if (++buf == kStRing) {
+          buf = 0;
+          ph ^= 1;
+        }
+      }
     }
   }
 }
@@ -259,8 +326,8 @@ __global__ void __launch_bounds__(256) halo_periodic_kernel(int ni, int nj, int 
 namespace {
 
 template <int OT>
-int launch_staged(const CUtensorMap& mapP, const CUtensorMap& mapC, const CUtensorMap& mapA,
-                  bool a2d, int ni, int nj, int nk, int nb, int kc, dim3 grid, const double* ext,
+int launch_staged(const CUtensorMap& mapP, const CUtensorMap& mapC, const CUtensorMap& mapF, int ni,
+                  int nj, int nk, int nb, int tiles, int grid, const double* A,
                   const StencilCoef& cf, double* out, uint32_t* err, cudaStream_t s) {
   static bool attr_set[64] = {};  // function attributes are per device
   int d = 0;
@@ -272,8 +339,8 @@ int launch_staged(const CUtensorMap& mapP, const CUtensorMap& mapC, const CUtens
     attr_set[d] = true;
   }
   KernelTimer kt_(s, "stencil_staged_kernel");
-  stencil_staged_kernel<OT><<<grid, kStThreads, kStSmem, s>>>(mapP, mapC, mapA, a2d, ni, nj, nk,
-                                                              nb, kc, ext, cf, out, err);
+  stencil_staged_kernel<OT><<<grid, kStThreads, kStSmem, s>>>(mapP, mapC, mapF, ni, nj, nk, nb,
+                                                              tiles, A, cf, out, err);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
 }
@@ -305,43 +372,35 @@ int launch_stencil_ext(int64_t ni, int64_t nj, int64_t nk, int64_t nb, int FDn,
     return fail(SKGEMM_ERR_INVALID_ARG, "stencil A_diag must be 16-byte aligned");
   const int64_t cols = ((ni + kStI - 1) / kStI) * ((nj + kStJ - 1) / kStJ);
   const int64_t tiles = (nb + 15) / 16;
-  const int64_t slabs = tiles * (16 / kSlab);
-  if (cols > INT32_MAX || slabs > 65535) return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
+  if (cols > INT32_MAX || tiles > 16383) return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
   const int64_t nix = ni + 2 * kFDn, njx = nj + 2 * kFDn, nkx = nk + 2 * kFDn;
   if (tiles * nkx > INT32_MAX || ni * nj * nk + 2 >= INT32_MAX)
     return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
   // Extended Psi as a 4-D tensor [tiles * nkx][njx][nix][16 lanes]: boxes of
-  // 4 lanes x 28 x 28 points (halo planes) and 4 lanes x 16 x 16 points (z
-  // entries); A as a 1-D tensor, boxes of 18 doubles. Zero fill outside.
-  CUtensorMap mapP, mapC, mapA;
+  // 8 lanes x 28 x 20 points (halo planes), 8 lanes x 16 x 8 points (z
+  // entries) and 4 such planes (filling the z queues). Zero fill outside.
+  CUtensorMap mapP, mapC, mapF;
   const uint64_t dims[4] = {16, (uint64_t)nix, (uint64_t)njx, (uint64_t)(tiles * nkx)};
   const uint64_t strides[3] = {16 * 8, (uint64_t)nix * 16 * 8, (uint64_t)(nix * njx) * 16 * 8};
   const uint32_t boxP[4] = {(uint32_t)kSlab, (uint32_t)kStHI, (uint32_t)kStHJ, 1};
   const uint32_t boxC[4] = {(uint32_t)kSlab, (uint32_t)kStI, (uint32_t)kStJ, 1};
-  // A: [nj nk][ni] with 16 x 16 boxes when its rows are 16-byte strided,
-  // else 1-D with 18-double boxes.
-  const bool a2d = ni % 2 == 0;
-  const uint64_t dimsA[2] = {a2d ? (uint64_t)ni : (uint64_t)(ni * nj * nk), (uint64_t)(nj * nk)};
-  const uint64_t stridesA[1] = {(uint64_t)ni * 8};
-  const uint32_t boxA[2] = {a2d ? (uint32_t)kStI : (uint32_t)kStARow, (uint32_t)kStJ};
+  const uint32_t boxF[4] = {(uint32_t)kSlab, (uint32_t)kStI, (uint32_t)kStJ, (uint32_t)kStFill};
   int st;
   if ((st = encode_tiled(&mapP, 4, ext, dims, strides, boxP, CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          CU_TENSOR_MAP_SWIZZLE_NONE)) ||
       (st = encode_tiled(&mapC, 4, ext, dims, strides, boxC, CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          CU_TENSOR_MAP_SWIZZLE_NONE)) ||
-      (st = encode_tiled(&mapA, a2d ? 2 : 1, A, dimsA, stridesA, boxA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+      (st = encode_tiled(&mapF, 4, ext, dims, strides, boxF, CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          CU_TENSOR_MAP_SWIZZLE_NONE)))
     return st;
-  // Split k only when the column tiles and slabs alone give fewer than four
-  // CTAs per SM; each chunk reloads 12 planes per column.
-  int64_t chunks = 1;
-  while (cols * slabs * chunks < 4LL * num_sms && nk / (chunks * 2) >= 16) chunks *= 2;
-  const int kc = (int)((nk + chunks - 1) / chunks);
-  const dim3 grid((unsigned)cols, (unsigned)slabs, (unsigned)((nk + kc - 1) / kc));
+  // One CTA per SM; slabs past nb have no work.
+  const int64_t work = cols * ((nb + kSlab - 1) / kSlab);
+  if (work > INT32_MAX) return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
+  const int grid = (int)std::min<int64_t>(num_sms, std::max<int64_t>(1, work * nk / kStMinSteps));
   if (out_tile == 32)
-    return launch_staged<32>(mapP, mapC, mapA, a2d, (int)ni, (int)nj, (int)nk, (int)nb, kc, grid, ext,
+    return launch_staged<32>(mapP, mapC, mapF, (int)ni, (int)nj, (int)nk, (int)nb, (int)work, grid, A,
                              cf, out, err, s);
-  return launch_staged<16>(mapP, mapC, mapA, a2d, (int)ni, (int)nj, (int)nk, (int)nb, kc, grid, ext,
+  return launch_staged<16>(mapP, mapC, mapF, (int)ni, (int)nj, (int)nk, (int)nb, (int)work, grid, A,
                            cf, out, err, s);
 }
 

@@ -34,6 +34,28 @@ def test_stencil_equals_oracle(cuda, ni, nj, nk, nb, T):
     assert np.isnan(got[lanes >= nb]).all()  # padding lanes untouched
 
 
+@pytest.mark.parametrize("ni,nj,nk,nb", [
+    (1, 1, 1, 1),          # one point, one band
+    (15, 7, 2, 7),         # below one tile, fewer planes than a queue
+    (17, 9, 13, 9),        # one past the tile and the slab on every axis
+    (16, 8, 40, 8),        # one tile: its planes shared out over CTAs
+    (31, 25, 14, 23),      # odd rows of A, shares across tile boundaries
+    (33, 17, 11, 200),     # more tiles than CTAs: whole waves and shares
+])
+def test_stencil_tiles_and_shares(cuda, ni, nj, nk, nb):
+    """Tile and slab edges and the split of planes over CTAs; equal bits."""
+    _, A, ext = extended_case(ni, nj, nk, nb, 3 * ni + nb)
+    K, T = ni * nj * nk, 32
+    out = torch.full(((nb + T - 1) // T * K * T,), np.nan, dtype=torch.float64, device="cuda")
+    skgemm.stencil_ext_dev(ni, nj, nk, nb, dev(ext), dev(A), CX, CX, CX, C0, out, T)
+    skgemm.stream_status()
+    want = oracle.stencil_ext(ext, A, ni, nj, nk, nb, CX, CX, CX, C0, T, threads=oracle.nthreads())
+    got = out.cpu().numpy()
+    lanes = np.arange(got.size) % T + (np.arange(got.size) // (K * T)) * T
+    assert np.array_equal(got[lanes < nb], want[lanes < nb])
+    assert np.isnan(got[lanes >= nb]).all()
+
+
 def test_halo_periodic_equals_oracle(cuda):
     ni, nj, nk, nb = 24, 20, 16, 40
     rng = np.random.default_rng(11)
