@@ -298,14 +298,24 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
   }
 }
 
-// One CTA per extended row (tile t, k_ex, j_ex): ext[(t K_ex + g_ex) 16 + l] =
-// local[(t K + g) 16 + l], g the periodic image of g_ex's interior point;
-// 16-byte lane pairs (the copy is bound by its index arithmetic).
-__global__ void __launch_bounds__(256) halo_periodic_kernel(int ni, int nj, int nk, int FDn,
-                                                            const double* __restrict__ local,
-                                                            double* __restrict__ ext) {
+// One warp per extended row (tile t, k_ex, j_ex): ext[(t K_ex + g_ex) 16 + l] =
+// local[(t K + g) 16 + l], g the periodic image of g_ex's interior point; 16-byte
+// lane pairs. Bound by memory once enough of it is asked for: kHaloLoads loads
+// stand before the first store (a 48-point row with its halo at once), and the
+// stores stream past L2. One 256-thread CTA per row, a load and a store at a time
+// -> this: 48^3 x 506 229 -> 199 us (6.7 TB/s, a plain copy's rate), 24^3 x 512
+// 64 -> 42 us, 48^3 x 72 40 -> 35 us. 4 loads in 8 warps: 204, 42 and 36 us; 8
+// loads took 260 us (48^3 rows end in a nearly empty second round); without the
+// streaming hint 234 us.
+constexpr int kHaloLoads = 15;
+constexpr int kHaloWarps = 4;
+__global__ void __launch_bounds__(kHaloWarps * 32) halo_periodic_kernel(
+    int64_t rows, int ni, int nj, int nk, int FDn, const double* __restrict__ local,
+    double* __restrict__ ext) {
   const int64_t nix = ni + 2 * FDn, njx = nj + 2 * FDn, nkx = nk + 2 * FDn;
-  const int64_t row = blockIdx.x;  // (t * nkx + kx) * njx + jx
+  // row = (t * nkx + kx) * njx + jx
+  const int64_t row = (int64_t)blockIdx.x * kHaloWarps + (threadIdx.x >> 5);
+  if (row >= rows) return;
   const int64_t jx = row % njx, kx = (row / njx) % nkx, t = row / (njx * nkx);
   int jl = (int)jx - FDn, kl = (int)kx - FDn;
   jl += jl < 0 ? nj : (jl >= nj ? -nj : 0);
@@ -314,10 +324,19 @@ __global__ void __launch_bounds__(256) halo_periodic_kernel(int ni, int nj, int 
   const double2* src = reinterpret_cast<const double2*>(local) +
                        (t * K + (int64_t)jl * ni + (int64_t)kl * ni * nj) * 8;
   double2* dst = reinterpret_cast<double2*>(ext) + row * nix * 8;
-  for (int e = threadIdx.x; e < (int)nix * 8; e += blockDim.x) {
-    int il = (e >> 3) - FDn;
-    il += il < 0 ? ni : (il >= ni ? -ni : 0);
-    dst[e] = src[il * 8 + (e & 7)];
+  const int n = (int)nix * 8;
+  for (int e0 = threadIdx.x & 31; e0 < n; e0 += 32 * kHaloLoads) {
+    double2 v[kHaloLoads];
+#pragma unroll
+    for (int x = 0; x < kHaloLoads; ++x) {
+      const int e = e0 + 32 * x;
+      int il = (e >> 3) - FDn;
+      il += il < 0 ? ni : (il >= ni ? -ni : 0);
+      if (e < n) v[x] = __ldg(src + il * 8 + (e & 7));
+    }
+#pragma unroll
+    for (int x = 0; x < kHaloLoads; ++x)
+      if (e0 + 32 * x < n) __stcs(dst + e0 + 32 * x, v[x]);
   }
 }
 
@@ -419,7 +438,8 @@ int launch_halo_periodic(int64_t ni, int64_t nj, int64_t nk, int64_t nb, int FDn
   const int64_t rows = ((nb + 15) / 16) * (nk + 2 * FDn) * (nj + 2 * FDn);
   if (rows > INT32_MAX) return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
   KernelTimer kt_(s, "halo_periodic_kernel");
-  halo_periodic_kernel<<<(unsigned)rows, 256, 0, s>>>((int)ni, (int)nj, (int)nk, FDn, local, ext);
+  halo_periodic_kernel<<<(unsigned)((rows + kHaloWarps - 1) / kHaloWarps), kHaloWarps * 32, 0, s>>>(
+      rows, (int)ni, (int)nj, (int)nk, FDn, local, ext);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
 }

@@ -66,6 +66,27 @@ def test_halo_periodic_equals_oracle(cuda):
     assert np.array_equal(ext.cpu().numpy(), oracle.halo_periodic(local, ni, nj, nk, nb))
 
 
+@pytest.mark.parametrize("ni,nj,nk,nb,FDn", [
+    (1, 1, 1, 1, 1),     # one point, every row a wrap
+    (6, 7, 6, 17, 6),    # halo as wide as the domain
+    (47, 3, 5, 16, 3),  # a row of 53 points: under one round of loads
+    (48, 6, 6, 16, 6),   # 60 points: one round exactly
+    (49, 6, 7, 33, 6),   # one point over
+    (130, 2, 3, 8, 2),   # three rounds
+    (5, 4, 3, 40, 0),    # no halo: a copy
+])
+def test_halo_rows(cuda, ni, nj, nk, nb, FDn):
+    """Row lengths around the loads a warp has in flight, and a row count that is
+    no multiple of the warps in a block."""
+    rng = np.random.default_rng(ni + nb)
+    local = rng.standard_normal((nb + 15) // 16 * ni * nj * nk * 16)
+    ext = torch.full((oracle.ext_size(ni, nj, nk, nb, FDn),), np.nan, dtype=torch.float64,
+                     device="cuda")
+    skgemm.halo_periodic_dev(ni, nj, nk, nb, dev(local), ext, FDn)
+    skgemm.stream_status()
+    assert np.array_equal(ext.cpu().numpy(), oracle.halo_periodic(local, ni, nj, nk, nb, FDn))
+
+
 def test_stencil_feeds_hs(cuda):
     """Psi (band-packed) -> periodic halo -> H Psi (32-band-packed) -> Hs =
     Psi^T H Psi with the GEMM, all on the device; against Dot2 of the oracle's
