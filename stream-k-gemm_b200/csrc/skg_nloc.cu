@@ -13,10 +13,10 @@
 // back-projection sums fused), so results equal it bit for bit:
 //  * nloc_forward_kernel: CTA per (block, 32 bands, 16 columns) — for each of
 //    the block's projectors in order, gathered psi rows staged in shared
-//    memory (double-buffered asynchronous copies), each (column, band) thread
-//    summing them in row order; then the block's gamma scalings in order;
+//    memory (asynchronous copies, chunks ahead), each thread summing its (column,
+//    band) products in row order; then the block's gamma scalings in order;
 //  * nloc_chi_c_kernel: the back-projection rows chi_p C_p of every projector
-//    (spans of 64-row tiles x 64 bands, C and chi staged in shared memory),
+//    (spans of 64-row tiles x 64 bands, C in registers, chi in shared memory),
 //    into a scratch of total rows x nb;
 //  * nloc_backward_kernel: thread per (touched grid point, band pair) — walks
 //    the point's (projector, row) entries in projector order (an inverse index
@@ -50,12 +50,11 @@ struct skgemm_nloc {
   // back-projection row tiles (projector, first row)
   int64_t ntiles = 0;
   int64_t *d_tile_proj = nullptr, *d_tile_r0 = nullptr;
-  int64_t total_rows = 0, max_cols = 0;
+  int64_t total_rows = 0;
   // scratch: the coefficient blocks ([column][band], total_cols x nb), then
   // the back-projection rows (total_rows x nb)
   double* d_coef = nullptr;
   int64_t coef_cap = 0;
-  bool chi_c_smem_set = false;  // the chi*C kernel's shared-memory attribute
   std::vector<int64_t> blk_width;  // host copy of each block's ncol
   std::mutex mu;
 };
@@ -64,21 +63,32 @@ namespace skg {
 
 namespace {
 
-// Forward CTA: (block q, 32 bands, 16 columns); thread (band bl = tid % 32,
-// columns 4 jq .. 4 jq + 3, jq = tid / 32). The CTA walks the block's
-// projectors in order and each projector's rows in chunks of 32: per chunk,
-// 32 gathered rows x 32 bands of psi and the matching 32 rows x 16 columns
-// of chi land in shared memory by asynchronous copies, double-buffered (24 KB
-// a CTA, so that all CTAs of the apply are resident at once; the
-// next chunk's gathers are in flight while the current one is summed). Every
-// thread adds its four columns' products over a chunk's rows in row order —
-// the reference's order, so the sums are exact to it — and folds each
-// projector's sum into the block coefficient with fma(dv, sum, C).
-// Coefficients stored [column][band].
+// chi on the device: each projector's columns in groups of kNlocCols, a group
+// row-major [nrow][kNlocCols], columns past ncol zero. A chunk of rows of a group
+// is then contiguous, for whole 16-byte copies.
+//
+// Forward CTA: (block q, 32 bands, 16 columns); thread (bands bl, bl + 1, columns
+// jl, jl + 1). The CTA walks the block's projectors in order and each projector's
+// rows in chunks of kNlocRows: a chunk's gathered rows x 32 bands of psi and its
+// rows x 16 columns of chi land in shared memory by asynchronous copies,
+// kNlocRing - 1 chunks ahead, the gathered row numbers one chunk before that (24
+// KB a CTA: all CTAs of 64 atoms x 512 bands are resident at once). Every thread
+// adds its products over a chunk's rows in row order — the reference's order, so
+// the sums are exact to it — and folds each projector's sum into the block
+// coefficient with fma(dv, sum, C). Coefficients stored [column][band].
+// Bound by the latency of gathers and the adds' order (a projector's rows are one
+// chain per output) at small sizes, by the issue rate at large ones. Before: 32-row
+// chunks, one ahead, their row numbers loaded just before the copies, chi copied 8
+// bytes at a time from its columns, five 8-byte shared loads for four sums.
+// 64 balls of ~800 points x 16 columns x 512 bands 137 -> 99 us, 37 bands 105 -> 46
+// us; 20 balls of ~380 points x 9 columns x 100 bands 50 -> 25 us.
 constexpr int kNlocBands = 32;
 constexpr int kNlocCols = 16;
-constexpr int kNlocRows = 32;
+constexpr int kNlocRows = 16;
+constexpr int kNlocRing = 4;
 constexpr int kNlocThreads = kNlocBands * kNlocCols / 4;
+static_assert(kNlocRows * kNlocCols == 2 * kNlocThreads, "one 16-byte piece of chi a thread");
+static_assert(kNlocRows * kNlocBands == 4 * kNlocThreads, "two 16-byte pieces of psi a thread");
 
 __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
     int64_t nb, int64_t K, double dv, const int64_t* __restrict__ blk,
@@ -88,188 +98,230 @@ __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
     const uint32_t* __restrict__ index, const double* __restrict__ chi,
     const double* __restrict__ gamma, const double* __restrict__ psi16,
     double* __restrict__ coef) {
-  __shared__ __align__(16) double rows[2][kNlocRows][kNlocBands];
-  __shared__ __align__(16) double xs[2][kNlocCols][kNlocRows];
+  __shared__ __align__(16) double rows[kNlocRing][kNlocRows][kNlocBands];
+  __shared__ __align__(16) double xs[kNlocRing][kNlocRows][kNlocCols];
   const int64_t q = blockIdx.x;
   const int64_t b0 = (int64_t)blockIdx.y * kNlocBands;
   const int64_t jb = (int64_t)blockIdx.z * kNlocCols;  // the CTA's first column
-  const int bl = threadIdx.x % kNlocBands;
-  const int jq = threadIdx.x / kNlocBands;
+  const int bl = 2 * (threadIdx.x % (kNlocBands / 2));
+  const int jl = 2 * (threadIdx.x / (kNlocBands / 2));
   const int64_t col0 = blk[4 * q], nc = blk[4 * q + 1];
   if (jb >= nc) return;  // the whole CTA past the block
-  const int ncc = (int)min((int64_t)kNlocCols, nc - jb);  // columns of this CTA
-  const int64_t b = b0 + bl;
   const int64_t e_begin = blk[4 * q + 2], e_end = blk_end[2 * q];
-  // Issue the copies of chunk r0 of projector entry e into buffer buf.
-  auto issue = [&](int64_t e, int64_t r0, int buf) {
-    const int p = blk_proj[e];
-    const int64_t nr = nrow[p];
-    const int nrr = (int)min((int64_t)kNlocRows, nr - r0);
-    const uint32_t* idx = index + row_off[p];
-    // psi rows: 64 rows x 2 band tiles x 8 pieces of 16 bytes (two bands).
-#pragma unroll
-    for (int i = threadIdx.x; i < kNlocRows * kNlocBands / 2; i += kNlocThreads) {
-      const int rr = i / (kNlocBands / 2), cb = 2 * (i % (kNlocBands / 2));
-      const int64_t bb = b0 + cb;
-      const bool ok = rr < nrr && bb < nb;
-      const double* src = psi16;
-      if (ok) src = psi16 + ((bb / 16) * K + (int64_t)__ldg(idx + r0 + rr)) * 16 + (bb % 16);
-      cp_async16(&rows[buf][rr][cb], src, ok ? 16u : 0u);
-    }
-    const double* x = chi + chi_off[p] + jb * nr;
-#pragma unroll
-    for (int i = threadIdx.x; i < kNlocCols * kNlocRows; i += kNlocThreads) {
-      const int jj = i / kNlocRows, rr = i % kNlocRows;
-      const bool ok = jj < ncc && rr < nrr;
-      cp_async8(&xs[buf][jj][rr], ok ? x + jj * nr + r0 + rr : chi, ok ? 8u : 0u);
+  const int64_t b = b0 + bl;
+  // This thread's copies: bands bl, bl + 1 of rows cr and cr + kNlocRows / 2, and
+  // 16 bytes of chi.
+  const int cr = threadIdx.x / (kNlocBands / 2);
+  const bool band_ok = b < nb;
+  const double* pb = psi16 + (band_ok ? (b / 16) * K * 16 + b % 16 : 0);
+
+  // Issuing cursor: a projector entry, its rows and the chunk's first row; the
+  // chunk's row numbers for this thread's copies.
+  int64_t ie = e_begin, ib = 0;
+  int ir0 = 0, inr = 0;
+  const double* ix = chi;
+  uint32_t n0 = 0, n1 = 0;
+  auto enter = [&]() {  // entry ie
+    if (ie < e_end) {
+      const int p = blk_proj[ie];
+      inr = (int)nrow[p];
+      ib = row_off[p];
+      ix = chi + chi_off[p] + jb * inr;
     }
   };
-  // Chunk cursor over (projector entry, first row); advance returns false at
-  // the block's end.
-  auto advance = [&](int64_t& e, int64_t& r0) -> bool {
-    r0 += kNlocRows;
-    while (e < e_end && r0 >= (int64_t)nrow[blk_proj[e]]) {
-      ++e;
-      r0 = 0;
+  auto numbers = [&]() {
+    if (ie < e_end) {
+      const uint32_t* idx = index + ib + ir0 + cr;
+      if (ir0 + cr < inr) n0 = __ldg(idx);
+      if (ir0 + cr + kNlocRows / 2 < inr) n1 = __ldg(idx + kNlocRows / 2);
     }
-    return e < e_end;
   };
-  int64_t e = e_begin, r0 = 0;
-  // Skip leading projectors without rows.
-  while (e < e_end && nrow[blk_proj[e]] == 0) ++e;
+  auto issue = [&](int buf) {
+    if (ie < e_end) {
+      const int left = inr - ir0;
+      if (band_ok && cr < left) cp_async16(&rows[buf][cr][bl], pb + (int64_t)n0 * 16, 16u);
+      if (band_ok && cr + kNlocRows / 2 < left)
+        cp_async16(&rows[buf][cr + kNlocRows / 2][bl], pb + (int64_t)n1 * 16, 16u);
+      const int o = 2 * threadIdx.x;
+      if (o / kNlocCols < left) cp_async16(&xs[buf][0][0] + o, ix + (int64_t)ir0 * kNlocCols + o, 16u);
+      ir0 += kNlocRows;
+      if (ir0 >= inr) {
+        ++ie;
+        ir0 = 0;
+        enter();
+      }
+    }
+    cp_async_commit();
+  };
+  enter();
+  for (int s = 0; s < kNlocRing - 1; ++s) {
+    numbers();
+    issue(s);
+  }
+  numbers();
+
   double acc[4] = {};
   double sum[4] = {};
-  if (e < e_end) {
-    issue(e, r0, 0);
-    cp_async_commit();
-  }
   int buf = 0;
-  int64_t done_e = e_begin;  // projectors before this one are folded into acc
-  while (e < e_end) {
-    int64_t ne = e, nr0 = r0;
-    const bool more = advance(ne, nr0);
-    if (more) issue(ne, nr0, buf ^ 1);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int p = blk_proj[e];
-    const int nrr = (int)min((int64_t)kNlocRows, (int64_t)nrow[p] - r0);
-    for (int rr = 0; rr < nrr; ++rr) {
-      const double v = rows[buf][rr][bl];
+  for (int64_t e = e_begin; e < e_end; ++e) {
+    const int nr = (int)nrow[blk_proj[e]];
+    for (int r0 = 0; r0 < nr; r0 += kNlocRows) {
+      cp_async_wait<kNlocRing - 2>();
+      __syncthreads();  // the chunk has landed; the one before it is consumed
+      issue((buf + kNlocRing - 1) % kNlocRing);
+      numbers();
+      const double* rb = &rows[buf][0][bl];
+      const double* xb = &xs[buf][0][jl];
+      auto row = [&](int rr) {
+        const double2 v = *reinterpret_cast<const double2*>(rb + rr * kNlocBands);
+        const double2 x = *reinterpret_cast<const double2*>(xb + rr * kNlocCols);
+        sum[0] = __dadd_rn(sum[0], __dmul_rn(x.x, v.x));
+        sum[1] = __dadd_rn(sum[1], __dmul_rn(x.x, v.y));
+        sum[2] = __dadd_rn(sum[2], __dmul_rn(x.y, v.x));
+        sum[3] = __dadd_rn(sum[3], __dmul_rn(x.y, v.y));
+      };
+      if (nr - r0 >= kNlocRows) {
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
-        sum[jj] = __dadd_rn(sum[jj], __dmul_rn(xs[buf][4 * jq + jj][rr], v));
-    }
-    // Projector e ends with this chunk: fold its sum; projectors without
-    // rows between e and the next chunk's contribute zero sums.
-    if (!more || ne != e) {
-      for (int64_t f = done_e; f <= e; ++f) {
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) acc[jj] = fma(dv, f == e ? sum[jj] : 0.0, acc[jj]);
+        for (int rr = 0; rr < kNlocRows; ++rr) row(rr);
+      } else {
+        for (int rr = 0; rr < nr - r0; ++rr) row(rr);
       }
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) sum[jj] = 0.0;
-      done_e = e + 1;
+      buf = (buf + 1) % kNlocRing;
     }
-    __syncthreads();  // buffer buf consumed before the next issue refills it
-    buf ^= 1;
-    e = ne;
-    r0 = nr0;
-  }
-  // Trailing projectors without rows.
-  for (int64_t f = done_e; f < e_end; ++f) {
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[jj] = fma(dv, 0.0, acc[jj]);
+    for (int i = 0; i < 4; ++i) {  // projector e into the block
+      acc[i] = fma(dv, sum[i], acc[i]);
+      sum[i] = 0.0;
+    }
   }
   if (b >= nb) return;
 #pragma unroll
-  for (int jj = 0; jj < 4; ++jj) {
-    const int64_t j = jb + 4 * jq + jj;
+  for (int jj = 0; jj < 2; ++jj) {
+    const int64_t j = jb + jl + jj;
     if (j >= nc) break;
-    double a = acc[jj];
-    for (int64_t f = blk[4 * q + 3]; f < blk_end[2 * q + 1]; ++f)
-      a = __dmul_rn(a, __ldg(gamma + blk_scale[f] + j));
-    coef[(col0 + j) * nb + b] = a;
+    double a0 = acc[2 * jj], a1 = acc[2 * jj + 1];
+    for (int64_t f = blk[4 * q + 3]; f < blk_end[2 * q + 1]; ++f) {
+      const double gm = __ldg(gamma + blk_scale[f] + j);
+      a0 = __dmul_rn(a0, gm);
+      a1 = __dmul_rn(a1, gm);
+    }
+    coef[(col0 + j) * nb + b] = a0;
+    if (b + 1 < nb) coef[(col0 + j) * nb + b + 1] = a1;
   }
 }
 
 // Back-projection, step 1: temp_p[r, b] = sum_k chi_p[r, k] C_p[k, b] (fused,
 // k ascending: the reference's gemm_ab order) for every projector row, into
 // temp[(row_off_p + r) * nb + b]. CTA = (a span of up to kNlocSpan row tiles
-// of 64 rows of one projector, 64 bands): C's columns for the 64 bands are
-// staged in shared memory once, then each row tile's chi rows are staged and
-// its 64 x 64 outputs written.
+// of 64 rows of one projector, 64 bands); thread = a band pair and every
+// kNlocWarps-th group of 4 rows. A column group's C stays in registers, its chi rows
+// are copied to shared memory ahead of their use and read as broadcasts. Further
+// column groups continue from the stored sums, so the order is the same for any
+// number of columns.
+// Was: C and chi staged in shared memory behind one barrier, a row tile at a time.
+// 64 balls of ~800 points x 16 columns x 512 bands 90 -> 65 us (writing temp alone
+// takes 32 us), 37 bands 25 -> 17 us. Spans of 4 tiles: 64 and 21 us. A second and
+// third column group cost a pass over temp each: 40 columns 57 -> 65 us, with the
+// forward kernel 168 -> 148 us.
 constexpr int kNlocTileR = 64;
 constexpr int kNlocTileB = 64;
 constexpr int kNlocMaxCols = 64;
-constexpr int kNlocSpan = 4;
+constexpr int kNlocSpan = 2;
+constexpr int kNlocWarps = 4;
+static_assert(kNlocSpan == 2, "the waits of nloc_chi_c_kernel");
 
-__global__ void __launch_bounds__(256) nloc_chi_c_kernel(
-    int64_t nb, int max_cols, const int64_t* __restrict__ tile_proj,
-    const int64_t* __restrict__ tile_r0,
+__global__ void __launch_bounds__(kNlocWarps * 32) nloc_chi_c_kernel(
+    int64_t nb, const int64_t* __restrict__ tile_proj, const int64_t* __restrict__ tile_r0,
     const uint32_t* __restrict__ nrow, const uint32_t* __restrict__ ncol,
     const int64_t* __restrict__ row_off, const int64_t* __restrict__ chi_off,
     const int64_t* __restrict__ proj_col, const double* __restrict__ chi,
     const double* __restrict__ coef, double* __restrict__ temp) {
-  extern __shared__ double nsm[];
-  double* cs = nsm;                     // [max_cols][kNlocTileB]
-  double* xs = nsm + max_cols * kNlocTileB;  // [kNlocTileR][nc + 1]
+  __shared__ __align__(16) double xs[kNlocSpan][kNlocTileR][kNlocCols];
   const int64_t tile = blockIdx.x;
   const int p = (int)tile_proj[tile];
   const int64_t span0 = tile_r0[tile];
-  const int64_t nr = nrow[p], nc = ncol[p];
-  const int64_t b0 = (int64_t)blockIdx.y * kNlocTileB;
-  const double* c = coef + proj_col[p] * nb;
-  for (int i = threadIdx.x; i < nc * kNlocTileB; i += blockDim.x) {
-    const int k = i / kNlocTileB, bb = i % kNlocTileB;
-    cs[k * kNlocTileB + bb] = (b0 + bb < nb) ? c[k * nb + b0 + bb] : 0.0;
-  }
-  // Thread: band pairs 2 q4, 2 q4 + 1 and 32 + 2 q4, 33 + 2 q4 of the tile
-  // (q4 = tid % 16; 16-byte loads and stores, consecutive lanes on
-  // consecutive pairs) and rows rg, rg + 16, rg + 32, rg + 48 (rg = tid / 16):
-  // per column, four chi and four C values feed 16 multiply-adds, each
-  // output's sum over the columns in order.
-  const int q4 = threadIdx.x % 16, rg = threadIdx.x / 16;
-  for (int t = 0; t < kNlocSpan; ++t) {
-    const int64_t r0 = span0 + (int64_t)t * kNlocTileR;
-    if (r0 >= nr) break;
-    const int nrr = (int)min((int64_t)kNlocTileR, nr - r0);
-    if (t > 0) __syncthreads();  // the previous tile's chi rows are consumed
-    const double* x = chi + chi_off[p] + r0;
-    for (int i = threadIdx.x; i < nc * kNlocTileR; i += blockDim.x) {
-      const int k = i / kNlocTileR, rr = i % kNlocTileR;
-      xs[rr * (nc + 1) + k] = rr < nrr ? x[k * nr + rr] : 0.0;
+  const int nr = (int)min((int64_t)nrow[p] - span0, (int64_t)kNlocSpan * kNlocTileR);
+  const int nc = (int)ncol[p];
+  const int64_t b = (int64_t)blockIdx.y * kNlocTileB + 2 * (threadIdx.x % 32);
+  const int warp = threadIdx.x / 32;
+  const bool one = b < nb, two = b + 1 < nb;
+  // 16-byte accesses where every row of temp starts on 16 bytes.
+  const bool wide = two && nb % 2 == 0 && (reinterpret_cast<uintptr_t>(temp) & 15) == 0;
+  double* out = temp + (row_off[p] + span0) * nb + b;
+  for (int k0 = 0; k0 < nc; k0 += kNlocCols) {
+    if (k0 > 0) __syncthreads();  // the group before is consumed
+    const double* x = chi + chi_off[p] + (int64_t)k0 * nrow[p] + span0 * kNlocCols;
+#pragma unroll
+    for (int t = 0; t < kNlocSpan; ++t) {
+#pragma unroll
+      for (int i = 0; i < kNlocTileR * kNlocCols / 2; i += kNlocWarps * 32) {
+        const int o = t * kNlocTileR * kNlocCols + 2 * (i + (int)threadIdx.x);
+        if (o / kNlocCols < nr) cp_async16(&xs[0][0][0] + o, x + o, 16u);
+      }
+      cp_async_commit();
     }
-    __syncthreads();
-    double tt[4][4] = {};
-    for (int k = 0; k < nc; ++k) {
-      double cv[4], xv[4];
+    const int ncg = min(kNlocCols, nc - k0);
+    const double* c = coef + (proj_col[p] + k0) * nb + b;
+    double c0[kNlocCols], c1[kNlocCols];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) cv[jj] = cs[k * kNlocTileB + 32 * (jj >> 1) + 2 * q4 + (jj & 1)];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) xv[i] = xs[(rg + 16 * i) * (nc + 1) + k];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) tt[i][jj] = fma(xv[i], cv[jj], tt[i][jj]);
+    for (int k = 0; k < kNlocCols; ++k) {
+      c0[k] = k < ncg && one ? c[k * nb] : 0.0;
+      c1[k] = k < ncg && two ? c[k * nb + 1] : 0.0;
     }
-    double* out = temp + (row_off[p] + r0) * nb + b0 + 2 * q4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rr = rg + 16 * i;
-      if (rr >= nrr) break;
+    for (int t = 0; t < kNlocSpan; ++t) {
+      if (t * kNlocTileR >= nr) break;
+      if (t == 0)
+        cp_async_wait<kNlocSpan - 1>();
+      else
+        cp_async_wait<0>();
+      __syncthreads();
+      for (int r0 = 4 * warp; r0 < kNlocTileR; r0 += 4 * kNlocWarps) {
+        const int r = t * kNlocTileR + r0;
+        if (r >= nr || !one) break;
+        double t0[4] = {}, t1[4] = {};
+        if (k0 > 0) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        double* o = out + (int64_t)rr * nb + 32 * h;
-        const int64_t bb = b0 + 32 * h + 2 * q4;
-        if (bb + 1 < nb && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
-          *reinterpret_cast<double2*>(o) = make_double2(tt[i][2 * h], tt[i][2 * h + 1]);
-        } else {
-          if (bb < nb) o[0] = tt[i][2 * h];
-          if (bb + 1 < nb) o[1] = tt[i][2 * h + 1];
+          for (int i = 0; i < 4; ++i)
+            if (r + i < nr) {
+              t0[i] = out[(r + i) * nb];
+              if (two) t1[i] = out[(r + i) * nb + 1];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kNlocCols; k += 2) {
+          if (k >= ncg) break;
+          double2 v[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            v[i] = *reinterpret_cast<const double2*>(&xs[t][r0 + i][k]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            t0[i] = fma(v[i].x, c0[k], t0[i]);
+            t1[i] = fma(v[i].x, c1[k], t1[i]);
+          }
+          if (k + 1 < ncg) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              t0[i] = fma(v[i].y, c0[k + 1], t0[i]);
+              t1[i] = fma(v[i].y, c1[k + 1], t1[i]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (r + i >= nr) break;
+          double* o = out + (int64_t)(r + i) * nb;
+          if (wide) {
+            *reinterpret_cast<double2*>(o) = make_double2(t0[i], t1[i]);
+          } else {
+            o[0] = t0[i];
+            if (two) o[1] = t1[i];
+          }
         }
       }
     }
+    cp_async_wait<0>();
   }
 }
 
@@ -330,15 +382,17 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
   DeviceState* dev = current_device(&st);
   if (!dev) return st;
   std::vector<int64_t> row_off(P), chi_off(P);
-  int64_t rows = 0, chis = 0, gams = 0;
-  std::vector<int64_t> gam_off(P);
+  int64_t rows = 0, chis = 0, gams = 0, chi_in = 0;
+  std::vector<int64_t> gam_off(P), in_off(P);
   const int64_t total = P > 0 ? offsets[P] : 0;
   for (int64_t p = 0; p < P; ++p) {
     row_off[p] = rows;
     chi_off[p] = chis;
     gam_off[p] = gams;
     rows += nrow[p];
-    chis += (int64_t)nrow[p] * ncol[p];
+    in_off[p] = chi_in;
+    chi_in += (int64_t)nrow[p] * ncol[p];
+    chis += (int64_t)nrow[p] * ((ncol[p] + kNlocCols - 1) / kNlocCols) * kNlocCols;
     gams += ncol[p];
     if ((int64_t)offsets[p] + ncol[p] > total)
       return fail(SKGEMM_ERR_INVALID_ARG, "projector block past the total column count");
@@ -346,7 +400,7 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
       return fail(SKGEMM_ERR_UNSUPPORTED, "projectors of more than 64 columns");
   }
   if (rows > 0 && !index) return fail(SKGEMM_ERR_INVALID_ARG, "null index array");
-  if ((chis > 0 && !chi) || (gams > 0 && !gamma))
+  if ((chi_in > 0 && !chi) || (gams > 0 && !gamma))
     return fail(SKGEMM_ERR_INVALID_ARG, "null coefficient array");
   for (int64_t i = 0; i < rows; ++i)
     if (index[i] >= (uint64_t)K) return fail(SKGEMM_ERR_INVALID_ARG, "grid index out of range");
@@ -430,7 +484,6 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
   std::vector<int64_t> tile_proj, tile_r0;
   for (int64_t p = 0; p < P; ++p) {
     if (nrow[p] == 0 || ncol[p] == 0) continue;
-    h->max_cols = std::max<int64_t>(h->max_cols, ncol[p]);
     for (int64_t r0 = 0; r0 < nrow[p]; r0 += kNlocTileR * kNlocSpan) {
       tile_proj.push_back(p);
       tile_r0.push_back(r0);
@@ -439,7 +492,12 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
   h->ntiles = (int64_t)tile_proj.size();
   std::vector<uint32_t> vnrow(nrow, nrow + P), vncol(ncol, ncol + P);
   std::vector<uint32_t> vindex(index, index + rows);
-  std::vector<double> vchi(chi, chi + chis), vgam(gamma, gamma + gams);
+  std::vector<double> vchi(chis, 0.0), vgam(gamma, gamma + gams);
+  for (int64_t p = 0; p < P; ++p)
+    for (int64_t j = 0; j < ncol[p]; ++j)
+      for (int64_t r = 0; r < nrow[p]; ++r)
+        vchi[chi_off[p] + (j / kNlocCols * nrow[p] + r) * kNlocCols + j % kNlocCols] =
+            chi[in_off[p] + j * nrow[p] + r];
   if ((st = upload(&h->d_nrow, vnrow)) || (st = upload(&h->d_ncol, vncol)) ||
       (st = upload(&h->d_index, vindex)) || (st = upload(&h->d_row_off, row_off)) ||
       (st = upload(&h->d_chi_off, chi_off)) || (st = upload(&h->d_chi, vchi)) ||
@@ -501,19 +559,10 @@ int nloc_apply(skgemm_nloc* h, int64_t nb, double dv, const double* psi16, doubl
     dim3 grid((unsigned)h->ntiles, (unsigned)((nb + kNlocTileB - 1) / kNlocTileB));
     if (h->ntiles > INT32_MAX || grid.y > 65535u)
       return fail(SKGEMM_ERR_INVALID_ARG, "too many projector rows or bands");
-    // Shared memory for the set's widest projector (C columns and chi rows).
-    const int mc = (int)h->max_cols;
-    const size_t smem = ((size_t)mc * kNlocTileB + kNlocTileR * (size_t)(mc + 1)) * 8;
-    if (!h->chi_c_smem_set) {  // per handle: a handle belongs to one device
-      const size_t smem_max = (kNlocMaxCols * kNlocTileB + kNlocTileR * (kNlocMaxCols + 1)) * 8;
-      SKG_CUDA(cudaFuncSetAttribute(nloc_chi_c_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-      h->chi_c_smem_set = true;
-    }
     KernelTimer kt_(s, "nloc_chi_c_kernel");
-    nloc_chi_c_kernel<<<grid, 256, smem, s>>>(nb, mc, h->d_tile_proj, h->d_tile_r0, h->d_nrow,
-                                              h->d_ncol, h->d_row_off, h->d_chi_off,
-                                              h->d_proj_blk_col, h->d_chi, h->d_coef, temp);
+    nloc_chi_c_kernel<<<grid, kNlocWarps * 32, 0, s>>>(
+        nb, h->d_tile_proj, h->d_tile_r0, h->d_nrow, h->d_ncol, h->d_row_off, h->d_chi_off,
+        h->d_proj_blk_col, h->d_chi, h->d_coef, temp);
     SKG_CUDA(cudaGetLastError());
   }
   const int64_t nbk = h->ntouch * ((nb + 1) / 2);  // threads: (touched point, band pair)

@@ -33,6 +33,33 @@ def test_nloc_equals_oracle(cuda, K, nb, nrow, ncol, P, images, T):
     h.close()
 
 
+@pytest.mark.parametrize("nb,nrow,ncol", [
+    (1, 1, 1),      # one row, one column, one band
+    (31, 15, 2),    # below a chunk
+    (33, 16, 15),   # one chunk
+    (2, 17, 16),    # one row over, a whole column group
+    (65, 63, 17),   # below a row tile, two column groups
+    (64, 65, 33),   # one row over a tile, three column groups
+    (17, 129, 64),  # one row over a span, the widest
+    (130, 50, 9),   # fewer chunks than the ring ahead of the last
+])
+def test_nloc_chunk_edges(cuda, nb, nrow, ncol):
+    """Rows, columns and bands around the chunks, column groups and tiles that the
+    kernels stage; equal bits."""
+    K = 700
+    pj = oracle.nloc_random(K, nrow, ncol, 3, seed=nb + nrow, images=2)
+    rng = np.random.default_rng(nrow)
+    psi16 = rng.uniform(-1, 1, (nb + 15) // 16 * K * 16)
+    base = rng.uniform(-1, 1, (nb + 31) // 32 * K * 32)
+    want = oracle.nloc_project(pj, psi16, nb, K, 0.02, base.copy(), 32)
+    h = handle(pj, K)
+    out = torch.from_numpy(base.copy()).cuda()
+    h.apply(nb, 0.02, torch.from_numpy(psi16).cuda(), out, 32)
+    skgemm.stream_status()
+    assert np.array_equal(out.cpu().numpy(), want)
+    h.close()
+
+
 def test_nloc_handle_reused_across_band_counts(cuda):
     """One handle applied at growing band counts (its scratch regrows) and
     twice at the same count (out accumulates): each call equals the oracle."""
