@@ -168,7 +168,7 @@ int skgemm_dgemm_packed_dev(int64_t M, int64_t N, int64_t K, const double* A_pac
  * allocate every buffer themselves).
  * Same contract as skgemm_dgemm_packed_dev (native FP64, 128 x 128 tiles);
  * the result agrees with it within FP64 rounding (relative Frobenius error
- * <= 1e-13), not bit for bit, since the regular entry may pick 64 x 64 tiles
+ * <= 1e-13), not bit for bit, since the regular entry may pick smaller tiles
  * and so a different Stream-K split. Its Stream-K scratch is a static device
  * array of 148 partial-tile slots (19.4 MB), held on each GPU where the
  * library's no-alloc code has been loaded until the process exits; a launch
