@@ -49,9 +49,8 @@ struct StencilCoef {
 // reference kernels: the output equals theirs bit for bit. Every wait is
 // bounded; on expiry the CTA records the error and skips the remaining waits.
 //
-// Bound by the shared-memory pipe: 20 16-byte loads per column and band pair
-// and the stage itself are 1.7 kcycles of it per plane (335 us of 48^3 x 512's
-// 351 us). TMA moves one box row per 1.3 cycles whatever its length, so the
+// Bound by the shared-memory pipe, 89% busy: 20 16-byte loads per column and
+// band pair, and the stage itself is written through it. TMA moves one box row per 1.3 cycles whatever its length, so the
 // 32-byte rows of a 4-band slab on 16 x 16 columns took 297 us without any
 // arithmetic against 225 us for these 64-byte rows (400 us and 351 us in all).
 // Whole launches, one CTA per tile with its queues loaded at its start, 4-band
