@@ -489,7 +489,7 @@ def kernel_rooflines(skgemm, step, torch, steps, peaks, band, grid, q, S, Pn):
                 "i8_gemm2_kernel": (Ls * FLOP_SYRK, "TOP/s", i8_peak, "tensor"),
                 "i8_rot_kernel": (Lr * FLOP_ROT, "TOP/s", i8_peak, "tensor"),
                 "convert_tma_kernel": (E * (8 + rb * Ls), "GB/s", hbm, "hbm"),
-                "row_norms_kernel": (E * 8, "GB/s", hbm, "hbm"),
+                "norm_partials_kernel": (E * 8, "GB/s", hbm, "hbm"),
                 "convert_short_kernel": (E * (8 + rb * Lr), "GB/s", hbm, "hbm"),
                 "crt_residues_band_kernel": (E * (rb * Lr + 8), "GB/s", hbm, "hbm")}
     if step.prec is None:

@@ -259,21 +259,13 @@ __device__ __forceinline__ uint32_t residue_bf16x2(const Digits& a, const Digits
 }
 
 // ------------------------------------------------- packed-T operand prep
-// Row exponents mu[row] of a packed-T operand ([ceil(R/T)][K][T]): each CTA sums
-// the squares of one panel's rows over k-chunk c into part[(p*C + c)*T + r], and
-// the panel's last CTA to finish adds the chunks in order and writes the
-// exponents (a kernel of its own for that was a launch on the way to every
-// conversion). arrived[p] counts the panel's CTAs and returns to 0. Rows past R
-// get 0.
+// Partial sums of squares of each row of a packed-T operand
+// ([ceil(R/T)][K][T]): part[(p*C + c)*T + r] over k-chunk c.
 template <int T, bool KM = false>
-__global__ void __launch_bounds__(256) row_norms_kernel(int64_t R, int64_t K,
-                                                       const double* __restrict__ X, int C,
-                                                       double* __restrict__ part,
-                                                       unsigned* __restrict__ arrived,
-                                                       int gamma_bits, int64_t Rpad,
-                                                       int* __restrict__ mu) {
+__global__ void __launch_bounds__(256) norm_partials_kernel(int64_t R, int64_t K,
+                                                           const double* __restrict__ X,
+                                                           int C, double* __restrict__ part) {
   __shared__ double red[256];
-  __shared__ bool last;
   const int p = blockIdx.x, c = blockIdx.y;
   // KM: thread (kl = tid % 16, r = tid / 16), so that a warp reads two rows'
   // whole 128-byte k-blocks; each (r, kl) sum is the packed layout's, and
@@ -300,34 +292,30 @@ __global__ void __launch_bounds__(256) row_norms_kernel(int64_t R, int64_t K,
   }
   red[slot] = acc;
   __syncthreads();
-  const int64_t row = (int64_t)p * T + threadIdx.x;
-  double s = 0.0;
   if (threadIdx.x < T) {
+    double s = 0.0;
     for (int j = 0; j < KL; ++j) s += red[j * T + threadIdx.x];
-    if (row >= R) s = 0.0;
+    const int64_t row = (int64_t)p * T + threadIdx.x;
+    part[((int64_t)p * C + c) * T + threadIdx.x] = row < R ? s : 0.0;
   }
-  if (C > 1) {
-    if (threadIdx.x < T) {
-      __stcg(&part[((int64_t)p * C + c) * T + threadIdx.x], s);
-      __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      last = atomicAdd(&arrived[p], 1u) == (unsigned)C - 1;
-      if (last) arrived[p] = 0;  // every CTA of the panel has arrived
-      __threadfence();
-    }
-    __syncthreads();
-    if (!last) return;
-    if (threadIdx.x < T) {
-      s = 0.0;
-      for (int j = 0; j < C; ++j) s += __ldcg(&part[((int64_t)p * C + j) * T + threadIdx.x]);
-    }
+}
+
+// Row exponents mu[row] (row < Rpad) of a packed-T operand from its norm
+// partials; rows past R (padding) get 0.
+template <int T>
+__global__ void row_exponents_kernel(int64_t R, int64_t Rpad, int C, const double* __restrict__ part,
+                                     int gamma_bits, int* __restrict__ mu) {
+  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= Rpad) return;
+  int m = 0;
+  if (row < R) {
+    const int64_t p = row / T;
+    const int rin = (int)(row - p * T);
+    double sq = 0.0;
+    for (int c = 0; c < C; ++c) sq += part[(p * C + c) * T + rin];
+    m = row_exponent(sq, gamma_bits);
   }
-  if (threadIdx.x < T && row < Rpad) {
-    // C = 1 sums 0.0 + s as the chunked path does.
-    mu[row] = row < R ? row_exponent(0.0 + s, gamma_bits) : 0;
-  }
+  mu[row] = m;
 }
 
 // Residues of a packed-T operand -> res[l][Rpad][KP] (K-major bytes).
@@ -873,7 +861,6 @@ struct LanePlan {
 
 struct OzakiStream {
   DeviceBuffer res_a, res_b, part_a, part_b, mu_a, mu_b, partials, rbytes;
-  DeviceBuffer cnt_a, cnt_b;  // the norm passes' counters: zero between calls
   cudaEvent_t fork2 = nullptr, join2 = nullptr;
   // Helper stream forked from the caller's stream: the norm pass of B runs
   // there while A is converted (the conversion leaves HBM bandwidth idle).
@@ -1353,21 +1340,10 @@ int launch_short_L(DeviceState* dev, const CUtensorMap& map, int64_t R, int64_t 
   return SKGEMM_OK;
 }
 
-// One counter per panel for row_norms_kernel, zero between calls.
-int ensure_counters(DeviceBuffer& cnt, int64_t panels, cudaStream_t s) {
-  const size_t had = cnt.bytes;
-  int st;
-  if ((st = cnt.ensure((size_t)panels * sizeof(unsigned))) != SKGEMM_OK) return st;
-  if (cnt.bytes == had) return SKGEMM_OK;
-  if (debug_fill_enabled()) SKG_CUDA(cudaStreamSynchronize(nullptr));  // after the 0xFF fill
-  SKG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes, s));
-  return SKGEMM_OK;
-}
-
 template <int T>
 int prep_norms(int64_t R, int64_t K, int64_t KP, int64_t Rpad, const double* X, int L,
-               DeviceBuffer& res, DeviceBuffer& part, DeviceBuffer& mu, DeviceBuffer& cnt,
-               cudaStream_t s, bool bf = false, bool km = false) {
+               DeviceBuffer& res, DeviceBuffer& part, DeviceBuffer& mu, cudaStream_t s,
+               bool bf = false, bool km = false) {
   if ((reinterpret_cast<uintptr_t>(X) & 15) != 0)
     return fail(SKGEMM_ERR_INVALID_ARG, "operand base must be 16-byte aligned");
   if (K > ((int64_t)1 << 31) - 128) return fail(SKGEMM_ERR_INVALID_ARG, "K too large");
@@ -1378,16 +1354,19 @@ int prep_norms(int64_t R, int64_t K, int64_t KP, int64_t Rpad, const double* X, 
   if ((st = part.ensure((size_t)P_in * C * T * sizeof(double))) != SKGEMM_OK) return st;
   if ((st = mu.ensure((size_t)Rpad * sizeof(int))) != SKGEMM_OK) return st;
   if (km && T != 16) return fail(SKGEMM_ERR_INVALID_ARG, "K-major operand with 32-wide panels");
-  if ((st = ensure_counters(cnt, P_in, s)) != SKGEMM_OK) return st;
-  KernelTimer kt_(s, "row_norms_kernel");
-  const dim3 grid((unsigned)P_in, (unsigned)C);
-  if (km)
-    row_norms_kernel<16, true><<<grid, 256, 0, s>>>(R, K, X, C, (double*)part.ptr,
-                                                    (unsigned*)cnt.ptr, gamma_for(L), Rpad,
-                                                    (int*)mu.ptr);
-  else
-    row_norms_kernel<T><<<grid, 256, 0, s>>>(R, K, X, C, (double*)part.ptr, (unsigned*)cnt.ptr,
-                                             gamma_for(L), Rpad, (int*)mu.ptr);
+  {
+    KernelTimer kt_(s, "norm_partials_kernel");
+    if (km)
+      norm_partials_kernel<16, true><<<dim3((unsigned)P_in, C), 256, 0, s>>>(R, K, X, C,
+                                                                            (double*)part.ptr);
+    else
+      norm_partials_kernel<T><<<dim3((unsigned)P_in, C), 256, 0, s>>>(R, K, X, C,
+                                                                      (double*)part.ptr);
+  }
+  SKG_CUDA(cudaGetLastError());
+  KernelTimer kt_(s, "row_exponents_kernel");
+  row_exponents_kernel<T><<<(unsigned)((Rpad + 255) / 256), 256, 0, s>>>(
+      R, Rpad, C, (const double*)part.ptr, gamma_for(L), (int*)mu.ptr);
   SKG_CUDA(cudaGetLastError());
   return SKGEMM_OK;
 }
@@ -1433,8 +1412,7 @@ int prep_convert(DeviceState* dev, int64_t R, int64_t K, int64_t KP, int64_t Rpa
 template <int T>
 int prep_packed(DeviceState* dev, int64_t R, int64_t K, int64_t KP, int64_t Rpad,
                 const double* X, int L, DeviceBuffer& res, DeviceBuffer& part, DeviceBuffer& mu,
-                DeviceBuffer& cnt, uint32_t* err, cudaStream_t s, bool bf = false,
-                bool km = false) {
+                uint32_t* err, cudaStream_t s, bool bf = false, bool km = false) {
   int st;
   // Short rows (K <= 512) and a one-chunk norm pass (ceil(R/16) >= 600): one
   // pass, convert_short_kernel (same exponents and residues bit for bit),
@@ -1475,7 +1453,7 @@ int prep_packed(DeviceState* dev, int64_t R, int64_t K, int64_t KP, int64_t Rpad
     SKG_DISPATCH_L(L, (launch_short_L<LL, false, false>(dev, map, R, K, KP, Rpad, (int*)mu.ptr,
                                                         (uint8_t*)res.ptr, err, s)))
   }
-  if ((st = prep_norms<T>(R, K, KP, Rpad, X, L, res, part, mu, cnt, s, bf, km))) return st;
+  if ((st = prep_norms<T>(R, K, KP, Rpad, X, L, res, part, mu, s, bf, km))) return st;
   return prep_convert<T>(dev, R, K, KP, Rpad, X, L, res, mu, err, s, bf, km);
 }
 
@@ -1599,15 +1577,6 @@ int pair_product(DeviceState* dev, OzakiStream* os, StreamWorkspace* ws, int64_t
   return SKGEMM_OK;
 }
 
-// The helper stream and its fork / join events.
-int ensure_aux(OzakiStream* os) {
-  if (os->aux) return SKGEMM_OK;
-  SKG_CUDA(cudaStreamCreateWithFlags(&os->aux, cudaStreamNonBlocking));
-  SKG_CUDA(cudaEventCreateWithFlags(&os->fork, cudaEventDisableTiming));
-  SKG_CUDA(cudaEventCreateWithFlags(&os->join, cudaEventDisableTiming));
-  return SKGEMM_OK;
-}
-
 // Residues of A (packed16, M rows) into os->res_a and, unless Bp is null, of
 // B (packed32, N rows) into os->res_b: norms(A) | norms(B) on the helper
 // stream, convert(A), join, convert(B).
@@ -1619,16 +1588,20 @@ int prep_pair(DeviceState* dev, OzakiStream* os, StreamWorkspace* ws, int64_t M,
   const int64_t RA = (M + kI8BN - 1) / kI8BN * kI8BN;  // 256-multiples serve both box heights
   const int64_t RB = (N + kI8BN - 1) / kI8BN * kI8BN;
   if (!Bp)
-    return prep_packed<16>(dev, M, K, KP, RA, Ap, L, os->res_a, os->part_a, os->mu_a, os->cnt_a, ws->err, s,
+    return prep_packed<16>(dev, M, K, KP, RA, Ap, L, os->res_a, os->part_a, os->mu_a, ws->err, s,
                            bf);
-  if ((st = ensure_aux(os))) return st;
+  if (!os->aux) {
+    SKG_CUDA(cudaStreamCreateWithFlags(&os->aux, cudaStreamNonBlocking));
+    SKG_CUDA(cudaEventCreateWithFlags(&os->fork, cudaEventDisableTiming));
+    SKG_CUDA(cudaEventCreateWithFlags(&os->join, cudaEventDisableTiming));
+  }
   SKG_CUDA(cudaEventRecord(os->fork, s));
   SKG_CUDA(cudaStreamWaitEvent(os->aux, os->fork, 0));
   const int st_b =
-      prep_norms<32>(N, K, KP, RB, Bp, L, os->res_b, os->part_b, os->mu_b, os->cnt_b, os->aux, bf);
+      prep_norms<32>(N, K, KP, RB, Bp, L, os->res_b, os->part_b, os->mu_b, os->aux, bf);
   SKG_CUDA(cudaEventRecord(os->join, os->aux));  // join even when the B step failed
   if (st_b) return st_b;
-  if ((st = prep_packed<16>(dev, M, K, KP, RA, Ap, L, os->res_a, os->part_a, os->mu_a, os->cnt_a, ws->err,
+  if ((st = prep_packed<16>(dev, M, K, KP, RA, Ap, L, os->res_a, os->part_a, os->mu_a, ws->err,
                             s, bf)))
     return st;
   SKG_CUDA(cudaStreamWaitEvent(s, os->join, 0));
@@ -1688,7 +1661,11 @@ int subspace_impl(int64_t K, int64_t M, const double* Psi, const double* HPsi, d
   OzakiStream* os = ozaki_stream(dev, s);
   const int64_t KP = (K + 127) / 128 * 128;
   const bool bf = is_bf16(opts);
-  if ((st = ensure_aux(os))) return st;
+  if (!os->aux) {
+    SKG_CUDA(cudaStreamCreateWithFlags(&os->aux, cudaStreamNonBlocking));
+    SKG_CUDA(cudaEventCreateWithFlags(&os->fork, cudaEventDisableTiming));
+    SKG_CUDA(cudaEventCreateWithFlags(&os->join, cudaEventDisableTiming));
+  }
   if (!os->fork2) {
     SKG_CUDA(cudaEventCreateWithFlags(&os->fork2, cudaEventDisableTiming));
     SKG_CUDA(cudaEventCreateWithFlags(&os->join2, cudaEventDisableTiming));
@@ -1702,7 +1679,7 @@ int subspace_impl(int64_t K, int64_t M, const double* Psi, const double* HPsi, d
   const int64_t RA = (M + kI8BN - 1) / kI8BN * kI8BN;
   SKG_CUDA(cudaEventRecord(os->fork, s));
   SKG_CUDA(cudaStreamWaitEvent(os->aux, os->fork, 0));
-  int st_b = prep_norms<32>(M, K, KP, RA, HPsi, L, os->res_b, os->part_b, os->mu_b, os->cnt_b, os->aux, bf);
+  int st_b = prep_norms<32>(M, K, KP, RA, HPsi, L, os->res_b, os->part_b, os->mu_b, os->aux, bf);
   if (!st_b)
     st_b = prep_convert<32>(dev, M, K, KP, RA, HPsi, L, os->res_b, os->mu_b, ws->err, os->aux, bf);
   SKG_CUDA(cudaEventRecord(os->join, os->aux));  // recorded even when a B step failed
@@ -1710,7 +1687,7 @@ int subspace_impl(int64_t K, int64_t M, const double* Psi, const double* HPsi, d
     SKG_CUDA(cudaStreamWaitEvent(s, os->join, 0));
     return st_b;
   }
-  if ((st = prep_packed<16>(dev, M, K, KP, RA, Psi, L, os->res_a, os->part_a, os->mu_a, os->cnt_a, ws->err,
+  if ((st = prep_packed<16>(dev, M, K, KP, RA, Psi, L, os->res_a, os->part_a, os->mu_a, ws->err,
                             s, bf))) {
     SKG_CUDA(cudaStreamWaitEvent(s, os->join, 0));
     return st;
@@ -1864,9 +1841,7 @@ int ozaki_reserve(DeviceState* dev, cudaStream_t s, int64_t Nd, int64_t nb, int 
       (st = os->part_a.ensure(n.part_a)) || (st = os->part_b.ensure(n.part_b)) ||
       (st = os->mu_a.ensure(n.mu_a)) || (st = os->mu_b.ensure(n.mu_b)) ||
       (st = os->partials.ensure(n.partials)) ||
-      (st = os->rbytes.ensure(n.rbytes)) ||
-      (st = ensure_counters(os->cnt_a, (std::max(Nd, nb) + 15) / 16, s)) ||
-      (st = ensure_counters(os->cnt_b, (nb + 31) / 32, s)))
+      (st = os->rbytes.ensure(n.rbytes)))
     return st;
   return SKGEMM_OK;
 }
@@ -1889,7 +1864,7 @@ int ozaki_release_stream(DeviceState* dev, cudaStream_t s) {
     cudaEventDestroy(os->join2);
   }
   for (DeviceBuffer* b : {&os->res_a, &os->res_b, &os->part_a, &os->part_b, &os->mu_a, &os->mu_b,
-                          &os->partials, &os->rbytes, &os->cnt_a, &os->cnt_b})
+                          &os->partials, &os->rbytes})
     b->release();
   delete os;
   m.erase(it);
@@ -2012,19 +1987,12 @@ int ozaki_rot(int64_t Nd, int64_t nb, const double* A, const double* Q, double* 
   if ((st = os->rbytes.ensure((size_t)L * Nd * nb))) return st;
   // Grid-packed Psi is a packed16 operand with rows = grid points, K = bands;
   // band-packed Psi (a_band) the K-major form of the same operand.
-  // Q's residues (nb / 16 CTAs, 9 .. 70 us on their own) on the helper stream,
-  // under Psi's conversion.
-  if ((st = ensure_aux(os))) return st;
-  SKG_CUDA(cudaEventRecord(os->fork, s));
-  SKG_CUDA(cudaStreamWaitEvent(os->aux, os->fork, 0));
-  const int st_q = launch_local(nb, nb, KP, RB, Q, 16, nb, L, (uint8_t*)os->res_b.ptr,
-                                (int*)os->mu_b.ptr, os->aux, bf);
-  SKG_CUDA(cudaEventRecord(os->join, os->aux));  // join even when a step failed
-  st = st_q ? st_q
-            : prep_packed<16>(dev, Nd, nb, KP, RA, A, L, os->res_a, os->part_a, os->mu_a,
-                              os->cnt_a, ws->err, s, bf, a_band);
-  SKG_CUDA(cudaStreamWaitEvent(s, os->join, 0));
-  if (st) return st;
+  if ((st = prep_packed<16>(dev, Nd, nb, KP, RA, A, L, os->res_a, os->part_a, os->mu_a, ws->err,
+                            s, bf, a_band)))
+    return st;
+  if ((st = launch_local(nb, nb, KP, RB, Q, 16, nb, L, (uint8_t*)os->res_b.ptr,
+                         (int*)os->mu_b.ptr, s, bf)))
+    return st;
   CUtensorMap mA, mB;
   if ((st = make_res_map(&mA, os->res_a.ptr, KPb, RA, L, kI8BM))) return st;
   if ((st = make_res_map(&mB, os->res_b.ptr, KPb, RB, L, kI8BN))) return st;
