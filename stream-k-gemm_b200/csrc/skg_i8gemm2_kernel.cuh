@@ -40,10 +40,7 @@ constexpr int kI8P2Stages = 6;
 constexpr int kI8P2TileBytes = 128 * kI8BK;  // 16 KB: 128 rows x one k-block
 constexpr int kI8P2StageBytes = 2 * kI8P2TileBytes;
 constexpr int kI8P2SmemBytes = kI8P2Stages * kI8P2StageBytes + 1024 + 256;
-// Units schedule: eight 32 x 128-byte store boxes (one per epilogue warp) too.
-constexpr int kI8P2BoxBytes = 32 * 128;
-constexpr int kI8P2UnitsSmemBytes = kI8P2SmemBytes + kI8EpiWarps * kI8P2BoxBytes;
-static_assert(kI8P2UnitsSmemBytes <= 232448, "pair kernel exceeds 227 KB of shared memory");
+static_assert(kI8P2SmemBytes <= 232448, "pair kernel exceeds 227 KB of shared memory");
 static_assert((2 * kI8P2Stages + 4) * 8 + 8 <= 256, "pair kernel barrier area");
 
 // Item of a cluster: pair tile t2 = w mod T2, lane q = w / T2 for
@@ -75,44 +72,7 @@ __device__ __forceinline__ bool i8p2_next_item(const I8Params& p, int cl, int nc
   }
 }
 
-// Item of a cluster on the units schedule (the rotation: huge M, full K = nb per
-// item): u = cluster + j * clusters in the order (modulus, 256-row tile, column
-// tile): the clusters running at one time share A's tiles and one modulus's B,
-// and read and write one span of a plane. This CTA's half is `rank`.
-__device__ __forceinline__ bool i8p2_next_unit(const I8Params& p, int cl, int ncl, int rank,
-                                               I8Cursor& cur, I8Item& it) {
-  const int64_t u = (int64_t)cl + (int64_t)cur.item * ncl;
-  const int64_t r = u / p.tiles_n;
-  if (r >= (int64_t)p.tiles_m2 * p.L) return false;
-  it.tn = (int)(u - r * p.tiles_n);
-  it.l = (int)(r / p.tiles_m2);
-  it.tm = 2 * (int)(r - (int64_t)it.l * p.tiles_m2) + rank;
-  it.kb0 = 0;
-  it.kb1 = p.KB;
-  it.slot = 0;
-  it.t = 0;
-  ++cur.item;
-  return true;
-}
-
-template <bool UNITS>
-__device__ __forceinline__ bool i8p2_next(const I8Params& p, int cl, int ncl, int rank,
-                                          I8Cursor& cur, I8Item& it) {
-  if constexpr (UNITS)
-    return i8p2_next_unit(p, cl, ncl, rank, cur, it);
-  else
-    return i8p2_next_item(p, cl, ncl, rank, cur, it);
-}
-
-// UNITS: the rotation's products for nb > 512 (INT8; K = nb too long for the
-// kernel that keeps B resident, i8_rot_kernel), whose epilogue this shares: each
-// epilogue warp reduces its 32 rows x 128 columns modulo m_l into a swizzled
-// shared-memory box and one lane TMA-stores it (mapB2 is the residue map). On one
-// CTA (48 KB of operands per 4.2 M MACs, 16-byte residue stores scattered over 32
-// rows) the products took 0.93 ms at 110592 x 768, 0.87 at 65536 x 1024 and 1.62
-// at 32768 x 2048; here 0.70, 0.72 and 1.29 ms (0.80, 0.77, 1.47 with the
-// moduli innermost).
-template <bool BF, bool UNITS = false>
+template <bool BF>
 __global__ void __launch_bounds__(kI8Threads, 1)
     i8_gemm2_kernel(const __grid_constant__ CUtensorMap mapA,
                     const __grid_constant__ CUtensorMap mapB,
@@ -120,9 +80,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
-  uint8_t* boxes = smem + kI8P2Stages * kI8P2StageBytes;
-  uint64_t* full_bar =
-      reinterpret_cast<uint64_t*>(boxes + (UNITS ? kI8EpiWarps * kI8P2BoxBytes : 0));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kI8P2Stages * kI8P2StageBytes);
   uint64_t* empty_bar = full_bar + kI8P2Stages;
   uint64_t* tfull_bar = empty_bar + kI8P2Stages;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -138,7 +96,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   {
     I8Cursor cur;
     I8Item probe;
-    if (!i8p2_next<UNITS>(p, cl, ncl, rank, cur, probe)) return;
+    if (!i8p2_next_item(p, cl, ncl, rank, cur, probe)) return;
   }
 
   if (threadIdx.x == 0) {
@@ -171,7 +129,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     if (lane == 0) {
       tma_prefetch_desc(&mapA);
       tma_prefetch_desc(&mapB);
-      if (UNITS || p.T1 > 0) tma_prefetch_desc(&mapB2);
+      if (p.T1 > 0) tma_prefetch_desc(&mapB2);
       int stage = 0;
       uint32_t phase = 0;
       I8Cursor cur;
@@ -179,7 +137,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       const int half = p.bn / 2;
       const uint32_t tx = 2 * (kI8P2TileBytes + (uint32_t)half * kI8BK);  // both CTAs' loads
       I8Item it;
-      while (!*abort_flag && i8p2_next<UNITS>(p, cl, ncl, rank, cur, it)) {
+      while (!*abort_flag && i8p2_next_item(p, cl, ncl, rank, cur, it)) {
         const CUtensorMap* mb = (p.T1 > 0 && it.t >= p.T1) ? &mapB2 : &mapB;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err)) {
@@ -226,7 +184,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       uint32_t acc_phase = 0;
       I8Cursor cur;
       I8Item it;
-      while (!*abort_flag && i8p2_next<UNITS>(p, cl, ncl, rank, cur, it)) {
+      while (!*abort_flag && i8p2_next_item(p, cl, ncl, rank, cur, it)) {
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err)) {
           *abort_flag = 1;
           break;
@@ -277,7 +235,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     int32_t run[BF ? 128 : 1];
 #pragma unroll
     for (int j = 0; j < (BF ? 128 : 1); ++j) run[j] = 0;
-    while (i8p2_next<UNITS>(p, cl, ncl, rank, cur, it)) {
+    while (i8p2_next_item(p, cl, ncl, rank, cur, it)) {
       if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err)) {
         *abort_flag = 1;
         break;
@@ -285,56 +243,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kI8BN);
       int32_t* dst = p.partials + ((int64_t)it.slot * kI8BM + row_in_tile) * kI8BN;
-      if constexpr (UNITS) {
-        const int half = (warp - 2) >> 2;
-        uint8_t* box = boxes + (warp - 2) * kI8P2BoxBytes;
-        uint8_t* my_row = box + lane * 128;
-        const int sw = lane & 7;  // 128-byte swizzle of this box row
-        const int x = it.tn * kI8BN + half * 128, y = it.tm * kI8BM + quarter * 32;
-        // The box is free once the previous unit's store has read it.
-        if (lane == 0) bulk_wait_read_all();
-        __syncwarp();
-        if (x < p.N && y < p.M) {
-          const uint32_t m = c_i8mod.m[it.l], magic = c_i8mod.magic[it.l];
-          const uint32_t off = c_i8mod.offset[it.l];
-#pragma unroll 1
-          for (int c = 0; c < 4; c += 2) {
-            uint32_t v0[32], v1[32];
-            tmem_ld_32x32b_x32(taddr + half * 128 + c * 32, v0);
-            tmem_ld_32x32b_x32(taddr + half * 128 + c * 32 + 32, v1);
-            tmem_ld_wait();
-            if (m != 256u) {  // m = 256: the accumulator's low byte
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                v0[j] = mod_exact29(v0[j] + off, m, magic);
-                v1[j] = mod_exact29(v1[j] + off, m, magic);
-              }
-            }
-            uint32_t w[16];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              w[j] = __byte_perm(__byte_perm(v0[4 * j], v0[4 * j + 1], 0x0040),
-                                 __byte_perm(v0[4 * j + 2], v0[4 * j + 3], 0x0040), 0x5410);
-              w[8 + j] = __byte_perm(__byte_perm(v1[4 * j], v1[4 * j + 1], 0x0040),
-                                     __byte_perm(v1[4 * j + 2], v1[4 * j + 3], 0x0040), 0x5410);
-            }
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-              *reinterpret_cast<uint4*>(my_row + (((2 * c + h) ^ sw) << 4)) =
-                  make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
-          }
-        }
-        tc_fence_before();
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive_remote(tempty0 + acc * 8);
-          if (x < p.N && y < p.M) {
-            tma_store_3d(&mapB2, box, x, y, it.l);
-            bulk_commit_group();
-          }
-        }
-      } else if (BF) {
+      if (BF) {
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
           uint32_t v[16];
@@ -358,15 +267,13 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       }
       // The accumulator is free as soon as it has been read: one arrival per
       // warp on rank 0's tempty barrier (remote for rank 1).
-      if (!UNITS) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(tempty0 + acc * 8);
-      }
-      if (BF && !UNITS) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(tempty0 + acc * 8);
+      if (BF) {
         I8Item nx;
         I8Cursor peek = cur;
-        if (!i8p2_next<UNITS>(p, cl, ncl, rank, peek, nx) || nx.slot != it.slot) {
+        if (!i8p2_next_item(p, cl, ncl, rank, peek, nx) || nx.slot != it.slot) {
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {
             int4* d4 = reinterpret_cast<int4*>(dst + (c_begin + cc) * 32);
@@ -386,7 +293,6 @@ __global__ void __launch_bounds__(kI8Threads, 1)
         acc_phase ^= 1;
       }
     }
-    if (UNITS && lane == 0) bulk_wait_all();
   }
 
   // Teardown: every role's loop is bounded, so every thread of both CTAs

@@ -94,8 +94,7 @@ struct I8Params {
   // `tiles`, which then holds both halves of every pair).
   int T2;
   const int4* pairs;
-  int bn;        // columns of a pair tile: a multiple of 32, at most 256
-  int tiles_m2;  // kSchedUnits on CTA pairs: 256-row tiles
+  int bn;  // columns of a pair tile: a multiple of 32, at most 256
 };
 
 // Moduli and the constants of an exact remainder by multiply-high: with

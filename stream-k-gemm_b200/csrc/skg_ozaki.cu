@@ -1141,12 +1141,11 @@ bool lanes_pair_enabled() {
   return v == 1;
 }
 
-cudaLaunchConfig_t pair_config(int grid, cudaStream_t s, cudaLaunchAttribute* attr,
-                               bool units = false) {
+cudaLaunchConfig_t pair_config(int grid, cudaStream_t s, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kI8Threads);
-  cfg.dynamicSmemBytes = units ? kI8P2UnitsSmemBytes : kI8P2SmemBytes;
+  cfg.dynamicSmemBytes = kI8P2SmemBytes;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
@@ -1157,17 +1156,16 @@ cudaLaunchConfig_t pair_config(int grid, cudaStream_t s, cudaLaunchAttribute* at
   return cfg;
 }
 
-template <bool BF, bool UNITS = false>
+template <bool BF>
 int pair_setup(DeviceState* dev, int* clusters) {
   static int ncl[64] = {0};
   if (!ncl[dev->device]) {
-    SKG_CUDA(cudaFuncSetAttribute(i8_gemm2_kernel<BF, UNITS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  UNITS ? kI8P2UnitsSmemBytes : kI8P2SmemBytes));
+    SKG_CUDA(cudaFuncSetAttribute(i8_gemm2_kernel<BF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kI8P2SmemBytes));
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = pair_config(2 * (dev->num_sms / 2), nullptr, attr, UNITS);
+    cudaLaunchConfig_t cfg = pair_config(2 * (dev->num_sms / 2), nullptr, attr);
     int n = 0;
-    SKG_CUDA(cudaOccupancyMaxActiveClusters(&n, (const void*)i8_gemm2_kernel<BF, UNITS>, &cfg));
+    SKG_CUDA(cudaOccupancyMaxActiveClusters(&n, (const void*)i8_gemm2_kernel<BF>, &cfg));
     if (n < 1) return fail(SKGEMM_ERR_CUDA, "INT8 pair kernel: no cluster of two fits");
     ncl[dev->device] = n;
   }
@@ -1183,13 +1181,13 @@ int lanes_pair_units(DeviceState* dev, bool bf) {
   return n;
 }
 
-template <bool BF, bool UNITS = false>
+template <bool BF>
 int launch_i8_pair_t(const CUtensorMap& mA, const CUtensorMap& mB, const CUtensorMap& mB2,
                      const I8Params& p, int clusters, cudaStream_t s) {
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = pair_config(2 * clusters, s, attr, UNITS);
-  KernelTimer kt_(s, UNITS ? "i8_gemm2_units_kernel" : "i8_gemm2_kernel");
-  SKG_CUDA(cudaLaunchKernelEx(&cfg, i8_gemm2_kernel<BF, UNITS>, mA, mB, mB2, p));
+  cudaLaunchConfig_t cfg = pair_config(2 * clusters, s, attr);
+  KernelTimer kt_(s, "i8_gemm2_kernel");
+  SKG_CUDA(cudaLaunchKernelEx(&cfg, i8_gemm2_kernel<BF>, mA, mB, mB2, p));
   return SKGEMM_OK;
 }
 
@@ -1996,20 +1994,18 @@ int ozaki_rot(int64_t Nd, int64_t nb, const double* A, const double* Q, double* 
   CUtensorMap mA, mB;
   if ((st = make_res_map(&mA, os->res_a.ptr, KPb, RA, L, kI8BM))) return st;
   if ((st = make_res_map(&mB, os->res_b.ptr, KPb, RB, L, kI8BN))) return st;
-  // Residue bytes [L][Nd][nb], written by 32 x 128-byte TMA store boxes where the
-  // output is at least a box.
-  const bool boxed = !bf && nb % 16 == 0 && nb >= 128 && Nd >= 128;
-  CUtensorMap mR;
-  if (boxed) {
-    uint64_t dims[3] = {(uint64_t)nb, (uint64_t)Nd, (uint64_t)L};
-    uint64_t strides[2] = {(uint64_t)nb, (uint64_t)(Nd * nb)};
-    uint32_t box[3] = {128, 32, 1};
-    if ((st = encode_tiled(&mR, 3, os->rbytes.ptr, dims, strides, box,
-                           CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B)))
-      return st;
-  }
-  if (boxed && KP / 128 <= kI8RotKbMax) {
-    // B_l[tn] fits in shared memory: the B-resident schedule.
+  if (!bf && KP / 128 <= kI8RotKbMax && nb % 16 == 0 && nb >= 128 && Nd >= 128) {
+    // B_l[tn] fits in shared memory: the B-resident schedule, residue bytes
+    // [L][Nd][nb] written by 32 x 128-byte TMA store boxes.
+    CUtensorMap mR;
+    {
+      uint64_t dims[3] = {(uint64_t)nb, (uint64_t)Nd, (uint64_t)L};
+      uint64_t strides[2] = {(uint64_t)nb, (uint64_t)(Nd * nb)};
+      uint32_t box[3] = {128, 32, 1};
+      if ((st = encode_tiled(&mR, 3, os->rbytes.ptr, dims, strides, box,
+                             CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B)))
+        return st;
+    }
     I8RotParams p;
     memset(&p, 0, sizeof(p));
     p.L = L;
@@ -2036,22 +2032,9 @@ int ozaki_rot(int64_t Nd, int64_t nb, const double* A, const double* Q, double* 
     p.residues = (uint8_t*)os->rbytes.ptr;
     p.ldr = nb;
     p.err = ws->err;
-    int ncl = 0;
-    if (boxed && lanes_pair_enabled() && (st = pair_setup<false, true>(dev, &ncl))) return st;
-    if (ncl > 0) {
-      // nb > 512: CTA pairs (65536 x 1024: 0.72 ms, 0.87 on one CTA).
-      p.bn = kI8BN;
-      p.tiles_m2 = (p.tiles_m + 1) / 2;
-      if ((st = make_res_map(&mB, os->res_b.ptr, KPb, RB, L, p.bn / 2))) return st;
-      const int64_t items = (int64_t)p.tiles_m2 * L * p.tiles_n;
-      if ((st = launch_i8_pair_t<false, true>(mA, mB, mR, p, (int)std::min<int64_t>(ncl, items),
-                                              s)))
-        return st;
-    } else {
-      const int64_t units = (int64_t)p.tiles_m * L * p.tiles_n;
-      const int grid = (int)std::min<int64_t>(dev->num_sms, units);
-      if ((st = launch_i8(dev, mA, mB, p, grid, s, bf))) return st;
-    }
+    const int64_t units = (int64_t)p.tiles_m * L * p.tiles_n;
+    const int grid = (int)std::min<int64_t>(dev->num_sms, units);
+    if ((st = launch_i8(dev, mA, mB, p, grid, s, bf))) return st;
   }
   {
     const uint8_t* rb = (const uint8_t*)os->rbytes.ptr;

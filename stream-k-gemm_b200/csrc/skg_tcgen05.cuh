@@ -167,13 +167,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
 }
-// The same arrival with the default (CTA-scope release) semantics, for an
-// accumulator handed back after tcgen05.wait::ld and a tcgen05 fence, where no
-// other memory has to become visible; the cluster-scope release above waits for
-// a memory barrier.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
 // All threads of both CTAs (release / acquire at cluster scope).
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
