@@ -50,13 +50,43 @@ int debug_poison(void* p, size_t bytes, cudaStream_t s) {
   return SKGEMM_OK;
 }
 
+namespace {
+// The current device's stream for table uploads (created on first use).
+int table_stream(cudaStream_t* s) {
+  static std::mutex mu;
+  static cudaStream_t streams[64] = {};
+  int d = 0;
+  SKG_CUDA(cudaGetDevice(&d));
+  if (d < 0 || d >= 64) return fail(SKGEMM_ERR_NO_DEVICE, "device index out of range");
+  std::lock_guard<std::mutex> lk(mu);
+  if (!streams[d]) SKG_CUDA(cudaStreamCreateWithFlags(&streams[d], cudaStreamNonBlocking));
+  *s = streams[d];
+  return SKGEMM_OK;
+}
+}  // namespace
+
+int upload_table(void* dst, const void* src, size_t bytes) {
+  cudaStream_t s = nullptr;
+  if (int st = table_stream(&s)) return st;
+  SKG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  SKG_CUDA(cudaStreamSynchronize(s));
+  return SKGEMM_OK;
+}
+
+int fill_table(void* dst, int byte, size_t bytes) {
+  cudaStream_t s = nullptr;
+  if (int st = table_stream(&s)) return st;
+  SKG_CUDA(cudaMemsetAsync(dst, byte, bytes, s));
+  SKG_CUDA(cudaStreamSynchronize(s));
+  return SKGEMM_OK;
+}
+
 int DeviceBuffer::ensure(size_t need) {
   if (need <= bytes) return SKGEMM_OK;
   release();
   SKG_CUDA(cudaMalloc(&ptr, need));
   bytes = need;
-  if (debug_fill_enabled()) SKG_CUDA(cudaMemset(ptr, 0xFF, need));
-  return SKGEMM_OK;
+  return debug_fill_enabled() ? fill_table(ptr, 0xFF, need) : SKGEMM_OK;
 }
 
 void DeviceBuffer::release() {

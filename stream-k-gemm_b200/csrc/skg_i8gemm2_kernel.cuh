@@ -59,6 +59,7 @@ __device__ __forceinline__ bool i8p2_next_item(const I8Params& p, int cl, int nc
       continue;
     }
     const I8Segment s = p.segs[idx];
+    if (!i8_segment_ok(p, s)) return false;
     const int4 pr = p.pairs[t2];
     it.l = s.l;
     it.kb0 = s.kb0;
@@ -92,12 +93,10 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   const int rank = (int)cluster_ctarank();
   const int cl = blockIdx.x >> 1, ncl = gridDim.x >> 1;
 
-  // Clusters with no work leave together (both ranks see the same items).
-  {
-    I8Cursor cur;
-    I8Item probe;
-    if (!i8p2_next_item(p, cl, ncl, rank, cur, probe)) return;
-  }
+  // Clusters with no work leave, both ranks together: the test reads launch
+  // parameters only. A rank that left alone would leave the other one in the pair's
+  // TMEM allocation, the one wait here that has no bound.
+  if (cl >= p.T2 * p.Q) return;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kI8P2Stages; ++s) {

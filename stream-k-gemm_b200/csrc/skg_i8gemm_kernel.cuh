@@ -83,6 +83,7 @@ struct I8Params {
   const int2* tiles;            // [T] (tm, tn)
   const int* lane_seg_off;      // [Q+1] offsets into segs
   const I8Segment* segs;        // segments of all lanes
+  int slots;                    // partial slots of the plan
   int32_t* partials;            // [slots][T][128][256]
   // kSchedUnits
   int tiles_m, tiles_n;
@@ -143,6 +144,17 @@ struct I8Cursor {
   int seg = 0;
 };
 
+// A segment inside the problem. Tables that are not what the host built would
+// otherwise drive loops and stores of any length: the role that meets one stops,
+// and the bounded waits of the others end.
+__device__ __forceinline__ bool i8_segment_ok(const I8Params& p, const I8Segment& s) {
+  if ((uint32_t)s.l < (uint32_t)p.L && s.kb0 >= 0 && s.kb0 <= s.kb1 && s.kb1 <= p.KB &&
+      (uint32_t)s.slot < (uint32_t)p.slots)
+    return true;
+  atomicOr(p.err, kDevErrBadSchedule);
+  return false;
+}
+
 __device__ __forceinline__ bool i8_next_item(const I8Params& p, int cta, I8Cursor& cur,
                                              I8Item& it) {
   if (p.sched == kSchedLanes) {
@@ -161,6 +173,7 @@ __device__ __forceinline__ bool i8_next_item(const I8Params& p, int cta, I8Curso
         continue;
       }
       const I8Segment s = p.segs[idx];
+      if (!i8_segment_ok(p, s)) return false;
       const int2 tt = p.tiles[t];
       it.l = s.l;
       it.kb0 = s.kb0;

@@ -1092,7 +1092,13 @@ int get_lane_plan(DeviceState* dev, int M, int N, int KB, int L, bool syrk, int 
   memcpy(host.data() + s0 + s1 + s2, tile_index.data(), tile_index.size() * sizeof(int));
   memcpy(host.data() + s0 + s1 + s2 + s3, mod_off.data(), mod_off.size() * sizeof(int));
   memcpy(host.data() + s0 + s1 + s2 + s3 + s4, mod_slots.data(), mod_slots.size() * sizeof(int));
-  SKG_CUDA(cudaMemcpy(b, host.data(), host.size(), cudaMemcpyHostToDevice));
+  // Complete before any stream's kernel reads it: the conversion of a small operand is
+  // done before a copy on the default stream need be.
+  if ((st = upload_table(b, host.data(), host.size()))) {
+    pl->buf.release();
+    delete pl;
+    return st;
+  }
   pl->tiles = reinterpret_cast<int2*>(b);
   pl->lane_seg_off = reinterpret_cast<int*>(b + s0);
   pl->segs = reinterpret_cast<I8Segment*>(b + s0 + s1);
@@ -1217,6 +1223,7 @@ int launch_lanes(DeviceState* dev, const LanePlan* pl, const void* resA, int64_t
   p.tiles = pl->tiles;
   p.lane_seg_off = pl->lane_seg_off;
   p.segs = pl->segs;
+  p.slots = pl->slots;
   p.T2 = pl->T2;
   p.pairs = pl->pairs;
   p.bn = pl->bn;

@@ -47,6 +47,14 @@ int cuda_fail(cudaError_t e, const char* what);
 bool debug_fill_enabled();
 int debug_poison(void* p, size_t bytes, cudaStream_t s);
 
+// Host -> device copy of a table (up to any size) and byte fill of device memory
+// that the kernels of every stream may follow: the copy or fill has finished when the
+// call returns. cudaMemcpy from pageable memory may return before its transfer, and
+// cudaMemset does; both run on the default stream, which non-blocking streams do
+// not wait for.
+int upload_table(void* dst, const void* src, size_t bytes);
+int fill_table(void* dst, int byte, size_t bytes);
+
 struct DeviceBuffer {
   void* ptr = nullptr;
   size_t bytes = 0;
