@@ -334,16 +334,14 @@ int configure(BatchPlan* P, Config c) {
     const size_t slots = (size_t)fixup_slots(grid, 1);
     if ((st = P->d_part.ensure(slots * BM * BN * sizeof(double)))) return st;
     if ((st = P->d_flags.ensure(slots * sizeof(uint32_t)))) return st;
-    SKG_CUDA(cudaMemcpy(P->d_probs.ptr, hp.data(), hp.size() * sizeof(Fp64Params),
-                        cudaMemcpyHostToDevice));
-    SKG_CUDA(cudaMemcpy(P->d_maps.ptr, hm.data(), hm.size() * sizeof(CUtensorMap),
-                        cudaMemcpyHostToDevice));
-    SKG_CUDA(cudaMemcpy(P->d_iters.ptr, hb.data(), hb.size() * sizeof(int64_t),
-                        cudaMemcpyHostToDevice));
+    if ((st = upload_table(P->d_probs.ptr, hp.data(), hp.size() * sizeof(Fp64Params))) ||
+        (st = upload_table(P->d_maps.ptr, hm.data(), hm.size() * sizeof(CUtensorMap))) ||
+        (st = upload_table(P->d_iters.ptr, hb.data(), hb.size() * sizeof(int64_t))))
+      return st;
   }
   if (!P->d_err.ptr) {
     if ((st = P->d_err.ensure(sizeof(uint32_t)))) return st;
-    SKG_CUDA(cudaMemset(P->d_err.ptr, 0, sizeof(uint32_t)));
+    if ((st = fill_table(P->d_err.ptr, 0, sizeof(uint32_t)))) return st;
   }
   G.probs = (const Fp64Params*)P->d_probs.ptr;
   G.maps = (const CUtensorMap*)P->d_maps.ptr;
@@ -451,7 +449,7 @@ int read_err(BatchPlan* P) {
   uint32_t word = 0;
   SKG_CUDA(cudaMemcpy(&word, P->d_err.ptr, sizeof(word), cudaMemcpyDeviceToHost));
   if (word == 0) return SKGEMM_OK;
-  SKG_CUDA(cudaMemset(P->d_err.ptr, 0, sizeof(uint32_t)));
+  if (int st = fill_table(P->d_err.ptr, 0, sizeof(uint32_t))) return st;
   char buf[160];
   snprintf(buf, sizeof(buf), "batched launch: device-side wait ran past its budget (0x%x)", word);
   return fail(SKGEMM_ERR_DEVICE_TIMEOUT, buf);
@@ -888,7 +886,7 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
     if ((st = sl.flags.ensure(nflags * sizeof(uint32_t)))) return st;
     if (!sl.err.ptr) {
       if ((st = sl.err.ensure(sizeof(uint32_t)))) return st;
-      SKG_CUDA(cudaMemset(sl.err.ptr, 0, sizeof(uint32_t)));
+      if ((st = fill_table(sl.err.ptr, 0, sizeof(uint32_t)))) return st;
     }
     if (!sl.ev) SKG_CUDA(cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming));
   }
@@ -960,7 +958,7 @@ int group_ring_error(GroupRing* R) {
     uint32_t word = 0;
     SKG_CUDA(cudaMemcpy(&word, sl.err.ptr, sizeof(word), cudaMemcpyDeviceToHost));
     if (word) {
-      SKG_CUDA(cudaMemset(sl.err.ptr, 0, sizeof(uint32_t)));
+      if (int st = fill_table(sl.err.ptr, 0, sizeof(uint32_t))) return st;
       char buf[120];
       snprintf(buf, sizeof(buf), "grouped launch: device-side wait ran past its budget (0x%x)",
                word);

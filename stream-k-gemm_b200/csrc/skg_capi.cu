@@ -105,13 +105,14 @@ int StreamWorkspace::ensure(size_t slots, size_t nflags) {
   flags = nullptr;
   partial_slots = num_flags = 0;
   SKG_CUDA(cudaMalloc(&partials, slots * kBM * kBN * sizeof(double)));
-  if (debug_fill_enabled())
-    SKG_CUDA(cudaMemset(partials, 0xFF, slots * kBM * kBN * sizeof(double)));
+  int st;
+  if (debug_fill_enabled() && (st = fill_table(partials, 0xFF, slots * kBM * kBN * sizeof(double))))
+    return st;
   SKG_CUDA(cudaMalloc(&flags, nflags * sizeof(uint32_t)));
-  SKG_CUDA(cudaMemset(flags, 0, nflags * sizeof(uint32_t)));
+  if ((st = fill_table(flags, 0, nflags * sizeof(uint32_t)))) return st;
   if (!err) {
     SKG_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
-    SKG_CUDA(cudaMemset(err, 0, sizeof(uint32_t)));
+    if ((st = fill_table(err, 0, sizeof(uint32_t)))) return st;
   }
   partial_slots = slots;
   num_flags = nflags;
@@ -172,7 +173,7 @@ int consume_device_error(StreamWorkspace* ws, cudaStream_t s) {
   uint32_t word = 0;
   SKG_CUDA(cudaMemcpy(&word, ws->err, sizeof(word), cudaMemcpyDeviceToHost));
   if (word == 0) return SKGEMM_OK;
-  SKG_CUDA(cudaMemset(ws->err, 0, sizeof(uint32_t)));
+  if (int st = fill_table(ws->err, 0, sizeof(uint32_t))) return st;
   char buf[160];
   snprintf(buf, sizeof(buf), "device-side wait ran past its budget (error word 0x%x)", word);
   return fail(SKGEMM_ERR_DEVICE_TIMEOUT, buf);

@@ -355,8 +355,7 @@ template <typename T>
 int upload(T** dst, const std::vector<T>& v) {
   if (v.empty()) return SKGEMM_OK;
   SKG_CUDA(cudaMalloc(dst, v.size() * sizeof(T)));
-  SKG_CUDA(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return SKGEMM_OK;
+  return upload_table(*dst, v.data(), v.size() * sizeof(T));
 }
 
 void release(skgemm_nloc* h) {

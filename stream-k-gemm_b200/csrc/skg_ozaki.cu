@@ -880,6 +880,13 @@ I8ModConsts g_modc;
 bool g_modc_ready = false;
 
 
+template <class T>
+int upload_symbol(const T& symbol, const void* src, size_t bytes) {
+  void* p = nullptr;
+  SKG_CUDA(cudaGetSymbolAddress(&p, symbol));
+  return upload_table(p, src, bytes);
+}
+
 int ensure_consts(DeviceState* dev) {
   OzakiDevice& od = g_oz[dev->device];
   if (od.consts_ready) return SKGEMM_OK;
@@ -920,15 +927,16 @@ int ensure_consts(DeviceState* dev) {
     g_modc.offset24[l] = (uint32_t)((acc24 + kModuli[l] - 1) / kModuli[l] * kModuli[l]);
   }
   g_modc_ready = true;
-  SKG_CUDA(cudaMemcpyToSymbol(c_i8mod, &g_modc, sizeof(g_modc)));
+  int st;
+  if ((st = upload_symbol(c_i8mod, &g_modc, sizeof(g_modc)))) return st;
   CrtConsts cc[kI8MaxModuli + 1];
   memset(cc, 0, sizeof(cc));
   for (int L = kMinModuli; L <= kI8MaxModuli; ++L) cc[L] = make_crt(L, nullptr);
-  SKG_CUDA(cudaMemcpyToSymbol(c_res, rc, sizeof(rc)));
-  SKG_CUDA(cudaMemcpyToSymbol(c_crt, cc, sizeof(cc)));
+  if ((st = upload_symbol(c_res, rc, sizeof(rc))) || (st = upload_symbol(c_crt, cc, sizeof(cc))))
+    return st;
   double inv_mod[kI8MaxModuli];
   for (int l = 0; l < kI8MaxModuli; ++l) inv_mod[l] = 1.0 / (double)kModuli[l];
-  SKG_CUDA(cudaMemcpyToSymbol(c_inv_mod, inv_mod, sizeof(inv_mod)));
+  if ((st = upload_symbol(c_inv_mod, inv_mod, sizeof(inv_mod)))) return st;
   od.consts_ready = true;
   return SKGEMM_OK;
 }
@@ -2118,7 +2126,7 @@ int igemm_s8(int64_t M, int64_t N, int64_t K, const int8_t* A, int64_t lda, cons
 int probe_i8_peak(DeviceState* dev, double* tops) {
   uint32_t* sink = nullptr;
   SKG_CUDA(cudaMalloc(&sink, 2 * sizeof(uint32_t)));
-  SKG_CUDA(cudaMemset(sink, 0, 2 * sizeof(uint32_t)));
+  if (int st = fill_table(sink, 0, 2 * sizeof(uint32_t))) return st;
   // More shared memory than two CTAs can share: one CTA (one 512-column TMEM
   // allocation) per SM.
   const int smem = 160 * 1024;
