@@ -488,22 +488,24 @@ __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
       pow2_pair(mu[g * 16 + r], s1, s2);
       cur_g = g;
     }
-    const bool ok = mbar_wait(&bar[s], (phase >> s) & 1u, err);
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], (phase >> s) & 1u, err))) {
+      // A lost load: the warp stops at its first wait that runs out, stores nothing
+      // more and leaves when the loads behind it have landed.
+      for (int j = 1; j < kConvStages && n + j < nmine; ++j) {
+        const int sj = (s + j) % kConvStages;
+        mbar_wait(&bar[sj], (phase >> sj) & 1u, err);
+      }
+      return;
+    }
     phase ^= 1u << s;
     constexpr int ES = BF ? 2 : 1;  // bytes per residue
     uint8_t* dst = res + ((g * 16 + r) * KP + kb * 32 + 16 * h) * ES;
     const int64_t lstride = Rpad * KP * ES;
-    if (ok && BF) {
+    if (BF) {
       uint8_t* row = res + ((g * 16 + r) * KP + kb * 32) * 2;
       convert_stage_bf16<L, KM>(buf + s * kConvTile, r, h, s1, s2, row, lstride);
-    } else if (ok) {
-      convert_stage_i8<L, KM>(buf + s * kConvTile, r, h, s1, s2, dst, lstride);
     } else {
-#pragma unroll
-      for (int l = 0; l < L; ++l)
-#pragma unroll
-        for (int e = 0; e < ES; ++e)
-          reinterpret_cast<uint4*>(dst + l * lstride)[e] = make_uint4(0, 0, 0, 0);
+      convert_stage_i8<L, KM>(buf + s * kConvTile, r, h, s1, s2, dst, lstride);
     }
     __syncwarp();  // stage s consumed by every lane before it is refilled
     s = (s + 1) % kConvStages;
@@ -584,7 +586,9 @@ __global__ void __launch_bounds__(kShortThreads, 3) convert_short_kernel(
       }
       red[kl * 16 + r] = acc;
     }
-    __syncthreads();
+    // A lost load: the CTA stores nothing more and leaves at the first wait that runs
+    // out (only this group's loads are in flight).
+    if (!__syncthreads_and(ok)) return;
     if (threadIdx.x < 16) {
       double part = 0.0;
       for (int j = 0; j < 16; ++j) part += red[j * 16 + threadIdx.x];
@@ -605,15 +609,10 @@ __global__ void __launch_bounds__(kShortThreads, 3) convert_short_kernel(
     const int64_t lstride = Rpad * KP * ES;
     for (int kb = warp; kb < KB; kb += kShortThreads / 32) {
       uint8_t* row = res + ((g * 16 + r) * KP + kb * 32) * ES;
-      if (ok && BF) {
+      if (BF)
         convert_stage_bf16<L, KM>(tiles + kb * kConvTile, r, h, s1, s2, row, lstride);
-      } else if (ok) {
+      else
         convert_stage_i8<L, KM>(tiles + kb * kConvTile, r, h, s1, s2, row + 16 * h, lstride);
-      } else {
-        for (int l = 0; l < L; ++l)
-          for (int e = 0; e < ES; ++e)
-            reinterpret_cast<uint4*>(row + 16 * h * ES + l * lstride)[e] = make_uint4(0, 0, 0, 0);
-      }
     }
     __syncthreads();  // the tiles (and sc, red) are consumed before the next group
   }
