@@ -450,9 +450,7 @@ int read_err(BatchPlan* P) {
   SKG_CUDA(cudaMemcpy(&word, P->d_err.ptr, sizeof(word), cudaMemcpyDeviceToHost));
   if (word == 0) return SKGEMM_OK;
   if (int st = fill_table(P->d_err.ptr, 0, sizeof(uint32_t))) return st;
-  char buf[160];
-  snprintf(buf, sizeof(buf), "batched launch: device-side wait ran past its budget (0x%x)", word);
-  return fail(SKGEMM_ERR_DEVICE_TIMEOUT, buf);
+  return fail(SKGEMM_ERR_DEVICE_TIMEOUT, "batched launch: " + device_error_text(word));
 }
 
 int build_plan(const skgemm_batch_item_t* items, int n, BatchPlan* P) {
@@ -959,10 +957,7 @@ int group_ring_error(GroupRing* R) {
     SKG_CUDA(cudaMemcpy(&word, sl.err.ptr, sizeof(word), cudaMemcpyDeviceToHost));
     if (word) {
       if (int st = fill_table(sl.err.ptr, 0, sizeof(uint32_t))) return st;
-      char buf[120];
-      snprintf(buf, sizeof(buf), "grouped launch: device-side wait ran past its budget (0x%x)",
-               word);
-      return fail(SKGEMM_ERR_DEVICE_TIMEOUT, buf);
+      return fail(SKGEMM_ERR_DEVICE_TIMEOUT, "grouped launch: " + device_error_text(word));
     }
   }
   return SKGEMM_OK;

@@ -174,9 +174,27 @@ int consume_device_error(StreamWorkspace* ws, cudaStream_t s) {
   SKG_CUDA(cudaMemcpy(&word, ws->err, sizeof(word), cudaMemcpyDeviceToHost));
   if (word == 0) return SKGEMM_OK;
   if (int st = fill_table(ws->err, 0, sizeof(uint32_t))) return st;
-  char buf[160];
-  snprintf(buf, sizeof(buf), "device-side wait ran past its budget (error word 0x%x)", word);
-  return fail(SKGEMM_ERR_DEVICE_TIMEOUT, buf);
+  return fail(SKGEMM_ERR_DEVICE_TIMEOUT, device_error_text(word));
+}
+
+std::string device_error_text(uint32_t word) {
+  std::string s;
+  auto add = [&](uint32_t bit, const char* what) {
+    if (word & bit) s += (s.empty() ? "" : ", ") + std::string(what);
+  };
+  add(kDevErrMbarTimeout | kDevErrFixupTimeout, "device-side wait ran past its budget");
+  add(kDevErrBadSchedule, "schedule table outside the problem");
+  const struct {
+    uint32_t bit;
+    const char* kernel;
+  } in[] = {{kDevErrFp64, "fp64"},           {kDevErrConvert, "convert_tma_kernel"},
+            {kDevErrConvertShort, "convert_short_kernel"}, {kDevErrI8, "i8_gemm_kernel"},
+            {kDevErrI8Pair, "i8_gemm2_kernel"}, {kDevErrI8Rot, "i8_rot_kernel"},
+            {kDevErrStencil, "stencil_staged_kernel"}};
+  for (const auto& k : in) add(k.bit, k.kernel);
+  char buf[40];
+  snprintf(buf, sizeof(buf), " (error word 0x%x)", word);
+  return s + buf;
 }
 
 // ------------------------------------------------------- kernel timing

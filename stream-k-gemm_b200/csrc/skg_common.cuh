@@ -24,6 +24,14 @@ enum DeviceError : uint32_t {
   kDevErrMbarTimeout = 1u << 0,   // an mbarrier wait exceeded its iteration cap
   kDevErrFixupTimeout = 1u << 1,  // a Stream-K partial-tile flag never arrived
   kDevErrBadSchedule = 1u << 2,   // schedule arithmetic produced an impossible segment
+  // The kernel whose mbarrier wait ran out (set beside kDevErrMbarTimeout).
+  kDevErrFp64 = 1u << 8,
+  kDevErrConvert = 1u << 9,
+  kDevErrConvertShort = 1u << 10,
+  kDevErrI8 = 1u << 11,
+  kDevErrI8Pair = 1u << 12,
+  kDevErrI8Rot = 1u << 13,
+  kDevErrStencil = 1u << 14,
 };
 
 // Budgets of the spin loops. An mbarrier wait normally completes within
@@ -81,22 +89,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: returns false (and records the error) when `budget_ns` of
-// device time or kMbarSpinCap polls run out.
+// Bounded wait: returns false (and records the error, with the kernel's `code`) when
+// `budget_ns` of device time or kMbarSpinCap polls run out.
 __device__ __forceinline__ bool mbar_wait_ns(uint64_t* bar, uint32_t parity, uint32_t* err,
-                                             uint64_t budget_ns) {
+                                             uint64_t budget_ns, uint32_t code = 0) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t it = 1; it < kMbarSpinCap; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 255u) == 0 && globaltimer_ns() - t0 > budget_ns) break;
   }
-  if (err) atomicOr(err, kDevErrMbarTimeout);
+  if (err) atomicOr(err, kDevErrMbarTimeout | code);
   return false;
 }
 // The kernels' wait: the 8 s budget.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err) {
-  return mbar_wait_ns(bar, parity, err, kMbarBudgetNs);
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err,
+                                          uint32_t code) {
+  return mbar_wait_ns(bar, parity, err, kMbarBudgetNs, code);
 }
 
 // --------------------------------------------------------------------------

@@ -360,7 +360,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
           prefetched = sg.pid;
         }
         for (int k = sg.kb; k < sg.ke; ++k) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, S.err())) *abort_flag = 1;
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, S.err(), kDevErrFp64)) *abort_flag = 1;
           if (*abort_flag) break;
           uint8_t* sa = smem + stage * TS::kStage;
           uint8_t* sb = sa + TS::kABytes;
@@ -440,7 +440,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     // 1.617, 1.617, 1.616 / 0.930, 0.923, 0.923 / 1.685, 1.680, 1.681).
 #pragma unroll 3
     for (int k = sg.kb; k < sg.ke && !aborted; ++k) {
-      if (!mbar_wait(&full_bar[stage], phase, S.err())) {
+      if (!mbar_wait(&full_bar[stage], phase, S.err(), kDevErrFp64)) {
         aborted = true;
         *abort_flag = 1;
         break;

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       while (!*abort_flag && i8p2_next_item(p, cl, ncl, rank, cur, it)) {
         const CUtensorMap* mb = (p.T1 > 0 && it.t >= p.T1) ? &mapB2 : &mapB;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err)) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err, kDevErrI8Pair)) {
             *abort_flag = 1;
             break;
           }
@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           ph ^= 1;
         }
         if (rank == 0)
-          mbar_wait(&full_bar[s2], ph, p.err);
+          mbar_wait(&full_bar[s2], ph, p.err, kDevErrI8Pair);
         else
-          mbar_wait(&empty_bar[s2], ph, p.err);
+          mbar_wait(&empty_bar[s2], ph, p.err, kDevErrI8Pair);
       }
     }
   } else if (warp == 1) {
@@ -184,14 +184,14 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       I8Cursor cur;
       I8Item it;
       while (!*abort_flag && i8p2_next_item(p, cl, ncl, rank, cur, it)) {
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err)) {
+        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err, kDevErrI8Pair)) {
           *abort_flag = 1;
           break;
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kI8BN);
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.err)) {
+          if (!mbar_wait(&full_bar[stage], phase, p.err, kDevErrI8Pair)) {
             *abort_flag = 1;
             break;
           }
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 #pragma unroll
     for (int j = 0; j < (BF ? 128 : 1); ++j) run[j] = 0;
     while (i8p2_next_item(p, cl, ncl, rank, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err)) {
+      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Pair)) {
         *abort_flag = 1;
         break;
       }

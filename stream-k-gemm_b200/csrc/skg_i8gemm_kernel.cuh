@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       while (!*abort_flag && i8_next_item(p, cta, cur, it)) {
         const CUtensorMap* mb = (p.T1 > 0 && it.t >= p.T1) ? &mapB2 : &mapB;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err)) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err, kDevErrI8)) {
             *abort_flag = 1;
             break;
           }
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           s2 += kI8Stages;
           ph ^= 1;
         }
-        mbar_wait(&full_bar[s2], ph, p.err);
+        mbar_wait(&full_bar[s2], ph, p.err, kDevErrI8);
       }
     }
   } else if (warp == 1) {
@@ -351,14 +351,14 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       I8Cursor cur;
       I8Item it;
       while (!*abort_flag && i8_next_item(p, cta, cur, it)) {
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err)) {
+        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err, kDevErrI8)) {
           *abort_flag = 1;
           break;
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kI8BN);
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.err)) {
+          if (!mbar_wait(&full_bar[stage], phase, p.err, kDevErrI8)) {
             *abort_flag = 1;
             break;
           }
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 #pragma unroll
     for (int j = 0; j < (BF ? 128 : 1); ++j) run[j] = 0;
     while (i8_next_item(p, cta, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err)) {
+      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8)) {
         *abort_flag = 1;
         break;
       }
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
         if (it.l != cur_l) {
           // B_l[tn] for the next run of units: all k blocks, one barrier.
           if (cur_l >= 0) {
-            if (!mbar_wait(bempty, bempty_ph, p.err)) {
+            if (!mbar_wait(bempty, bempty_ph, p.err, kDevErrI8Rot)) {
               *abort_flag = 1;
               break;
             }
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           cur_l = it.l;
         }
         for (int kb = 0; kb < p.KB; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err)) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.err, kDevErrI8Rot)) {
             *abort_flag = 1;
             break;
           }
@@ -643,9 +643,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           s2 += kI8RotStages;
           ph ^= 1;
         }
-        mbar_wait(&full_bar[s2], ph, p.err);
+        mbar_wait(&full_bar[s2], ph, p.err, kDevErrI8Rot);
       }
-      if (b_loads > 0) mbar_wait(bfull, (uint32_t)((b_loads - 1) & 1), p.err);
+      if (b_loads > 0) mbar_wait(bfull, (uint32_t)((b_loads - 1) & 1), p.err, kDevErrI8Rot);
     }
   } else if (warp == 1) {
     // --------------------------------------------------------- MMA issuer
@@ -664,21 +664,21 @@ __global__ void __launch_bounds__(kI8Threads, 1)
         if (it.l != cur_l) {
           // Every MMA issued so far read the old B: release it once they finish.
           if (cur_l >= 0) umma_commit(bempty);
-          if (!mbar_wait(bfull, bfull_ph, p.err)) {
+          if (!mbar_wait(bfull, bfull_ph, p.err, kDevErrI8Rot)) {
             *abort_flag = 1;
             break;
           }
           bfull_ph ^= 1;
           cur_l = it.l;
         }
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err)) {
+        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.err, kDevErrI8Rot)) {
           *abort_flag = 1;
           break;
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kI8BN);
         for (int kb = 0; kb < p.KB; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.err)) {
+          if (!mbar_wait(&full_bar[stage], phase, p.err, kDevErrI8Rot)) {
             *abort_flag = 1;
             break;
           }
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     int cur = 0;
     I8Item it;
     while (rot_next_item(p, cta, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err)) {
+      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Rot)) {
         *abort_flag = 1;
         break;
       }
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(128, 1) i8_peak_kernel(int iters, uint32_t* si
   }
   __syncwarp();
   if (threadIdx.x < 32) {  // warp 0, converged: tcgen05.ld is warp-collective
-    const bool ok = mbar_wait(done, 0, sink + 1);
+    const bool ok = mbar_wait(done, 0, sink + 1, 0);
     tc_fence_after();
     uint32_t v[32];
     tmem_ld_32x32b_x32(tmem_base, v);

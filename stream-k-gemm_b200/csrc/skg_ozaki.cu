@@ -488,12 +488,12 @@ __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
       pow2_pair(mu[g * 16 + r], s1, s2);
       cur_g = g;
     }
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], (phase >> s) & 1u, err))) {
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], (phase >> s) & 1u, err, kDevErrConvert))) {
       // A lost load: the warp stops at its first wait that runs out, stores nothing
       // more and leaves when the loads behind it have landed.
       for (int j = 1; j < kConvStages && n + j < nmine; ++j) {
         const int sj = (s + j) % kConvStages;
-        mbar_wait(&bar[sj], (phase >> sj) & 1u, err);
+        mbar_wait(&bar[sj], (phase >> sj) & 1u, err, kDevErrConvert);
       }
       return;
     }
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kShortThreads, 3) convert_short_kernel(
           tma_load_3d(tiles + kb * kConvTile, &map, bar, 0, kb * 32, (int)g);
       }
     }
-    const bool ok = mbar_wait(bar, phase, err);
+    const bool ok = mbar_wait(bar, phase, err, kDevErrConvertShort);
     phase ^= 1;
     for (int t = threadIdx.x; t < 256; t += kShortThreads) {  // partial (r, kl) = t
       const int r = t & 15, kl = t >> 4;

@@ -198,6 +198,9 @@ int expire_fixup_wait(DeviceState* dev, double budget_ms, cudaStream_t s);
 // `s` already synchronised).
 int batch_consume_error(DeviceState* dev, cudaStream_t s);
 
+// What a device error word says: the kinds of failure, the kernels that met them and
+// the word itself, "<text> (error word 0x..)".
+std::string device_error_text(uint32_t word);
 // Reads and clears the error word of `ws` (synchronises `s`).
 int consume_device_error(StreamWorkspace* ws, cudaStream_t s);
 

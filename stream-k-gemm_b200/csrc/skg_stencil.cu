@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
       const double* Ak = A + i + (int64_t)(j0 + jl) * ni + k0 * plane_pts;
       for (int u = -kStFills; u < k1 - k0; ++u, ++it) {
         const uint32_t b = it % kStRing;
-        if (it >= kStRing && (*abort_flag || !mbar_wait(&empty[b], (it / kStRing - 1) & 1, err)))
+        if (it >= kStRing && (*abort_flag || !mbar_wait(&empty[b], (it / kStRing - 1) & 1, err, kDevErrStencil)))
           ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
     // the normal path: the consumers waited for every one of them).
     asm volatile("cp.async.wait_all;" ::: "memory");
     for (uint32_t v = it > kStRing ? it - kStRing : 0; v < it; ++v)
-      mbar_wait(&full[v % kStRing], (v / kStRing) & 1, err);
+      mbar_wait(&full[v % kStRing], (v / kStRing) & 1, err, kDevErrStencil);
     return;
   }
 
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
     double2 zqA[kZq], zqB[kZq];
 #pragma unroll
     for (int f = 0; f < kStFills; ++f) {  // planes k0 - 6 .. k0 + 5
-      if (!*abort_flag && !mbar_wait(&full[buf], ph, err)) *abort_flag = 1;
+      if (!*abort_flag && !mbar_wait(&full[buf], ph, err, kDevErrStencil)) *abort_flag = 1;
       const double2* C = reinterpret_cast<const double2*>(stages + buf * kStStage);
 #pragma unroll
       for (int d = 0; d < kStFill; ++d) {
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
 #pragma unroll
       for (int u = 0; u < kZq; ++u) {
         if (kb + u >= k1) break;
-          if (!*abort_flag && !mbar_wait(&full[buf], ph, err)) *abort_flag = 1;
+          if (!*abort_flag && !mbar_wait(&full[buf], ph, err, kDevErrStencil)) *abort_flag = 1;
         const double* st = stages + buf * kStStage;
         const double2* P = reinterpret_cast<const double2*>(st);
         const double2* C = reinterpret_cast<const double2*>(st + kStPlane);
