@@ -838,6 +838,7 @@ struct GroupRing {
     size_t host_bytes = 0;
     cudaEvent_t ev = nullptr;
     bool pending = false;
+    uint32_t* word = nullptr;  // pinned copy of err, taken after the slot's launch
   };
   DeviceState* dev = nullptr;
   std::vector<Slot> slots;
@@ -859,6 +860,7 @@ void group_ring_destroy(GroupRing* R) {
       cudaEventDestroy(sl.ev);
     }
     if (sl.host) cudaFreeHost(sl.host);
+    if (sl.word) cudaFreeHost(sl.word);
     sl.probs.release();
     sl.maps.release();
     sl.iters.release();
@@ -886,13 +888,17 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
       if ((st = sl.err.ensure(sizeof(uint32_t)))) return st;
       if ((st = fill_table(sl.err.ptr, 0, sizeof(uint32_t)))) return st;
     }
+    if (!sl.word) {
+      SKG_CUDA(cudaMallocHost((void**)&sl.word, sizeof(uint32_t)));
+      *sl.word = 0;
+    }
     if (!sl.ev) SKG_CUDA(cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming));
   }
   return SKGEMM_OK;
 }
 
 int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaStream_t s,
-                      int* tile_out) {
+                      int* tile_out, const uint32_t** word_out) {
   if (!R || R->slots.empty()) return fail(SKGEMM_ERR_INVALID_ARG, "null group ring");
   GroupRing::Slot& sl = R->slots[R->next];
   R->next = (R->next + 1) % (int)R->slots.size();
@@ -943,6 +949,10 @@ int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaS
     if (pr.M > 0 && pr.N > 0 && pr.K == 0 && pr.out_kind != kOutBand16)
       if ((st = run_k0(pr.out_kind, pr.M, pr.N, pr.D, pr.ldd, pr.gamma, pr.beta_zero, s)))
         return st;
+  if (word_out) {
+    SKG_CUDA(cudaMemcpyAsync(sl.word, sl.err.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    *word_out = sl.word;
+  }
   SKG_CUDA(cudaEventRecord(sl.ev, s));
   sl.pending = true;
   if (tile_out) *tile_out = tile;

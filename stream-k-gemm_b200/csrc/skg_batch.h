@@ -33,9 +33,11 @@ GroupRing* group_ring_create(DeviceState* dev, int depth);
 void group_ring_destroy(GroupRing* R);
 // Grows every slot for up to `max_problems` problems and the largest grid.
 int group_ring_reserve(GroupRing* R, int max_problems);
-// Enqueues one grouped launch of `probs` (K == 0 problems included) on `s`.
+// Enqueues one grouped launch of `probs` (K == 0 problems included) on `s`, and
+// behind it a copy of its device error word to *word_out (host memory of the slot,
+// valid once the launch has completed, until the slot's next submission).
 int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaStream_t s,
-                      int* tile_out);
+                      int* tile_out, const uint32_t** word_out = nullptr);
 // Reads and clears the slots' error words (call after synchronising).
 int group_ring_error(GroupRing* R);
 

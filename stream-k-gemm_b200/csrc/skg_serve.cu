@@ -194,6 +194,7 @@ struct Req {
 
 struct Batch {
   std::vector<int> s1, s2;  // requests whose S+Hs / rotation run in this launch
+  const uint32_t* word = nullptr;  // the launch's device error word, once it has completed
   double flop = 0.0;
   int problems = 0;
   cudaEvent_t ev = nullptr;
@@ -218,6 +219,9 @@ struct Exec {
   virtual int run_ozaki(Req& r) = 0;
   virtual bool req_ready(Req& r) = 0;
   virtual double req_time(Req& r) = 0;
+  // Device error word of a launch / request that has completed (0: none).
+  virtual uint32_t batch_word(Batch& b) { return b.word ? *b.word : 0; }
+  virtual uint32_t req_word(Req& r) { (void)r; return 0; }
   virtual int finish(Req& r, const skgemm_serve_request_t& io) = 0;
   virtual void idle(double next_arrival) = 0;
   // True when idle() could not move time forward (simulation with nothing
@@ -233,6 +237,7 @@ struct GpuExec : Exec {
   char* arena = nullptr;
   cudaStream_t comp = nullptr, gens = nullptr;
   std::vector<cudaStream_t> slots;
+  uint32_t* words = nullptr;  // pinned: each slot's error word as of its last request
   GroupRing* ring = nullptr;
   cudaEvent_t t0 = nullptr;
   std::chrono::steady_clock::time_point h0;
@@ -295,7 +300,7 @@ struct GpuExec : Exec {
       Req& r = R[i];
       probs.push_back(rot_problem(r.Ng, r.nb, p(r, r.lay.grid), p(r, r.lay.Q), p(r, r.lay.out)));
     }
-    int st = group_ring_submit(ring, probs, comp, nullptr);
+    int st = group_ring_submit(ring, probs, comp, nullptr, &b.word);
     if (st) return st;
     if (!(b.ev = ev())) return fail(SKGEMM_ERR_CUDA, "cudaEventCreate");
     SKG_CUDA(cudaEventRecord(b.ev, comp));
@@ -323,6 +328,11 @@ struct GpuExec : Exec {
     if ((st = skgemm_drot_dev_opt(r.Ng, r.nb, p(r, r.lay.grid), p(r, r.lay.Q), p(r, r.lay.out),
                                   &o, s)))
       return st;
+    // The error word travels behind the request's kernels; it is read when they have
+    // completed.
+    StreamWorkspace* ws = stream_workspace(dev, s, 1, &st);
+    if (!ws) return st;
+    SKG_CUDA(cudaMemcpyAsync(words + r.slot, ws->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (!(r.done_ev = ev())) return fail(SKGEMM_ERR_CUDA, "cudaEventCreate");
     SKG_CUDA(cudaEventRecord(r.done_ev, s));
     return SKGEMM_OK;
@@ -334,6 +344,7 @@ struct GpuExec : Exec {
     give(r.done_ev);
     return ms * 1e-3;
   }
+  uint32_t req_word(Req& r) override { return words[r.slot]; }
   int finish(Req& r, const skgemm_serve_request_t& io) override {
     const size_t n2 = (size_t)r.nb * r.nb * 8, big = (size_t)r.Ng * r.nb * 8;
     const int64_t nb32 = (r.nb + 31) / 32 * 32;
@@ -362,6 +373,7 @@ struct GpuExec : Exec {
     cudaDeviceSynchronize();
     for (cudaStream_t s : slots) skgemm_stream_release(s);
     if (ring) group_ring_destroy(ring);
+    if (words) cudaFreeHost(words);
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
     if (t0) cudaEventDestroy(t0);
     if (arena) cudaFree(arena);
@@ -459,6 +471,20 @@ int schedule(skgemm_serve_request_t* io, int n, skgemm_serve_options_t& o, Exec&
   double last_progress = ex.now();
   constexpr double kStallSeconds = 120.0;
 
+  // "request 3 (Ng 13824, nb 96)".
+  auto name = [&](const Req& r) {
+    char buf[80];
+    snprintf(buf, sizeof(buf), "request %d (Ng %lld, nb %lld)", r.idx, (long long)r.Ng,
+             (long long)r.nb);
+    return std::string(buf);
+  };
+  // A failure while work may still be in flight: said at once, because the caller's
+  // teardown waits for the device.
+  auto broken = [&](const std::string& what) {
+    fprintf(stderr, "skgemm serve: %s\n", what.c_str());
+    return fail(SKGEMM_ERR_DEVICE_TIMEOUT, "serve: " + what);
+  };
+
   auto complete = [&](Req& r, double t) -> int {
     r.done = t;
     r.state = kDone;
@@ -486,6 +512,12 @@ int schedule(skgemm_serve_request_t* io, int n, skgemm_serve_options_t& o, Exec&
         Batch b = flight.front();
         flight.pop_front();
         const double bt = ex.batch_time(b);
+        if (const uint32_t w = ex.batch_word(b)) {
+          std::string who;
+          for (const auto* v : {&b.s1, &b.s2})
+            for (int i : *v) who += (who.empty() ? "" : ", ") + name(R[i]);
+          return broken("a launch for " + who + ": " + device_error_text(w));
+        }
         for (int i : b.s1) {
           R[i].state = kReady2;
           ready2.push_back(i);
@@ -499,6 +531,8 @@ int schedule(skgemm_serve_request_t* io, int n, skgemm_serve_options_t& o, Exec&
         const int i = slot_req[k];
         if (i >= 0 && ex.req_ready(R[i])) {
           slot_req[k] = -1;
+          if (const uint32_t w = ex.req_word(R[i]))
+            return broken(name(R[i]) + ": " + device_error_text(w));
           if ((st = complete(R[i], ex.req_time(R[i])))) return st;
           progressed = true;
         }
@@ -592,8 +626,12 @@ int schedule(skgemm_serve_request_t* io, int n, skgemm_serve_options_t& o, Exec&
     if (progressed) {
       last_progress = ex.now();
     } else {
-      if (ex.now() - last_progress > kStallSeconds)
-        return fail(SKGEMM_ERR_DEVICE_TIMEOUT, "serve: no request made progress for 120 s");
+      if (ex.now() - last_progress > kStallSeconds) {
+        std::string who;
+        for (const Req& r : R)
+          if (r.state != kWait && r.state != kDone) who += (who.empty() ? "" : ", ") + name(r);
+        return broken("no request made progress for 120 s; admitted: " + who);
+      }
       const double before = ex.now();
       ex.idle(next < n ? R[order[next]].arrival : 1e300);
       if (ex.stalled(before)) return fail(SKGEMM_ERR_UNSUPPORTED, "serve: scheduler has no event to wait for");
@@ -661,6 +699,8 @@ int serve_run(skgemm_serve_request_t* io, int n, skgemm_serve_options_t* opts, b
     if ((st = group_ring_reserve(ex->ring, 3 * max_inflight))) return st;
     scratch = 3.0 * 148 * 128 * 128 * 8;
   } else {
+    SKG_CUDA(cudaMallocHost((void**)&ex->words, nslots * sizeof(uint32_t)));
+    memset(ex->words, 0, nslots * sizeof(uint32_t));
     for (int k = 0; k < nslots; ++k) {
       cudaStream_t s;
       SKG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
