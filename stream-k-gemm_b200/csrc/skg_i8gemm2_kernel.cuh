@@ -110,6 +110,11 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     *abort_flag = 0;
     fence_mbar_init();
   }
+  // Both CTAs run before either allocates: tcgen05.alloc and .dealloc of a pair are
+  // collective, need the peer CTA launched and not yet gone, and block without a
+  // bound. The CTAs of a cluster start and end a few cycles apart, more beside other
+  // streams' kernels.
+  cluster_sync_all();
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, kI8TmemCols);
     tmem_relinquish_pair();
@@ -301,6 +306,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   cluster_sync_all();
   tc_fence_after();
   if (warp == 1) tmem_dealloc_pair(tmem_base, kI8TmemCols);
+  cluster_sync_all();  // neither CTA is gone before the other has freed its part
 }
 
 }  // namespace skg

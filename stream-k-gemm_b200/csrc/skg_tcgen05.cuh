@@ -149,7 +149,7 @@ __device__ __forceinline__ void tmem_ld_wait() {
 // the same shared-memory offsets and accumulates rows 128 r .. of D into
 // CTA r's TMEM (all N columns). Every tcgen05 instruction of such a kernel
 // uses .cta_group::2; allocation and deallocation are collective: one warp
-// with the same warp index in each CTA of the pair.
+// with the same warp index in each CTA of the pair, while both CTAs are running.
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -169,6 +169,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 }
 // All threads of both CTAs (release / acquire at cluster scope).
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();  // the .aligned forms need the warp converged
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
