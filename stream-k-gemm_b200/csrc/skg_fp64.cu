@@ -291,8 +291,20 @@ int grouped_launch(const Fp64Group& g, cudaStream_t s) {
   // Flags start at zero for every launch (a stream-ordered memset, captured
   // together with the kernel when the pair is recorded into a graph).
   SKG_CUDA(cudaMemsetAsync(g.flags, 0, (size_t)fixup_slots(g.grid, 1) * sizeof(uint32_t), s));
-  fp64_grouped_kernel<TS><<<g.grid, TS::kThreads, TS::kSmem, s>>>(g);
-  SKG_CUDA(cudaGetLastError());
+  // Cooperative: the CTAs that finish a tile wait for every other CTA of the tile
+  // (shared_fixup), so all of the grid has to be resident, also beside another
+  // stream's grouped launch.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.grid);
+  cfg.blockDim = dim3(TS::kThreads);
+  cfg.dynamicSmemBytes = TS::kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  SKG_CUDA(cudaLaunchKernelEx(&cfg, fp64_grouped_kernel<TS>, g));
   return SKGEMM_OK;
 }
 
