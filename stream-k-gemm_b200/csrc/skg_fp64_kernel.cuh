@@ -234,6 +234,21 @@ __device__ __forceinline__ FixupSpan fixup_span(const Sched& S, int64_t tile_beg
   return f;
 }
 
+// Named barrier 1 over the consumer threads; true if `v` holds on all of them.
+template <int kThreads>
+__device__ __forceinline__ bool bar_and(bool v) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"((uint32_t)v), "n"(kThreads)
+      : "memory");
+  return all != 0;
+}
+
 // Shared fix-up of a tile split over more than two CTAs. All parts are in
 // workspace slots (the owner's in slot grid + first); CTA `cta` of first ..
 // red_last sums its slice of the tile's elements over the parts and stores
@@ -244,8 +259,9 @@ __device__ __forceinline__ FixupSpan fixup_span(const Sched& S, int64_t tile_beg
 // Slices of fewer than 256 elements are summed by several threads an element,
 // each over a contiguous run of parts, and the runs added in order. The CTAs
 // of a tile finish together (equal ranges), so nobody waits long; all CTAs
-// are co-resident. A flag that does not arrive within the budget is recorded
-// in the error word.
+// are co-resident (cooperative launches). A flag that does not arrive within the
+// budget is recorded in the error word, and the slice is not stored: the missing
+// part's slot holds an earlier tile's sums.
 template <class TS, bool AKM, class Sched>
 __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q, FixupSpan f,
                                           int cta, int tm, int tn, uint32_t pubval, double* red) {
@@ -253,10 +269,11 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
   constexpr int NJ = TS::NJ;
   const int tid = threadIdx.x;  // 0 .. TS::kCons - 1
   const int n = f.last - f.first + 1, nred = f.red_last - f.first + 1;
+  bool here = true;
   for (int j = tid; j < n; j += TS::kCons)
-    fixup_flag_wait(S.flags() + (j == 0 ? S.split().grid + f.first : f.first + j), pubval, S.err(),
-                    kFixupBudgetNs);
-  asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons) : "memory");
+    here &= fixup_flag_wait(S.flags() + (j == 0 ? S.split().grid + f.first : f.first + j), pubval,
+                            S.err(), kFixupBudgetNs);
+  if (!bar_and<TS::kCons>(here)) return;
   const int idx = cta - f.first;
   const int e0 = (int)((int64_t)idx * kSlot / nred), e1 = (int)((int64_t)(idx + 1) * kSlot / nred);
   const int ne = e1 - e0;
