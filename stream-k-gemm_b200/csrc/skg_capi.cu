@@ -692,38 +692,6 @@ void add_packed_chunk(HostCopy& up, int g, double* dst, const double* src, int T
          (size_t)panels);
 }
 
-struct HostPipe {
-  DeviceState* dev = nullptr;
-  cudaStream_t sc = nullptr, si = nullptr;
-  std::vector<cudaEvent_t> ev;
-  int init(DeviceState* d, int n) {
-    dev = d;
-    for (cudaStream_t* ps : {&dev->host_stream, &dev->host_h2d, &dev->host_d2h})
-      if (!*ps) SKG_CUDA(cudaStreamCreateWithFlags(ps, cudaStreamNonBlocking));
-    sc = dev->host_stream;
-    si = dev->host_h2d;
-    ev.assign(n, nullptr);
-    for (auto& e : ev) SKG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    return SKGEMM_OK;
-  }
-  // Waits for both streams, frees the events, reports device-side errors.
-  int finish(int st) {
-    cudaStreamSynchronize(si);
-    cudaStreamSynchronize(sc);
-    for (auto& e : ev)
-      if (e) cudaEventDestroy(e);
-    ev.clear();
-    if (st) return st;
-    StreamWorkspace* ws = nullptr;
-    {
-      std::lock_guard<std::mutex> lk2(dev->mu);
-      auto it = dev->ws.find(sc);
-      if (it != dev->ws.end()) ws = it->second;
-    }
-    return consume_device_error(ws, sc);
-  }
-};
-
 SKG_EXPORT int skgemm_dgemm_packed(int64_t M, int64_t N, int64_t K, const double* Ap,
                                    const double* Bp, double* D, double alpha, double gamma) {
   NvtxRange nvtx_(__func__);
@@ -748,7 +716,7 @@ SKG_EXPORT int skgemm_dgemm_packed(int64_t M, int64_t N, int64_t K, const double
     double* dA = (double*)dev->stage[0].ptr;
     double* dB = (double*)dev->stage[1].ptr;
     double* dD = (double*)dev->stage[3].ptr;
-    HostCopy up(dev, cudaMemcpyHostToDevice, hp.si);
+    HostCopy& up = hp.upload();
     auto k_of = [&](int c) { return K * c / C; };
     for (int c = 0; c < C; ++c) {
       add_packed_chunk(up, c, dA + PA * 16 * k_of(c), Ap, 16, M, K, k_of(c), k_of(c + 1) - k_of(c));
@@ -889,7 +857,7 @@ SKG_EXPORT int skgemm_dsyrk_packed(int64_t K, int64_t M, const double* Ap, doubl
     // returns as the caller passed it.
     cudaError_t e = cudaMemcpyAsync(dC, C, (size_t)M * M * 8, cudaMemcpyHostToDevice, hp.si);
     if (e != cudaSuccess) return hp.finish(cuda_fail(e, "SYRK upload"));
-    HostCopy up(dev, cudaMemcpyHostToDevice, hp.si);
+    HostCopy& up = hp.upload();
     auto k_of = [&](int c) { return K * c / nch; };
     for (int c = 0; c < nch; ++c)
       add_packed_chunk(up, c, dA + PA * 16 * k_of(c), Ap, 16, M, K, k_of(c), k_of(c + 1) - k_of(c));

@@ -241,4 +241,37 @@ void HostCopy::work(int w) {
   drain();
 }
 
+int HostPipe::init(DeviceState* d, int n) {
+  dev = d;
+  for (cudaStream_t* ps : {&dev->host_stream, &dev->host_h2d, &dev->host_d2h})
+    if (!*ps) SKG_CUDA(cudaStreamCreateWithFlags(ps, cudaStreamNonBlocking));
+  sc = dev->host_stream;
+  si = dev->host_h2d;
+  ev.assign(n, nullptr);
+  for (auto& e : ev) SKG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return SKGEMM_OK;
+}
+
+HostCopy& HostPipe::upload() {
+  up.reset(new HostCopy(dev, cudaMemcpyHostToDevice, si));
+  return *up;
+}
+
+int HostPipe::finish(int st) {
+  up.reset();  // before the wait: a copy enqueued behind it would outlive the call
+  cudaStreamSynchronize(si);
+  cudaStreamSynchronize(sc);
+  for (auto& e : ev)
+    if (e) cudaEventDestroy(e);
+  ev.clear();
+  if (st) return st;
+  StreamWorkspace* ws = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(dev->mu);
+    auto it = dev->ws.find(sc);
+    if (it != dev->ws.end()) ws = it->second;
+  }
+  return consume_device_error(ws, sc);
+}
+
 }  // namespace skg

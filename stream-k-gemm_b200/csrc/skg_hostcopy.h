@@ -11,6 +11,7 @@
 
 #include <atomic>
 #include <condition_variable>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -81,6 +82,21 @@ class HostCopy {
   bool staged_ = false, stop_ = false, started_ = false;
   cudaError_t err_ = cudaSuccess;
   size_t bytes_ = 0;
+};
+
+// Streams, events and the upload of one chunked host-pointer call (host_mu held).
+struct HostPipe {
+  DeviceState* dev = nullptr;
+  cudaStream_t sc = nullptr, si = nullptr;  // compute, uploads
+  std::vector<cudaEvent_t> ev;
+  std::unique_ptr<HostCopy> up;
+  int init(DeviceState* d, int n);
+  // The call's host -> device copies, on si.
+  HostCopy& upload();
+  // Ends the upload (its threads enqueue nothing more), waits for both streams, frees
+  // the events and reports device-side errors. Returns st if it is one: the pinned
+  // slots and the staging buffers are then free for the next call in any case.
+  int finish(int st);
 };
 
 // Frees the pinned slots of the device (host_mu held by the caller).
