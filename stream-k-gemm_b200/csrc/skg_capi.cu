@@ -161,7 +161,19 @@ StreamWorkspace* stream_workspace(DeviceState* dev, cudaStream_t s, size_t slots
   std::lock_guard<std::mutex> lk(dev->mu);
   StreamWorkspace*& ws = dev->ws[s];
   if (!ws) ws = new StreamWorkspace();
-  *status = ws->ensure(slots, nflags ? nflags : slots);
+  // A Stream-K launch (nflags given) takes the room of the largest one at once: two
+  // slots per CTA at one 128 x 128, two 64 x 64 or four 32 x 32 CTAs per SM. The grid
+  // depends on the shape, and growing with it would free memory under a warm stream.
+  // Where that does not fit, what this launch needs.
+  const size_t sms = (size_t)dev->num_sms;
+  const size_t most = nflags ? std::max(slots, 2 * sms) : slots;
+  const size_t most_flags = nflags ? std::max(nflags, 8 * sms) : slots;
+  if (slots <= ws->partial_slots && std::max(nflags, slots) <= ws->num_flags && ws->err) {
+    *status = SKGEMM_OK;
+  } else if ((*status = ws->ensure(most, most_flags)) == SKGEMM_ERR_OOM && nflags) {
+    cudaGetLastError();
+    *status = ws->ensure(slots, nflags);
+  }
   if (*status == SKGEMM_OK)
     *status = debug_poison(ws->partials, ws->partial_slots * kBM * kBN * sizeof(double), s);
   return *status == SKGEMM_OK ? ws : nullptr;
