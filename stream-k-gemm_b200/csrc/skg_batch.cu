@@ -897,6 +897,14 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
   return SKGEMM_OK;
 }
 
+size_t group_ring_bytes(const GroupRing* R) {
+  size_t n = 0;
+  for (const auto& sl : R->slots)
+    n += sl.probs.bytes + sl.maps.bytes + sl.iters.bytes + sl.part.bytes + sl.flags.bytes +
+         sl.err.bytes;
+  return n;
+}
+
 int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaStream_t s,
                       int* tile_out, const uint32_t** word_out) {
   if (!R || R->slots.empty()) return fail(SKGEMM_ERR_INVALID_ARG, "null group ring");

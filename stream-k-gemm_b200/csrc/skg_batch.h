@@ -38,6 +38,8 @@ int group_ring_reserve(GroupRing* R, int max_problems);
 // valid once the launch has completed, until the slot's next submission).
 int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaStream_t s,
                       int* tile_out, const uint32_t** word_out = nullptr);
+// Device memory the ring holds.
+size_t group_ring_bytes(const GroupRing* R);
 // Reads and clears the slots' error words (call after synchronising).
 int group_ring_error(GroupRing* R);
 

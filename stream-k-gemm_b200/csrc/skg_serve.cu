@@ -697,7 +697,7 @@ int serve_run(skgemm_serve_request_t* io, int n, skgemm_serve_options_t* opts, b
     const int max_inflight = o.max_inflight > 0 ? o.max_inflight : 64;
     ex->ring = group_ring_create(dev, 3);
     if ((st = group_ring_reserve(ex->ring, 3 * max_inflight))) return st;
-    scratch = 3.0 * 148 * 128 * 128 * 8;
+    scratch = (double)group_ring_bytes(ex->ring);
   } else {
     SKG_CUDA(cudaMallocHost((void**)&ex->words, nslots * sizeof(uint32_t)));
     memset(ex->words, 0, nslots * sizeof(uint32_t));

@@ -23,6 +23,7 @@ void group_ring_destroy(GroupRing*) {}
 int group_ring_reserve(GroupRing*, int) { return 0; }
 int group_ring_submit(GroupRing*, const std::vector<Fp64Problem>&, cudaStream_t, int*, const uint32_t**) { return 0; }
 int group_ring_error(GroupRing*) { return 0; }
+size_t group_ring_bytes(const GroupRing*) { return 0; }
 int ozaki_reserve(DeviceState*, cudaStream_t, int64_t, int64_t, int) { return 0; }
 size_t ozaki_stream_bytes(DeviceState*, cudaStream_t) { return 0; }
 }  // namespace skg
