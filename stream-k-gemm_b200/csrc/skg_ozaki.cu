@@ -964,6 +964,14 @@ int lanes_for(int sms, int T, int64_t W) {
   return 1;
 }
 
+// Columns of a plan's tiles. Pair plans (units > 0) cut N evenly, in multiples of 32
+// (the tiles' number stays).
+int lane_columns(int N, int units) {
+  if (units == 0) return kI8BN;
+  const int tiles_n = (N + kI8BN - 1) / kI8BN;
+  return ((N + tiles_n - 1) / tiles_n + 31) / 32 * 32;
+}
+
 // Lane schedule: T tiles x Q lanes, each lane a contiguous range of the
 // (modulus, k-block) space, cut into segments at modulus boundaries and at
 // seg_cap k-blocks (INT32 exactness).
@@ -989,8 +997,7 @@ int get_lane_plan(DeviceState* dev, int M, int N, int KB, int L, bool syrk, int 
   pl->KB = KB;
   pl->tiles_m = (M + kI8BM - 1) / kI8BM;
   pl->tiles_n = (N + kI8BN - 1) / kI8BN;
-  // Pair plans cut N evenly, in multiples of 32 (the tiles' number stays).
-  if (units > 0) pl->bn = ((N + pl->tiles_n - 1) / pl->tiles_n + 31) / 32 * 32;
+  pl->bn = lane_columns(N, units);
   const int bn = pl->bn;
   std::vector<int2> tiles;
   std::vector<int4> pairs;
@@ -1736,57 +1743,48 @@ struct OzakiNeed {
   }
 };
 
+// Norm partials of any operand of at most R rows: ceil(R'/T) panels of C chunks, C =
+// ceil(600 / panels) at most 64, so panels x C < panels + 600.
 size_t norm_part_bytes(int64_t R, int T) {
-  const int64_t P_in = (R + T - 1) / T;
-  const int64_t C = std::max<int64_t>(1, std::min<int64_t>(64, (600 + P_in - 1) / P_in));
-  return (size_t)P_in * C * T * sizeof(double);
+  return (size_t)((R + T - 1) / T + 600) * T * sizeof(double);
 }
 
-// Tiles and segment slots of the lane plan of (M, N, KB, L) (the counting
-// part of get_lane_plan).
-void lane_counts(int num_sms, int M, int N, int KB, int L, bool syrk, int seg_cap, int* T_out,
-                 int* slots_out, bool pair = false) {
-  const int tiles_m = (M + kI8BM - 1) / kI8BM, tiles_n = (N + kI8BN - 1) / kI8BN;
-  int T = 0;
-  for (int tm = 0; tm < tiles_m; ++tm)
-    for (int tn = 0; tn < tiles_n; ++tn)
-      if (!((syrk || pair) && tm * kI8BM > tn * kI8BN + kI8BN - 1)) ++T;
-  if (pair) T += tiles_m * tiles_n;
+// Partial slabs of any GEMM, SYRK or subspace pair of at most nb states and KB
+// k-blocks. The tile counts are get_lane_plan's (they change with 32 columns); a plan
+// on fewer k-blocks has no more lanes (lanes_for), and its slots are its lanes plus the
+// cuts at modulus boundaries and at the segment cap.
+size_t partials_bound(DeviceState* dev, int64_t nb, int64_t KB, int L) {
+  const int units = lanes_pair_units(dev, false);
   const int64_t W = (int64_t)L * KB;
-  const int Q = lanes_for(num_sms, T, W);
-  int slots = 0;
-  for (int q = 0; q < Q; ++q) {
-    int64_t it = (int64_t)q * W / Q, end = (int64_t)(q + 1) * W / Q;
-    while (it < end) {
-      const int l = (int)(it / KB);
-      int64_t stop = std::min<int64_t>(end, (int64_t)(l + 1) * KB);
-      stop = std::min<int64_t>(stop, it + seg_cap);
-      ++slots;
-      it = stop;
+  size_t most = 0;
+  for (int64_t n = 32; n < nb + 32; n += 32) {
+    const int N = (int)std::min(n, nb), tiles_m = (N + kI8BM - 1) / kI8BM,
+              tiles_n = (N + kI8BN - 1) / kI8BN, bn = lane_columns(N, units);
+    const int step = units > 0 ? 2 : 1;  // tile rows of an item
+    int upper = 0, all = 0;              // items of the SYRK's and the GEMM's tiles
+    for (int tn = 0; tn < tiles_n; ++tn)
+      for (int tm = 0; tm < tiles_m; tm += step) {
+        ++all;
+        if (tm * kI8BM <= tn * bn + bn - 1) ++upper;
+      }
+    for (int items : {upper, all, upper + all}) {
+      const int Q = lanes_for(units > 0 ? units : dev->num_sms, items, W);
+      const int64_t slots = Q + L - 1 + W / kSegKbCapSigned;
+      most = std::max(most, (size_t)slots * items * step * kI8BM * kI8BN * sizeof(int32_t));
     }
   }
-  *T_out = T;
-  *slots_out = slots;
+  return most;
 }
 
-OzakiNeed need_lanes(DeviceState* dev, int64_t M, int64_t N, int64_t K, int L, bool syrk,
-                     bool pair = false) {
+OzakiNeed need_lanes(DeviceState* dev, int64_t M, int64_t K, int L) {
   OzakiNeed n;
   const int64_t KP = (K + 127) / 128 * 128;
-  const int KB = (int)(KP / 128);
   const int64_t RA = (M + kI8BN - 1) / kI8BN * kI8BN;
-  const int64_t RB = (N + kI8BN - 1) / kI8BN * kI8BN;
-  n.res_a = (size_t)L * RA * KP;
+  n.res_a = n.res_b = (size_t)L * RA * KP;
   n.part_a = norm_part_bytes(M, 16);
-  n.mu_a = (size_t)RA * sizeof(int);
-  if (!syrk) {
-    n.res_b = (size_t)L * RB * KP;
-    n.part_b = norm_part_bytes(N, 32);
-    n.mu_b = (size_t)RB * sizeof(int);
-  }
-  int T = 0, slots = 0;
-  lane_counts(dev->num_sms, (int)M, (int)N, KB, L, syrk, kSegKbCapSigned, &T, &slots, pair);
-  n.partials = (size_t)slots * T * kI8BM * kI8BN * sizeof(int32_t);
+  n.part_b = norm_part_bytes(M, 32);
+  n.mu_a = n.mu_b = (size_t)RA * sizeof(int);
+  n.partials = partials_bound(dev, M, KP / 128, L);
   return n;
 }
 
@@ -1806,29 +1804,6 @@ OzakiNeed need_rot(int64_t Nd, int64_t nb, int L) {
 
 }  // namespace
 
-// Scratch a stream needs for Ozaki calls of `op` (SKGEMM_OP_*) on the given
-// shape (GEMM: M, N, K; SYRK: M, K; rotation: Nd = M, nb = N) with `slices`
-// moduli (0 = the automatic choice).
-int ozaki_scratch_bytes(DeviceState* dev, int op, int64_t M, int64_t N, int64_t K, int slices,
-                        size_t* bytes) {
-  skgemm_options_t o;
-  memset(&o, 0, sizeof(o));
-  o.precision = SKGEMM_PREC_OZAKI_I8;
-  o.slices = slices;
-  int L, gb, st;
-  OzakiNeed n;
-  if (op == SKGEMM_OP_ROT) {
-    if ((st = choose_L(&o, N, &L, &gb))) return st;
-    n = need_rot(M, N, L);
-  } else {
-    if ((st = choose_L(&o, K, &L, &gb))) return st;
-    n = need_lanes(dev, M, op == SKGEMM_OP_SYRK_PACKED ? M : N, K, L,
-                   op == SKGEMM_OP_SYRK_PACKED);
-  }
-  *bytes = n.total();
-  return SKGEMM_OK;
-}
-
 // Grows stream `s`'s Ozaki scratch to serve every call of the three ops and
 // of the subspace pair on shapes up to (Nd, nb) with `slices` moduli without
 // allocating later.
@@ -1840,9 +1815,7 @@ int ozaki_reserve(DeviceState* dev, cudaStream_t s, int64_t Nd, int64_t nb, int 
   int Lk, Lr, gb, st;
   if ((st = choose_L(&o, Nd, &Lk, &gb))) return st;
   if ((st = choose_L(&o, nb, &Lr, &gb))) return st;
-  OzakiNeed n = need_lanes(dev, nb, nb, Nd, Lk, false);
-  n.max_with(need_lanes(dev, nb, nb, Nd, Lk, true));
-  n.max_with(need_lanes(dev, nb, nb, Nd, Lk, false, true));  // the fused subspace pair
+  OzakiNeed n = need_lanes(dev, nb, Nd, Lk);  // GEMM, SYRK and the fused pair
   n.max_with(need_rot(Nd, nb, Lr));
   std::lock_guard<std::mutex> lk(g_oz_mu);
   if ((st = ensure_consts(dev))) return st;

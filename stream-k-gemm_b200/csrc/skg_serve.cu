@@ -720,6 +720,9 @@ int serve_run(skgemm_serve_request_t* io, int n, skgemm_serve_options_t* opts, b
   ex->h0 = std::chrono::steady_clock::now();
   st = serve::schedule(io, n, o, *ex, arena, nslots);
   cudaDeviceSynchronize();
+  // What is held now: no more than was reserved, or the budget was exceeded.
+  o.scratch_bytes = ex->ring ? (double)group_ring_bytes(ex->ring) : 0.0;
+  for (cudaStream_t s : ex->slots) o.scratch_bytes += (double)ozaki_stream_bytes(dev, s);
   return st;
 }
 

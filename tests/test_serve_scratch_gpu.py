@@ -14,3 +14,16 @@ def test_native_scratch_counts_both_slots_of_a_cta(cuda):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert o.scratch_bytes >= 3 * 2 * sms * 128 * 128 * 8
     assert o.scratch_bytes + o.peak_admitted_bytes <= 2e9
+
+
+@pytest.mark.parametrize("ng,nb", [(20000, 256), (6400, 1040), (40000, 528)])
+def test_split_path_scratch_is_reserved_for_every_smaller_request(cuda, ng, nb):
+    """The scratch reserved for the largest request holds whatever mix of smaller ones
+    comes with it: nothing is allocated later."""
+    def held(extra):
+        trace = [(0.0, ng, nb, 1)] + [(0.0, g, b, 2) for g, b in extra]
+        _, o = skgemm.serve(trace, precision=skgemm.PREC_OZAKI_I8, hbm_budget=40e9,
+                            realtime=False)
+        return o.scratch_bytes
+    smaller = [(16 * g, b) for g in (10, 100, ng // 16) for b in range(32, nb, 48)]
+    assert held(smaller) == held([])
