@@ -50,8 +50,6 @@ int debug_poison(void* p, size_t bytes, cudaStream_t s) {
   return SKGEMM_OK;
 }
 
-namespace {
-// The current device's stream for table uploads (created on first use).
 int table_stream(cudaStream_t* s) {
   static std::mutex mu;
   static cudaStream_t streams[64] = {};
@@ -63,7 +61,6 @@ int table_stream(cudaStream_t* s) {
   *s = streams[d];
   return SKGEMM_OK;
 }
-}  // namespace
 
 int upload_table(void* dst, const void* src, size_t bytes) {
   cudaStream_t s = nullptr;

@@ -64,9 +64,13 @@ namespace skg {
 namespace {
 
 // chi on the device: each projector's columns in groups of kNlocCols, a group
-// row-major [nrow][kNlocCols], columns past ncol zero. A chunk of rows of a group
-// is then contiguous, for whole 16-byte copies.
-//
+// row-major [nrow][group_pitch], a chunk of rows then contiguous, for whole 16-byte
+// copies. An odd last column has a zero one beside it.
+__host__ __device__ inline int group_pitch(int ncol, int k0) {  // the group from column k0
+  const int w = ncol - k0;
+  return w < 16 ? (w + 1) & ~1 : 16;
+}
+
 // Forward CTA: (block q, 32 bands, 16 columns); thread (bands bl, bl + 1, columns
 // jl, jl + 1). The CTA walks the block's projectors in order and each projector's
 // rows in chunks of kNlocRows: a chunk's gathered rows x 32 bands of psi and its
@@ -89,6 +93,7 @@ constexpr int kNlocCols = 16;
 constexpr int kNlocRows = 16;
 constexpr int kNlocRing = 4;
 constexpr int kNlocThreads = kNlocBands * kNlocCols / 4;
+static_assert(kNlocCols == 16, "group_pitch");
 static_assert(kNlocRows * kNlocCols == 2 * kNlocThreads, "one 16-byte piece of chi a thread");
 static_assert(kNlocRows * kNlocBands == 4 * kNlocThreads, "two 16-byte pieces of psi a thread");
 
@@ -114,6 +119,8 @@ __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
   // This thread's copies: bands bl, bl + 1 of rows cr and cr + kNlocRows / 2, and
   // 16 bytes of chi.
   const int cr = threadIdx.x / (kNlocBands / 2);
+  const int pitch = group_pitch((int)nc, (int)jb);
+  const int xr = threadIdx.x / (kNlocCols / 2), xc = 2 * (threadIdx.x % (kNlocCols / 2));
   const bool band_ok = b < nb;
   const double* pb = psi16 + (band_ok ? (b / 16) * K * 16 + b % 16 : 0);
 
@@ -144,8 +151,8 @@ __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
       if (band_ok && cr < left) cp_async16(&rows[buf][cr][bl], pb + (int64_t)n0 * 16, 16u);
       if (band_ok && cr + kNlocRows / 2 < left)
         cp_async16(&rows[buf][cr + kNlocRows / 2][bl], pb + (int64_t)n1 * 16, 16u);
-      const int o = 2 * threadIdx.x;
-      if (o / kNlocCols < left) cp_async16(&xs[buf][0][0] + o, ix + (int64_t)ir0 * kNlocCols + o, 16u);
+      if (xr < left && xc < pitch)
+        cp_async16(&xs[buf][xr][xc], ix + (int64_t)(ir0 + xr) * pitch + xc, 16u);
       ir0 += kNlocRows;
       if (ir0 >= inr) {
         ++ie;
@@ -212,6 +219,24 @@ __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
   }
 }
 
+// The caller's chi (each projector's columns one after the other, in_off) into the
+// device layout; CTA = a span of kNlocSpan row tiles of a projector.
+__global__ void __launch_bounds__(128) nloc_chi_layout_kernel(
+    const int64_t* __restrict__ tile_proj, const int64_t* __restrict__ tile_r0,
+    const uint32_t* __restrict__ nrow, const uint32_t* __restrict__ ncol,
+    const int64_t* __restrict__ in_off, const int64_t* __restrict__ chi_off,
+    const double* __restrict__ in, double* __restrict__ chi, int span) {
+  const int p = (int)tile_proj[blockIdx.x];
+  const int64_t nr = nrow[p], r1 = min(nr, tile_r0[blockIdx.x] + span);
+  const int nc = (int)ncol[p];
+  for (int64_t r = tile_r0[blockIdx.x] + threadIdx.x; r < r1; r += blockDim.x)
+    for (int j = 0; j < (nc + 1) / 2 * 2; ++j) {
+      const int k0 = j / kNlocCols * kNlocCols;
+      chi[chi_off[p] + k0 * nr + r * group_pitch(nc, k0) + (j - k0)] =
+          j < nc ? in[in_off[p] + j * nr + r] : 0.0;
+    }
+}
+
 // Back-projection, step 1: temp_p[r, b] = sum_k chi_p[r, k] C_p[k, b] (fused,
 // k ascending: the reference's gemm_ab order) for every projector row, into
 // temp[(row_off_p + r) * nb + b]. CTA = (a span of up to kNlocSpan row tiles
@@ -252,13 +277,15 @@ __global__ void __launch_bounds__(kNlocWarps * 32) nloc_chi_c_kernel(
   double* out = temp + (row_off[p] + span0) * nb + b;
   for (int k0 = 0; k0 < nc; k0 += kNlocCols) {
     if (k0 > 0) __syncthreads();  // the group before is consumed
-    const double* x = chi + chi_off[p] + (int64_t)k0 * nrow[p] + span0 * kNlocCols;
+    const int pitch = group_pitch(nc, k0);
+    const double* x = chi + chi_off[p] + (int64_t)k0 * nrow[p] + span0 * pitch;
 #pragma unroll
     for (int t = 0; t < kNlocSpan; ++t) {
 #pragma unroll
       for (int i = 0; i < kNlocTileR * kNlocCols / 2; i += kNlocWarps * 32) {
         const int o = t * kNlocTileR * kNlocCols + 2 * (i + (int)threadIdx.x);
-        if (o / kNlocCols < nr) cp_async16(&xs[0][0][0] + o, x + o, 16u);
+        const int r = o / kNlocCols, c = o % kNlocCols;
+        if (r < nr && c < pitch) cp_async16(&xs[0][0][0] + o, x + r * pitch + c, 16u);
       }
       cp_async_commit();
     }
@@ -358,6 +385,35 @@ int upload(T** dst, const std::vector<T>& v) {
   return upload_table(*dst, v.data(), v.size() * sizeof(T));
 }
 
+// chi (n doubles, projector p's columns from in_off[p]) into d_chi (total doubles) in
+// the kernels' layout: uploaded as it is and laid out on the device.
+int upload_chi(skgemm_nloc* h, const double* chi, int64_t n, int64_t total,
+               const std::vector<int64_t>& in_off) {
+  if (h->ntiles == 0) return SKGEMM_OK;
+  DeviceBuffer in, off;
+  auto lay_out = [&]() -> int {
+    int st;
+    cudaStream_t s = nullptr;
+    if ((st = in.ensure((size_t)n * sizeof(double))) ||
+        (st = off.ensure(in_off.size() * sizeof(int64_t))))
+      return st;
+    SKG_CUDA(cudaMalloc(&h->d_chi, (size_t)total * sizeof(double)));
+    if ((st = upload_table(off.ptr, in_off.data(), in_off.size() * sizeof(int64_t))) ||
+        (st = upload_table(in.ptr, chi, (size_t)n * sizeof(double))) || (st = table_stream(&s)))
+      return st;
+    nloc_chi_layout_kernel<<<(unsigned)h->ntiles, 128, 0, s>>>(
+        h->d_tile_proj, h->d_tile_r0, h->d_nrow, h->d_ncol, (const int64_t*)off.ptr, h->d_chi_off,
+        (const double*)in.ptr, h->d_chi, kNlocTileR * kNlocSpan);
+    SKG_CUDA(cudaGetLastError());
+    SKG_CUDA(cudaStreamSynchronize(s));
+    return SKGEMM_OK;
+  };
+  const int st = lay_out();
+  in.release();
+  off.release();
+  return st;
+}
+
 void release(skgemm_nloc* h) {
   void* ptrs[] = {h->d_nrow, h->d_ncol, h->d_index, h->d_row_off, h->d_chi_off, h->d_chi,
                   h->d_gamma, h->d_blk, h->d_blk_end, h->d_blk_proj, h->d_blk_scale,
@@ -393,7 +449,7 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
     rows += nrow[p];
     in_off[p] = chi_in;
     chi_in += (int64_t)nrow[p] * ncol[p];
-    chis += (int64_t)nrow[p] * ((ncol[p] + kNlocCols - 1) / kNlocCols) * kNlocCols;
+    chis += (int64_t)nrow[p] * ((ncol[p] + 1) / 2 * 2);  // all groups at their pitch
     gams += ncol[p];
     if ((int64_t)offsets[p] + ncol[p] > total)
       return fail(SKGEMM_ERR_INVALID_ARG, "projector block past the total column count");
@@ -493,21 +549,17 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
   h->ntiles = (int64_t)tile_proj.size();
   std::vector<uint32_t> vnrow(nrow, nrow + P), vncol(ncol, ncol + P);
   std::vector<uint32_t> vindex(index, index + rows);
-  std::vector<double> vchi(chis, 0.0), vgam(gamma, gamma + gams);
-  for (int64_t p = 0; p < P; ++p)
-    for (int64_t j = 0; j < ncol[p]; ++j)
-      for (int64_t r = 0; r < nrow[p]; ++r)
-        vchi[chi_off[p] + (j / kNlocCols * nrow[p] + r) * kNlocCols + j % kNlocCols] =
-            chi[in_off[p] + j * nrow[p] + r];
+  std::vector<double> vgam(gamma, gamma + gams);
   if ((st = upload(&h->d_nrow, vnrow)) || (st = upload(&h->d_ncol, vncol)) ||
       (st = upload(&h->d_index, vindex)) || (st = upload(&h->d_row_off, row_off)) ||
-      (st = upload(&h->d_chi_off, chi_off)) || (st = upload(&h->d_chi, vchi)) ||
+      (st = upload(&h->d_chi_off, chi_off)) || 
       (st = upload(&h->d_gamma, vgam)) || (st = upload(&h->d_blk, blk)) ||
       (st = upload(&h->d_blk_end, blk_end)) || (st = upload(&h->d_blk_proj, blk_proj)) ||
       (st = upload(&h->d_blk_scale, blk_scale)) || (st = upload(&h->d_proj_blk_col, proj_col)) ||
       (st = upload(&h->d_touch, touch)) || (st = upload(&h->d_touch_off, touch_off)) ||
       (st = upload(&h->d_ent_off, ent_off)) ||
-      (st = upload(&h->d_tile_proj, tile_proj)) || (st = upload(&h->d_tile_r0, tile_r0))) {
+      (st = upload(&h->d_tile_proj, tile_proj)) || (st = upload(&h->d_tile_r0, tile_r0)) ||
+      (st = upload_chi(h, chi, chi_in, chis, in_off))) {
     release(h);
     delete h;
     return st;
