@@ -826,14 +826,15 @@ int batch_consume_error(DeviceState* dev, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------- ring
-// A ring of grouped-launch workspaces: submission i uses slot i % depth, so a
-// launch's tables and partial slots stay untouched until `depth` later
-// submissions. Tables travel through pinned host memory with
+// A ring of grouped-launch tables: submission i uses slot i % depth, so a launch's
+// tables stay untouched until `depth` later submissions. All submissions go to one
+// stream, so that their launches follow one another and share the partial tiles and
+// flags. Tables travel through pinned host memory with
 // cudaMemcpyAsync on the launch stream (no host-side synchronisation unless
 // the slot's previous launch is still running).
 struct GroupRing {
   struct Slot {
-    DeviceBuffer probs, maps, iters, part, flags, err;
+    DeviceBuffer probs, maps, iters, err;
     void* host = nullptr;  // pinned staging of the three tables
     size_t host_bytes = 0;
     cudaEvent_t ev = nullptr;
@@ -842,6 +843,7 @@ struct GroupRing {
   };
   DeviceState* dev = nullptr;
   std::vector<Slot> slots;
+  DeviceBuffer part, flags;
   int next = 0;
 };
 
@@ -864,10 +866,10 @@ void group_ring_destroy(GroupRing* R) {
     sl.probs.release();
     sl.maps.release();
     sl.iters.release();
-    sl.part.release();
-    sl.flags.release();
     sl.err.release();
   }
+  R->part.release();
+  R->flags.release();
   delete R;
 }
 
@@ -878,12 +880,11 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
   const size_t part = std::max((size_t)fixup_slots(cap128, 1) * 128 * 128,
                                (size_t)fixup_slots(cap64, 1) * 64 * 64) * 8;
   const size_t nflags = (size_t)fixup_slots(std::max(cap128, cap64), 1);
+  if ((st = R->part.ensure(part)) || (st = R->flags.ensure(nflags * sizeof(uint32_t)))) return st;
   for (auto& sl : R->slots) {
     if ((st = sl.probs.ensure((size_t)max_problems * sizeof(Fp64Params)))) return st;
     if ((st = sl.maps.ensure((size_t)2 * max_problems * sizeof(CUtensorMap)))) return st;
     if ((st = sl.iters.ensure((size_t)(max_problems + 1) * sizeof(int64_t)))) return st;
-    if ((st = sl.part.ensure(part))) return st;
-    if ((st = sl.flags.ensure(nflags * sizeof(uint32_t)))) return st;
     if (!sl.err.ptr) {
       if ((st = sl.err.ensure(sizeof(uint32_t)))) return st;
       if ((st = fill_table(sl.err.ptr, 0, sizeof(uint32_t)))) return st;
@@ -898,10 +899,9 @@ int group_ring_reserve(GroupRing* R, int max_problems) {
 }
 
 size_t group_ring_bytes(const GroupRing* R) {
-  size_t n = 0;
+  size_t n = R->part.bytes + R->flags.bytes;
   for (const auto& sl : R->slots)
-    n += sl.probs.bytes + sl.maps.bytes + sl.iters.bytes + sl.part.bytes + sl.flags.bytes +
-         sl.err.bytes;
+    n += sl.probs.bytes + sl.maps.bytes + sl.iters.bytes + sl.err.bytes;
   return n;
 }
 
@@ -948,8 +948,8 @@ int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaS
     g.num_problems = np;
     g.total_iters = T.iter_begin.back();
     g.grid = (int)std::min<int64_t>(cap, g.total_iters);
-    g.workspace = (double*)sl.part.ptr;
-    g.flags = (uint32_t*)sl.flags.ptr;
+    g.workspace = (double*)R->part.ptr;
+    g.flags = (uint32_t*)R->flags.ptr;
     g.err = (uint32_t*)sl.err.ptr;
     if ((st = launch_fp64_group(tile, g, s))) return st;
   }

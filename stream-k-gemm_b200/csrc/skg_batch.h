@@ -27,7 +27,7 @@ int model_tile(const std::vector<Fp64Problem>& probs);
 // resolve SKGEMM_PREC_AUTO.
 double batch_native_estimate(const Fp64Problem& p);
 
-// A ring of `depth` grouped-launch workspaces for a stream of batches.
+// A ring of `depth` grouped-launch tables for the batches of one stream.
 struct GroupRing;
 GroupRing* group_ring_create(DeviceState* dev, int depth);
 void group_ring_destroy(GroupRing* R);

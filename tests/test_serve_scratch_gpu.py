@@ -8,11 +8,11 @@ pytestmark = pytest.mark.gpu
 
 
 def test_native_scratch_counts_both_slots_of_a_cta(cuda):
-    """Three launches' partial tiles: two 128 x 128 slots per SM each."""
+    """The launches follow one another on partial tiles of two 128 x 128 slots per SM."""
     _, o = skgemm.serve([(0.0, 1600, 64, 1)], precision=skgemm.PREC_NATIVE, hbm_budget=2e9,
                         realtime=False)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert o.scratch_bytes >= 3 * 2 * sms * 128 * 128 * 8
+    assert 2 * sms * 128 * 128 * 8 <= o.scratch_bytes <= 58e6
     assert o.scratch_bytes + o.peak_admitted_bytes <= 2e9
 
 
