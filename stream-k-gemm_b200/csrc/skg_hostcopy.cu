@@ -85,7 +85,10 @@ int HostCopy::start(bool gated) {
   for (const Piece& p : whole_)
     staged_ = staged_ && pageable(kind_ == cudaMemcpyHostToDevice ? p.src : p.dst);
   // Without pinned slots or threads the driver copies.
-  if (staged_ && slots_->ensure() != SKGEMM_OK) staged_ = false;
+  if (staged_ && slots_->ensure() != SKGEMM_OK) {
+    cudaGetLastError();  // or the next launch's check would report it
+    staged_ = false;
+  }
   if (!staged_) {
     int st = SKGEMM_OK;
     if (!gated)

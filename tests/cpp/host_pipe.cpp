@@ -1,7 +1,7 @@
 // HostPipe and HostCopy on a stand-in for the CUDA runtime: a call that fails while its
 // upload is under way must leave no copy to be enqueued behind its final wait.
-// Prints "<copies enqueued> <enqueued after the stream's wait> <after finish>" and, for
-// a call that ends well, whether every byte arrived.
+// Prints "<status> <copies enqueued> <of them after the stream's wait> <after finish>
+// <every byte arrived> <error left for the next launch's check>".
 #include <atomic>
 #include <chrono>
 #include <cstdio>
@@ -14,14 +14,23 @@
 
 static std::atomic<int> g_copies{0}, g_late{0};
 static std::atomic<bool> g_waited{false};
+static bool g_no_pinned = false;
+static cudaError_t g_last = cudaSuccess;
 
 extern "C" {
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
   a->type = cudaMemoryTypeUnregistered;
   return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = g_last;
+  g_last = cudaSuccess;
+  return e;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  *p = g_no_pinned ? nullptr : malloc(n);
+  return *p ? cudaSuccess : (g_last = cudaErrorMemoryAllocation);
+}
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)malloc(1); return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { free((void*)e); return cudaSuccess; }
@@ -52,6 +61,7 @@ int consume_device_error(StreamWorkspace*, cudaStream_t) { return SKGEMM_OK; }
 int main(int argc, char** argv) {
   using namespace skg;
   const bool failing = argc > 1 && !strcmp(argv[1], "fail");
+  g_no_pinned = argc > 1 && !strcmp(argv[1], "unpinned");
   const int chunks = 8;
   const size_t n = 4 << 20;
   std::vector<char> src(chunks * n), dst(chunks * n);
@@ -70,6 +80,7 @@ int main(int argc, char** argv) {
   const int got = hp.finish(st);
   const int seen = g_copies;
   std::this_thread::sleep_for(std::chrono::milliseconds(60));
-  printf("%d %d %d %d %d\n", got, seen, (int)g_late, (int)g_copies - seen, src == dst ? 1 : 0);
+  printf("%d %d %d %d %d %d\n", got, seen, (int)g_late, (int)g_copies - seen, src == dst ? 1 : 0,
+         (int)g_last);
   return 0;
 }
