@@ -240,7 +240,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 #pragma unroll
     for (int j = 0; j < (BF ? 128 : 1); ++j) run[j] = 0;
     while (i8p2_next_item(p, cl, ncl, rank, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Pair)) {
+      // One answer for the warp: the TMEM loads below need it converged.
+      if (!__all_sync(0xffffffffu,
+                      !*abort_flag && mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Pair))) {
         *abort_flag = 1;
         break;
       }

@@ -404,7 +404,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 #pragma unroll
     for (int j = 0; j < (BF ? 128 : 1); ++j) run[j] = 0;
     while (i8_next_item(p, cta, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8)) {
+      // One answer for the warp: the TMEM loads below need it converged.
+      if (!__all_sync(0xffffffffu,
+                      !*abort_flag && mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8))) {
         *abort_flag = 1;
         break;
       }
@@ -714,7 +716,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     int cur = 0;
     I8Item it;
     while (rot_next_item(p, cta, cur, it)) {
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Rot)) {
+      // One answer for the warp: the TMEM loads below need it converged.
+      if (!__all_sync(0xffffffffu,
+                      !*abort_flag && mbar_wait(&tfull_bar[acc], acc_phase, p.err, kDevErrI8Rot))) {
         *abort_flag = 1;
         break;
       }
