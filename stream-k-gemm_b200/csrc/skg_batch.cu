@@ -224,6 +224,7 @@ int build_group_tables(const std::vector<Fp64Problem>& probs, int tile, int orde
   T->params.reserve(n);
   T->maps.reserve(2 * n);
   T->useful = T->issued = 0.0;
+  T->max_tile_iters = 0;
   for (int idx : perm) {
     const Geom& g = geo[idx];
     if (g.iters == 0) continue;
@@ -255,6 +256,7 @@ int build_group_tables(const std::vector<Fp64Problem>& probs, int tile, int orde
     T->maps.push_back(ma);
     T->maps.push_back(mb);
     T->iter_begin.push_back(T->iter_begin.back() + g.iters);
+    T->max_tile_iters = std::max(T->max_tile_iters, g.ipt);
     T->useful += g.useful;
     T->issued += g.issued;
   }
@@ -326,6 +328,7 @@ int configure(BatchPlan* P, Config c) {
   memset(&G, 0, sizeof(G));
   G.num_problems = np;
   G.total_iters = total;
+  G.max_tile_iters = T.max_tile_iters;
   G.grid = grid;
   if (np > 0) {
     if ((st = P->d_probs.ensure(hp.size() * sizeof(Fp64Params)))) return st;
@@ -947,6 +950,7 @@ int group_ring_submit(GroupRing* R, const std::vector<Fp64Problem>& probs, cudaS
     g.iter_begin = (const int64_t*)sl.iters.ptr;
     g.num_problems = np;
     g.total_iters = T.iter_begin.back();
+    g.max_tile_iters = T.max_tile_iters;
     g.grid = (int)std::min<int64_t>(cap, g.total_iters);
     g.workspace = (double*)R->part.ptr;
     g.flags = (uint32_t*)R->flags.ptr;

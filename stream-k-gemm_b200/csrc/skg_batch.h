@@ -14,6 +14,7 @@ struct GroupTables {
   std::vector<CUtensorMap> maps;
   std::vector<int64_t> iter_begin;
   double useful = 0.0, issued = 0.0;  // MACs
+  int max_tile_iters = 0;
 };
 
 // Problems with work in `order` (1 as given, 2 most work first), their TMA

@@ -147,6 +147,7 @@ struct SingleSched {
 };
 
 // A group of problems: descriptors and tensor maps in global memory.
+template <bool SPREAD>
 struct GroupSched {
   const Fp64Group& g;
   __device__ __forceinline__ const IterSplit& split() const { return g.split; }
@@ -171,7 +172,7 @@ struct GroupSched {
   __device__ __forceinline__ uint32_t* flags() const { return g.flags; }
   __device__ __forceinline__ uint32_t* err() const { return g.err; }
   __device__ __forceinline__ uint32_t pub() const { return 1u; }
-  __device__ __forceinline__ bool spread() const { return true; }
+  __device__ __forceinline__ bool spread() const { return SPREAD; }
 };
 
 // Where iteration `it` (< it_end) falls: problem, tile, k-block range of this
@@ -662,10 +663,11 @@ __global__ void __launch_bounds__(Tile32::kThreads, Tile32::kMinBlocks)
   streamk_body<Tile32, true>(S);
 }
 
-template <class TS>
+// SPREAD: with the shared fix-up (tiles of kSharedParts parts or more in the group).
+template <class TS, bool SPREAD>
 __global__ void __launch_bounds__(TS::kThreads, TS::kMinBlocks)
     fp64_grouped_kernel(const __grid_constant__ Fp64Group g) {
-  const GroupSched S{g};
+  const GroupSched<SPREAD> S{g};
   streamk_body<TS>(S);
 }
 

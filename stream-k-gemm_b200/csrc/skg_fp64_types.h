@@ -140,6 +140,7 @@ struct Fp64Group {
   int num_problems;
   int64_t total_iters;
   int grid;
+  int max_tile_iters;  // the longest tile's iterations
   IterSplit split;    // make_split(total_iters, grid)
   double* workspace;  // 2 * grid slots of BM*BN doubles (shared fix-up)
   uint32_t* flags;    // 2 * grid flags, zero at launch

@@ -139,9 +139,9 @@ int fp64_grid_for(DeviceState* dev, const Fp64Problem& prob);
 // first launch).
 int fp64_preload(DeviceState* dev);
 // Grouped launch (batched path): CTAs per SM the grouped kernel of `tile`
-// (128 or 64) fits, and the launch itself (flag reset + cooperative kernel, both
-// capturable into a CUDA graph; the grid must not exceed SMs x blocks_per_sm, or
-// the launch is refused).
+// (128 or 64) fits, and the launch itself (flag reset + kernel, cooperative where tiles
+// are finished by several CTAs; both capturable into a CUDA graph). The grid must not
+// exceed SMs x blocks_per_sm.
 struct Fp64Group;
 int fp64_group_occupancy(DeviceState* dev, int tile, int* blocks_per_sm);
 int launch_fp64_group(int tile, const Fp64Group& g, cudaStream_t s);

@@ -34,3 +34,19 @@ def test_plans_on_several_streams_at_once(cuda, tile, graph):
         for it, d in zip(s, w):
             assert torch.equal(it.dD, d)
             it.check(sample=200 if it.op == S else 0)
+
+
+@pytest.mark.parametrize("tile", [128, 64])
+@pytest.mark.parametrize("grid", [1, 3, 4, 5, 6, 9, 40])
+@pytest.mark.parametrize("tiles", [1, 3])
+def test_tiles_around_the_shared_fixup_line(cuda, tile, grid, tiles):
+    """Tiles cut into fewer parts than the shared fix-up takes, just as many, and more,
+    alone and beside shorter ones (the group is launched with or without it)."""
+    S, G = skgemm.OP_SYRK_PACKED, skgemm.OP_GEMM_PACKED
+    items = [Item(G, 77, 40, 50, 6400)] + [Item(S, 80 + i, 30, 30, 900 + 16 * i)
+                                           for i in range(tiles - 1)]
+    p = skgemm.Plan([it.item() for it in items], tile=tile, grid=grid, tune=False, graph=False)
+    p.run()
+    p.status()
+    for it in items:
+        it.check()
