@@ -60,7 +60,9 @@ struct Schedule {
 //    rotation 1008 x 256 15 / 13; SYRK 10000 x 128 on 64 x 64 22 / 21, GEMM 23 /
 //    19; equal from about 230 (32 x 32) and 60 iterations a CTA (64 x 64), where
 //    the multiplications want all of them. 64 x 64 tiles in fewer than eight
-//    parts are not cut evenly enough by half (dense 1000^3 72 / 80).
+//    parts keep the full grid: half of it costs dense operands 7-12% (700 x 500 x
+//    900 31 / 33, 800^3 43 / 47, 1024^3 74 / 82, 500 x 500 x 2500 50 / 56) and
+//    gains packed ones little (GEMM 1000 x 512 27 / 25, 2500 x 512 47 / 47).
 //  * at most sqrt(14 iterations) parts a tile: an iteration costs about as much
 //    as the sums of 14 parts in the fix-up. SYRK 10000 x 32 17 / 11 (94 parts
 //    instead of 592), 32768 x 32 25 / 14.
@@ -284,13 +286,9 @@ int grouped_setup(int device, int* blocks_per_sm) {
   static int occ[64] = {0};
   if (device < 0 || device >= 64) return fail(SKGEMM_ERR_INVALID_ARG, "device index");
   if (!occ[device]) {
-    SKG_CUDA(cudaFuncSetAttribute(fp64_grouped_kernel<TS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, TS::kSmem));
-    int n = 0;
-    SKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp64_grouped_kernel<TS>,
-                                                           TS::kThreads, TS::kSmem));
-    if (n < 1) return fail(SKGEMM_ERR_UNSUPPORTED, "grouped kernel does not fit on an SM");
-    occ[device] = n;
+    int a = 0, b = 0, st;
+    if ((st = grouped_occupancy<TS, false>(&a)) || (st = grouped_occupancy<TS, true>(&b))) return st;
+    occ[device] = std::min(a, b);
   }
   *blocks_per_sm = occ[device];
   return SKGEMM_OK;
@@ -328,7 +326,7 @@ int grouped_launch(const Fp64Group& g, cudaStream_t s) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  SKG_CUDA(cudaLaunchKernelEx(&cfg, fp64_grouped_kernel<TS>, g));
+  SKG_CUDA(cudaLaunchKernelEx(&cfg, fp64_grouped_kernel<TS, true>, g));
   return SKGEMM_OK;
 }
 
