@@ -15,21 +15,21 @@
 // Work decomposition (Stream-K): the MAC-loop iterations of all tiles
 // (tiles * ceil(K/BK)) are split evenly over the persistent CTAs. A CTA whose
 // range starts inside a tile stores its partial accumulator to a workspace slot
-// and publishes a flag. A tile split over two CTAs is finished by the CTA that
-// owns its k = 0 segment: it waits (with a time budget) for the flag, adds the
-// partial and runs the epilogue. A tile split over more is finished by all the
+// and publishes a flag. A tile of fewer than kSharedParts parts is finished by the
+// CTA that owns its k = 0 segment: it waits (with a time budget) for the flags, adds
+// the partials and runs the epilogue. A tile of more parts is finished by all the
 // CTAs whose range ends in it (shared_fixup below), each a slice of the
 // elements. The reduction order is a pure function of the schedule, so results
 // are bitwise reproducible run to run.
 //
-// The same body serves one problem (fp64_streamk_kernel, BM = BN = 128, or
-// fp64_streamk_kernel64, BM = BN = 64) and a
-// group of problems in one launch (fp64_grouped_kernel<TileShape>, the
-// batched path: iterations of all problems concatenated, see Fp64Group).
+// The same body serves one problem (fp64_streamk_kernel, fp64_streamk_kernel64 and
+// fp64_streamk_kernel32: BM = BN = 128, 64 and 32) and a group of problems in one
+// launch (fp64_grouped_kernel<TileShape>, 128 or 64, the batched path: iterations of
+// all problems concatenated, see Fp64Group).
 //
 // Data movement: one producer warp issues TMA tile loads (128B-swizzled boxes
-// of 16 doubles x BK rows) into an NSTAGE ring; 8 consumer warps run FP64 DMMA
-// (m16n8k8) from shared memory. Every operand tile in shared memory is a set of
+// of 16 doubles x BK rows) into a ring of kStages; 8 consumer warps (4 on 32 x 32
+// tiles) run FP64 DMMA (m16n8k8) from shared memory. Every operand tile in shared memory is a set of
 // "chunks" [BK][16] doubles (16 rows/columns of the output, k-major rows of
 // 128 B), which is exactly the reference's packed panel layout
 // ([tiles][K][16], gemm_opt.cpp:342-354) restricted to a BK slice.
@@ -250,14 +250,14 @@ __device__ __forceinline__ bool bar_and(bool v) {
   return all != 0;
 }
 
-// Shared fix-up of a tile split over more than two CTAs. All parts are in
+// Shared fix-up of a tile of kSharedParts parts or more. All parts are in
 // workspace slots (the owner's in slot grid + first); CTA `cta` of first ..
 // red_last sums its slice of the tile's elements over the parts and stores
 // them. Added by the owner alone, the parts are a serial chain of
 // last - first reads of a whole tile by one SM: a 10000 x 32 SYRK (295 parts
-// of 32 KB) took 334 us and a 13824 x 128 GEMM (147 of 128 KB) 445 us, now 21
-// and 29 us. Here every SM reads one tile's worth.
-// Slices of fewer than 256 elements are summed by several threads an element,
+// of 32 KB) took 334 us and a 13824 x 128 GEMM (147 of 128 KB) 445 us, with this
+// alone 21 and 29 us. Here every SM reads one tile's worth.
+// Slices of fewer elements than threads are summed by several threads an element,
 // each over a contiguous run of parts, and the runs added in order. The CTAs
 // of a tile finish together (equal ranges), so nobody waits long; all CTAs
 // are co-resident (cooperative launches). A flag that does not arrive within the
@@ -283,7 +283,7 @@ __device__ __forceinline__ void shared_fixup(const Sched& S, const Fp64Params& q
   const double* others = S.workspace() + (int64_t)f.first * kSlot;
   const int64_t mb = (int64_t)tm * TS::BM, nbase = (int64_t)tn * TS::BN;
   auto finish = [&](int e, double v) {
-    // Slot element e = reg * 256 + thread: the accumulator layout.
+    // Slot element e = reg * kCons + thread: the accumulator layout.
     const int reg = e / TS::kCons, th = e % TS::kCons;
     const int r = reg & 3, j = (reg >> 2) % NJ, i = (reg >> 2) / NJ;
     const int w = th >> 5, l = th & 31, g = l >> 2, t = l & 3;
@@ -524,7 +524,7 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     // ---------------------------------------------------------- epilogue
     const bool owner = (sg.kb == 0);
     const bool complete = owner && (sg.ke == q.iters_per_tile);
-    const int ctid = threadIdx.x;  // 0..255
+    const int ctid = threadIdx.x;  // 0 .. TS::kCons - 1
     constexpr int kSlot = TS::BM * TS::BN;
     const int64_t tile_end = it - sg.kb + q.iters_per_tile;
     // An owner without the whole tile is in its last segment. It adds the

@@ -24,7 +24,7 @@ namespace skg {
 // device's host_mu like its staging buffers; at most 8 MB a direction) and
 // freed by host_slots_release (skgemm_stream_release of the default stream).
 struct HostSlots {
-    // Threads 4 / 6 / 8 / 12 with 1 MB slots: 57 MB up in 2.1 / 2.3 / 2.5 / 3.2 ms
+  // Threads 4 / 6 / 8 / 12 with 1 MB slots: 57 MB up in 2.1 / 2.3 / 2.5 / 3.2 ms
   // (512 KB slots 3.0 ms with 8, 2 MB 2.6 ms).
   static constexpr int kMaxThreads = 4;
   static constexpr size_t kSlotBytes = 1 << 20;

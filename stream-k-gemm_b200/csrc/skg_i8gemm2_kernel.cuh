@@ -27,9 +27,10 @@
 // Barriers: full[s] (rank 0: one arrival with the byte count of both CTAs'
 // loads), empty[s] and tfull[a] (each CTA: one arrival from rank 0's
 // multicast commit), tempty[a] (rank 0: one arrival per epilogue warp of
-// both CTAs; the peer's arrive remotely). Every wait is bounded; on expiry a
+// both CTAs; the peer's arrive remotely). Every mbarrier wait is bounded; on expiry a
 // CTA records the timeout and stops issuing work, the peer's waits then run
-// out as well, and both CTAs meet at the final cluster barrier.
+// out as well, and both CTAs meet at the final cluster barriers. The pair's TMEM
+// allocation and its release have no bound: both stand between cluster barriers.
 #pragma once
 
 #include "skg_i8gemm_kernel.cuh"

@@ -6,7 +6,9 @@
 // overflow.
 //
 // Operands are per-modulus residue matrices, K-major bytes:
-//   A_res[l][RA][KP], B_res[l][RB][KP]   (row r, k contiguous; zero padding)
+//   A_res[l][RA][KP], B_res[l][RB][KP]   (row r, k contiguous; zero past K;
+//   rows past the operand's last 16-row group hold anything, and only reach outputs
+//   that are not read)
 // loaded by TMA boxes {128 B of k, 128 (A) / 256 (B) rows, 1 modulus} with the
 // 128-byte swizzle, which is the canonical K-major SW128 UMMA layout.
 //

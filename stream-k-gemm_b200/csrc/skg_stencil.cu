@@ -50,9 +50,10 @@ struct StencilCoef {
 // bounded; on expiry the CTA records the error and skips the remaining waits.
 //
 // Bound by the shared-memory pipe, 89% busy: 20 16-byte loads per column and
-// band pair, and the stage itself is written through it. TMA moves one box row per 1.3 cycles whatever its length, so the
-// 32-byte rows of a 4-band slab on 16 x 16 columns took 297 us without any
-// arithmetic against 225 us for these 64-byte rows (400 us and 351 us in all).
+// band pair, and the stage itself is written through it. TMA moves one box row per
+// 1.3 cycles whatever its length, so the 32-byte rows of a 4-band slab on 16 x 16
+// columns took 297 us without any arithmetic against 225 us for these 64-byte rows
+// (400 us and 351 us in all).
 // Whole launches, one CTA per tile with its queues loaded at its start, 4-band
 // slabs -> this: 48^3 x 512 400 -> 351 us, 33 x 35 x 41 x 512 362 -> 243 us,
 // 56^3 x 318 475 -> 394 us, 48^3 x 72 86 -> 60 us, 24^3 x 24 31 -> 15 us.
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
 #pragma unroll
       for (int u = 0; u < kZq; ++u) {
         if (kb + u >= k1) break;
-          if (!*abort_flag && !mbar_wait(&full[buf], ph, err, kDevErrStencil)) *abort_flag = 1;
+        if (!*abort_flag && !mbar_wait(&full[buf], ph, err, kDevErrStencil)) *abort_flag = 1;
         const double* st = stages + buf * kStStage;
         const double2* P = reinterpret_cast<const double2*>(st);
         const double2* C = reinterpret_cast<const double2*>(st + kStPlane);
@@ -303,9 +304,11 @@ __global__ void __launch_bounds__(kStThreads, 1) stencil_staged_kernel(
 // stand before the first store (a 48-point row with its halo at once), and the
 // stores stream past L2. One 256-thread CTA per row, a load and a store at a time
 // -> this: 48^3 x 506 229 -> 199 us (6.7 TB/s, a plain copy's rate), 24^3 x 512
-// 64 -> 42 us, 48^3 x 72 40 -> 35 us. 4 loads in 8 warps: 204, 42 and 36 us; 8
-// loads took 260 us (48^3 rows end in a nearly empty second round); without the
-// streaming hint 234 us.
+// 64 -> 42 us, 48^3 x 72 40 -> 35 us, 33 x 35 x 41 x 512 130 -> 101 us. Longer rows
+// take a second round: 49^3 x 480 232 -> 200 us, 56^3 x 318 211 -> 189 us, 80^3 x 112
+// 197 -> 185 us; rounds of equal length are slower (207, 193 and 188 us). 4 loads in
+// 8 warps: 204, 42 and 36 us; 8 loads took 260 us on 48^3; without the streaming hint
+// 234 us.
 constexpr int kHaloLoads = 15;
 constexpr int kHaloWarps = 4;
 __global__ void __launch_bounds__(kHaloWarps * 32) halo_periodic_kernel(
