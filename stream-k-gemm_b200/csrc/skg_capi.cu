@@ -50,7 +50,8 @@ int debug_poison(void* p, size_t bytes, cudaStream_t s) {
   return SKGEMM_OK;
 }
 
-int table_stream(cudaStream_t* s) {
+// The current device's stream for table uploads (created on first use).
+static int table_stream(cudaStream_t* s) {
   static std::mutex mu;
   static cudaStream_t streams[64] = {};
   int d = 0;

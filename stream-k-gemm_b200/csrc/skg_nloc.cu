@@ -24,6 +24,7 @@
 //    scatter-adds keep the reference's order.
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -219,24 +220,6 @@ __global__ void __launch_bounds__(kNlocThreads) nloc_forward_kernel(
   }
 }
 
-// The caller's chi (each projector's columns one after the other, in_off) into the
-// device layout; CTA = a span of kNlocSpan row tiles of a projector.
-__global__ void __launch_bounds__(128) nloc_chi_layout_kernel(
-    const int64_t* __restrict__ tile_proj, const int64_t* __restrict__ tile_r0,
-    const uint32_t* __restrict__ nrow, const uint32_t* __restrict__ ncol,
-    const int64_t* __restrict__ in_off, const int64_t* __restrict__ chi_off,
-    const double* __restrict__ in, double* __restrict__ chi, int span) {
-  const int p = (int)tile_proj[blockIdx.x];
-  const int64_t nr = nrow[p], r1 = min(nr, tile_r0[blockIdx.x] + span);
-  const int nc = (int)ncol[p];
-  for (int64_t r = tile_r0[blockIdx.x] + threadIdx.x; r < r1; r += blockDim.x)
-    for (int j = 0; j < (nc + 1) / 2 * 2; ++j) {
-      const int k0 = j / kNlocCols * kNlocCols;
-      chi[chi_off[p] + k0 * nr + r * group_pitch(nc, k0) + (j - k0)] =
-          j < nc ? in[in_off[p] + j * nr + r] : 0.0;
-    }
-}
-
 // Back-projection, step 1: temp_p[r, b] = sum_k chi_p[r, k] C_p[k, b] (fused,
 // k ascending: the reference's gemm_ab order) for every projector row, into
 // temp[(row_off_p + r) * nb + b]. CTA = (a span of up to kNlocSpan row tiles
@@ -385,33 +368,41 @@ int upload(T** dst, const std::vector<T>& v) {
   return upload_table(*dst, v.data(), v.size() * sizeof(T));
 }
 
-// chi (n doubles, projector p's columns from in_off[p]) into d_chi (total doubles) in
-// the kernels' layout: uploaded as it is and laid out on the device.
-int upload_chi(skgemm_nloc* h, const double* chi, int64_t n, int64_t total,
-               const std::vector<int64_t>& in_off) {
-  if (h->ntiles == 0) return SKGEMM_OK;
-  DeviceBuffer in, off;
-  auto lay_out = [&]() -> int {
-    int st;
-    cudaStream_t s = nullptr;
-    if ((st = in.ensure((size_t)n * sizeof(double))) ||
-        (st = off.ensure(in_off.size() * sizeof(int64_t))))
-      return st;
-    SKG_CUDA(cudaMalloc(&h->d_chi, (size_t)total * sizeof(double)));
-    if ((st = upload_table(off.ptr, in_off.data(), in_off.size() * sizeof(int64_t))) ||
-        (st = upload_table(in.ptr, chi, (size_t)n * sizeof(double))) || (st = table_stream(&s)))
-      return st;
-    nloc_chi_layout_kernel<<<(unsigned)h->ntiles, 128, 0, s>>>(
-        h->d_tile_proj, h->d_tile_r0, h->d_nrow, h->d_ncol, (const int64_t*)off.ptr, h->d_chi_off,
-        (const double*)in.ptr, h->d_chi, kNlocTileR * kNlocSpan);
-    SKG_CUDA(cudaGetLastError());
-    SKG_CUDA(cudaStreamSynchronize(s));
-    return SKGEMM_OK;
-  };
-  const int st = lay_out();
-  in.release();
-  off.release();
-  return st;
+// chi (projector p's columns one after the other from in_off[p]) into d_chi (total
+// doubles) in the kernels' layout, row by row: the reads are as many streams as the
+// group has columns, the writes one.
+int upload_chi(skgemm_nloc* h, const double* chi, const uint32_t* nrow, const uint32_t* ncol,
+               const std::vector<int64_t>& in_off, int64_t total) {
+  if (total == 0) return SKGEMM_OK;
+  std::unique_ptr<double[]> buf(new double[total]);
+  double* out = buf.get();
+  for (int64_t p = 0; p < (int64_t)in_off.size(); ++p) {
+    const int64_t nr = nrow[p];
+    const int nc = (int)ncol[p];
+    for (int k0 = 0; k0 < nc; k0 += kNlocCols) {
+      const int w = std::min(kNlocCols, nc - k0), pitch = group_pitch(nc, k0);
+      const double* in = chi + in_off[p] + k0 * nr;
+      for (int64_t r = 0; r < nr; ++r, out += pitch) {
+        for (int j = 0; j < w; ++j) out[j] = in[j * nr + r];
+        if (w < pitch) out[w] = 0.0;
+      }
+    }
+  }
+  SKG_CUDA(cudaMalloc(&h->d_chi, (size_t)total * sizeof(double)));
+  return upload_table(h->d_chi, buf.get(), (size_t)total * sizeof(double));
+}
+
+// Sorts `rows` (ascending) by their index, rows of one index in their order: two stable
+// passes over 16 bits. A map of lists took most of a creation's time.
+void sort_by_index(const uint32_t* index, std::vector<int64_t>& rows) {
+  std::vector<int64_t> other(rows.size());
+  for (int shift = 0; shift < 32; shift += 16) {
+    std::vector<int64_t> at(65537, 0);
+    for (int64_t r : rows) ++at[((index[r] >> shift) & 0xFFFFu) + 1];
+    for (int v = 0; v < 65536; ++v) at[v + 1] += at[v];
+    for (int64_t r : rows) other[at[(index[r] >> shift) & 0xFFFFu]++] = r;
+    rows.swap(other);
+  }
 }
 
 void release(skgemm_nloc* h) {
@@ -502,12 +493,12 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
       bscale[blk_of[offsets[p]]].push_back(gam_off[p]);
     }
   }
-  // Inverse index: grid point -> (projector, row) in projector order.
-  std::map<uint32_t, std::vector<std::pair<int32_t, uint32_t>>> inv;
-  for (int64_t p = 0; p < P; ++p) {
-    if (nrow[p] == 0 || ncol[p] == 0) continue;
-    for (uint32_t r = 0; r < nrow[p]; ++r) inv[index[row_off[p] + r]].push_back({(int32_t)p, r});
-  }
+  // Inverse index: grid point -> its rows (of all projectors, in projector order).
+  std::vector<int64_t> ent_off;
+  ent_off.reserve(rows);
+  for (int64_t p = 0; p < P; ++p)
+    for (int64_t r = 0; ncol[p] > 0 && r < nrow[p]; ++r) ent_off.push_back(row_off[p] + r);
+  sort_by_index(index, ent_off);
   auto* h = new skgemm_nloc();
   h->device = dev->device;
   h->P = P;
@@ -529,13 +520,13 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
     blk_end[2 * q + 1] = (int64_t)blk_scale.size();
   }
   std::vector<uint32_t> touch;
-  std::vector<int64_t> touch_off{0};
-  std::vector<int64_t> ent_off;
-  for (const auto& kv : inv) {
-    touch.push_back(kv.first);
-    for (const auto& e : kv.second) ent_off.push_back(row_off[e.first] + e.second);
-    touch_off.push_back((int64_t)ent_off.size());
-  }
+  std::vector<int64_t> touch_off;
+  for (size_t e = 0; e < ent_off.size(); ++e)
+    if (e == 0 || index[ent_off[e]] != touch.back()) {
+      touch.push_back(index[ent_off[e]]);
+      touch_off.push_back((int64_t)e);
+    }
+  touch_off.push_back((int64_t)ent_off.size());
   h->ntouch = (int64_t)touch.size();
   h->total_rows = rows;
   std::vector<int64_t> tile_proj, tile_r0;
@@ -559,7 +550,7 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
       (st = upload(&h->d_touch, touch)) || (st = upload(&h->d_touch_off, touch_off)) ||
       (st = upload(&h->d_ent_off, ent_off)) ||
       (st = upload(&h->d_tile_proj, tile_proj)) || (st = upload(&h->d_tile_r0, tile_r0)) ||
-      (st = upload_chi(h, chi, chi_in, chis, in_off))) {
+      (st = upload_chi(h, chi, nrow, ncol, in_off, chis))) {
     release(h);
     delete h;
     return st;

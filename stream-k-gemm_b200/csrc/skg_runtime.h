@@ -54,8 +54,6 @@ int debug_poison(void* p, size_t bytes, cudaStream_t s);
 // not wait for.
 int upload_table(void* dst, const void* src, size_t bytes);
 int fill_table(void* dst, int byte, size_t bytes);
-// The current device's stream that they use (created on first use).
-int table_stream(cudaStream_t* s);
 
 struct DeviceBuffer {
   void* ptr = nullptr;
