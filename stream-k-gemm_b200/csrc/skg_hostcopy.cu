@@ -77,7 +77,6 @@ void HostCopy::add(int g, void* dst, size_t dpitch, const void* src, size_t spit
 }
 
 int HostCopy::start(bool gated) {
-  started_ = true;
   if (!gated) opened_ = (int)left_.size();
   const void* host = nullptr;
   if (!whole_.empty()) host = kind_ == cudaMemcpyHostToDevice ? whole_[0].src : whole_[0].dst;
@@ -89,12 +88,8 @@ int HostCopy::start(bool gated) {
     cudaGetLastError();  // or the next launch's check would report it
     staged_ = false;
   }
-  if (!staged_) {
-    int st = SKGEMM_OK;
-    if (!gated)
-      for (int g = 0; g < (int)left_.size() && !st; ++g) st = direct(g);
-    return st;
-  }
+  gated_ = gated;
+  if (!staged_) return SKGEMM_OK;
   try {
     // Pieces of a slot; smaller ones where a thread would get fewer than four, so that
     // no thread is left waiting for another's last piece.
@@ -121,22 +116,20 @@ int HostCopy::start(bool gated) {
     pieces_.clear();
     std::fill(left_.begin(), left_.end(), 0);
     staged_ = false;
-    int st = SKGEMM_OK;
-    if (!gated)
-      for (int g = 0; g < (int)left_.size() && !st; ++g) st = direct(g);
-    return st;
   }
   return SKGEMM_OK;
 }
 
 int HostCopy::direct(int g) {
-  for (const Piece& p : whole_)
-    if (p.group == g) {
-      if (p.height == 1)
-        SKG_CUDA(cudaMemcpyAsync(p.dst, p.src, p.width, kind_, s_));
-      else
-        SKG_CUDA(cudaMemcpy2DAsync(p.dst, p.dpitch, p.src, p.spitch, p.width, p.height, kind_, s_));
-    }
+  for (; next_direct_ <= g; ++next_direct_)
+    for (const Piece& p : whole_)
+      if (p.group == next_direct_) {
+        if (p.height == 1)
+          SKG_CUDA(cudaMemcpyAsync(p.dst, p.src, p.width, kind_, s_));
+        else
+          SKG_CUDA(
+              cudaMemcpy2DAsync(p.dst, p.dpitch, p.src, p.spitch, p.width, p.height, kind_, s_));
+      }
   return SKGEMM_OK;
 }
 
@@ -160,14 +153,14 @@ void HostCopy::fail_with(cudaError_t e) {
 }
 
 int HostCopy::wait_group(int g) {
-  if (!staged_) return SKGEMM_OK;
+  if (!staged_) return direct(g);
   std::unique_lock<std::mutex> lk(mu_);
   cv_.wait(lk, [&] { return left_[g] == 0 || stop_; });
   return err_ == cudaSuccess ? SKGEMM_OK : cuda_fail(err_, "host copy");
 }
 
 int HostCopy::finish() {
-  if (!staged_) return SKGEMM_OK;
+  if (!staged_) return gated_ ? SKGEMM_OK : direct((int)left_.size() - 1);
   for (std::thread& t : threads_) t.join();
   threads_.clear();
   return err_ == cudaSuccess ? SKGEMM_OK : cuda_fail(err_, "host copy");

@@ -51,7 +51,9 @@ class HostCopy {
   int start(bool gated = false);
   // The group's pieces may be enqueued from here on.
   int open(int g);
-  // H2D: returns when every piece of group g is enqueued on the stream.
+  // H2D: returns when every piece of group g is enqueued on the stream. Where the
+  // driver copies, only then: an event recorded next marks this group, not the later
+  // ones too.
   int wait_group(int g);
   // Every piece is enqueued (H2D) or in host memory (D2H).
   int finish();
@@ -66,7 +68,7 @@ class HostCopy {
   };
   void work(int w);
   void fail_with(cudaError_t e);
-  int direct(int g);
+  int direct(int g);  // enqueues the groups up to g that are not yet
 
   DeviceState* dev_;
   cudaMemcpyKind kind_;
@@ -78,8 +80,9 @@ class HostCopy {
   std::mutex mu_;
   std::condition_variable cv_;
   std::atomic<size_t> next_{0};
-  int opened_ = 0;  // groups below may run
-  bool staged_ = false, stop_ = false, started_ = false;
+  int opened_ = 0;       // groups below may run
+  int next_direct_ = 0;  // first group the driver has not been given
+  bool staged_ = false, stop_ = false, gated_ = false;
   cudaError_t err_ = cudaSuccess;
   size_t bytes_ = 0;
 };

@@ -14,12 +14,12 @@
 
 static std::atomic<int> g_copies{0}, g_late{0};
 static std::atomic<bool> g_waited{false};
-static bool g_no_pinned = false;
+static bool g_no_pinned = false, g_registered = false;
 static cudaError_t g_last = cudaSuccess;
 
 extern "C" {
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
-  a->type = cudaMemoryTypeUnregistered;
+  a->type = g_registered ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
@@ -62,6 +62,7 @@ int main(int argc, char** argv) {
   using namespace skg;
   const bool failing = argc > 1 && !strcmp(argv[1], "fail");
   g_no_pinned = argc > 1 && !strcmp(argv[1], "unpinned");
+  g_registered = argc > 1 && !strcmp(argv[1], "pinned");
   const int chunks = 8;
   const size_t n = 4 << 20;
   std::vector<char> src(chunks * n), dst(chunks * n);
@@ -75,6 +76,7 @@ int main(int argc, char** argv) {
   st = up.start();
   for (int c = 0; c < chunks && !st; ++c) {
     st = up.wait_group(c);
+    if ((g_registered || g_no_pinned) && g_copies != c + 1) st = SKGEMM_ERR_CUDA;  // later chunks' too
     if (failing && c == 1) st = SKGEMM_ERR_OOM;  // the chunk's launch failed
   }
   const int got = hp.finish(st);

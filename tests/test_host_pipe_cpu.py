@@ -24,13 +24,13 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("mode", ["fail", "ok", "unpinned"])
+@pytest.mark.parametrize("mode", ["fail", "ok", "unpinned", "pinned"])
 def test_no_copy_outlives_the_call(exe, mode):
     r = subprocess.run([exe, mode], capture_output=True, text=True, timeout=60, check=True)
     st, seen, late, after, whole, left = map(int, r.stdout.split())
     assert late == 0 and after == 0
     assert left == 0  # slots that cannot be pinned: the driver copies, nothing else changes
-    if mode != "fail":
+    if mode != "fail":  # pinned, unpinned: the driver copies, one chunk ahead of its event
         assert st == skgemm.OK and whole == 1 and seen >= 8
     else:
         assert st == skgemm.ERR_OOM and 0 < seen < 32
