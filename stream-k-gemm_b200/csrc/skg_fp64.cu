@@ -294,21 +294,13 @@ int grouped_setup(int device, int* blocks_per_sm) {
   return SKGEMM_OK;
 }
 
-// Whether a tile of the group can be in kSharedParts parts: its first and last part
-// and kSharedParts - 2 whole CTA ranges between them.
-bool group_spread(const Fp64Group& g) {
-  return g.max_tile_iters >= (kSharedParts - 2) * (g.total_iters / g.grid) + 2;
-}
-
 template <class TS>
 int grouped_launch(const Fp64Group& g, cudaStream_t s) {
   // Flags start at zero for every launch (a stream-ordered memset, captured
   // together with the kernel when the pair is recorded into a graph).
   SKG_CUDA(cudaMemsetAsync(g.flags, 0, (size_t)fixup_slots(g.grid, 1) * sizeof(uint32_t), s));
-  if (!group_spread(g)) {
+  if (!fp64_group_spread(g)) {
     // Only owners wait, for CTAs that never do: any number of CTAs may be resident.
-    // Without the shared fix-up the loop is 3% faster (the compiler's schedule):
-    // serving's launches of 25 problems 27.7 -> 28.4 TFLOP/s.
     fp64_grouped_kernel<TS, false><<<g.grid, TS::kThreads, TS::kSmem, s>>>(g);
     SKG_CUDA(cudaGetLastError());
     return SKGEMM_OK;
@@ -331,6 +323,17 @@ int grouped_launch(const Fp64Group& g, cudaStream_t s) {
 }
 
 }  // namespace
+
+// The shared fix-up needs a tile that can be in kSharedParts parts: its first and last
+// part and kSharedParts - 2 whole CTA ranges of q iterations between them. Its code
+// slows the loop of all tiles by 3% (the compiler's schedule; serving's launches of 25
+// problems 28.2 -> 27.7 TFLOP/s without such tiles), 0.03 (64 x 64 tiles) or 0.06 us an
+// iteration, and takes the owner 1.1 or 3 us a part off the longest tile: it pays from
+// about q / 40 parts.
+bool fp64_group_spread(const Fp64Group& g) {
+  const int64_t q = std::max<int64_t>(1, g.total_iters / g.grid);
+  return g.max_tile_iters >= (kSharedParts - 2) * q + 2 && 40 * (g.max_tile_iters / q) >= q;
+}
 
 int fp64_group_occupancy(DeviceState* dev, int tile, int* blocks_per_sm) {
   if (tile == 128) return grouped_setup<Tile128>(dev->device, blocks_per_sm);

@@ -144,6 +144,8 @@ struct SingleSched {
   __device__ __forceinline__ uint32_t* err() const { return p.err; }
   __device__ __forceinline__ uint32_t pub() const { return p.epoch; }
   __device__ __forceinline__ bool spread() const { return p.spread != 0; }
+  static constexpr bool kOwnersOnly = false;
+  __device__ __forceinline__ int64_t cta_begin(int c) const { return p.split.begin(c); }
 };
 
 // A group of problems: descriptors and tensor maps in global memory.
@@ -173,6 +175,14 @@ struct GroupSched {
   __device__ __forceinline__ uint32_t* err() const { return g.err; }
   __device__ __forceinline__ uint32_t pub() const { return 1u; }
   __device__ __forceinline__ bool spread() const { return SPREAD; }
+  // Without the shared fix-up the ranges are divided in 64 bits, and a tile's end is
+  // found where it is needed: the compiler's schedule of the whole loop follows (16
+  // sets of three problems 1198 -> 1170 us, rotations 4 x 65536 x 32 and 2 x 65536 x
+  // 256 792 -> 774).
+  static constexpr bool kOwnersOnly = !SPREAD;
+  __device__ __forceinline__ int64_t cta_begin(int c) const {
+    return kOwnersOnly ? (int64_t)c * g.total_iters / g.grid : g.split.begin(c);
+  }
 };
 
 // Where iteration `it` (< it_end) falls: problem, tile, k-block range of this
@@ -356,8 +366,8 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
   }
   __syncthreads();
 
-  const int64_t it_begin = S.split().begin(cta);
-  const int64_t it_end = S.split().begin(cta + 1);
+  const int64_t it_begin = S.cta_begin(cta);
+  const int64_t it_end = S.cta_begin(cta + 1);
 
   if (warp == TS::kWarps) {
     // ------------------------------------------------------------ producer
@@ -455,8 +465,10 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     // Three iterations a trip (half the ring), so that the loop's own work
     // spreads over 48 k: GEMM 512 x 512 x 110592 1.670 -> 1.617 ms, SYRK 0.933
     // -> 0.921, rotation 110592 x 512 1.710 -> 1.680 (two, four, six a trip:
-    // 1.617, 1.617, 1.616 / 0.930, 0.923, 0.923 / 1.685, 1.680, 1.681).
-#pragma unroll 3
+    // 1.617, 1.617, 1.616 / 0.930, 0.923, 0.923 / 1.685, 1.680, 1.681). Two in
+    // groups of 64 x 64 tiles without long ones, many of them rotations of few
+    // iterations: 16 sets of three problems 1170 -> 1140 us, their rotations 420 -> 408.
+#pragma unroll (Sched::kOwnersOnly && TS::BM == 64 ? 2 : 3)
     for (int k = sg.kb; k < sg.ke && !aborted; ++k) {
       if (!mbar_wait(&full_bar[stage], phase, S.err(), kDevErrFp64)) {
         aborted = true;
@@ -526,11 +538,15 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
     const bool complete = owner && (sg.ke == q.iters_per_tile);
     const int ctid = threadIdx.x;  // 0 .. TS::kCons - 1
     constexpr int kSlot = TS::BM * TS::BN;
-    const int64_t tile_end = it - sg.kb + q.iters_per_tile;
+    auto tile_end_of = [&]() -> int64_t {
+      if constexpr (Sched::kOwnersOnly)
+        return S.begin(sg.pid) + (int64_t)(sg.tile + 1) * q.iters_per_tile;
+      return it - sg.kb + q.iters_per_tile;
+    };
     // An owner without the whole tile is in its last segment. It adds the
     // other parts itself if they are few.
     const bool shared = owner && !complete && S.spread() && cta + kSharedParts <= S.split().grid &&
-                        S.split().begin(cta + kSharedParts - 1) < tile_end;
+                        S.cta_begin(cta + kSharedParts - 1) < tile_end_of();
     if (!owner || shared) {
       // Publish this CTA's partial tile (layout [reg][thread], coalesced).
       const int slot_id = owner ? S.split().grid + cta : cta;
@@ -553,8 +569,9 @@ __device__ __forceinline__ void streamk_body(const Sched& S) {
         // in ascending k order. A flag that does not arrive within the budget
         // is recorded in the error word and its partial is skipped; the CTA
         // keeps consuming its pipeline so no copy is left in flight.
+        const int64_t tile_end = tile_end_of();
         for (int c2 = cta + 1; c2 < S.split().grid; ++c2) {
-          if (S.split().begin(c2) >= tile_end) break;
+          if (S.cta_begin(c2) >= tile_end) break;
           if (ctid == 0)
             fixup_ok = fixup_flag_wait(S.flags() + c2, pubval, S.err(), kFixupBudgetNs) ? 1 : 0;
           asm volatile("bar.sync 1, %0;" ::"n"(TS::kCons));

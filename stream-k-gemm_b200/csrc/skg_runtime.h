@@ -143,6 +143,8 @@ int fp64_preload(DeviceState* dev);
 struct Fp64Group;
 int fp64_group_occupancy(DeviceState* dev, int tile, int* blocks_per_sm);
 int launch_fp64_group(int tile, const Fp64Group& g, cudaStream_t s);
+// Whether the launch of `g` finishes tiles by several CTAs (two slots and flags a CTA).
+bool fp64_group_spread(const Fp64Group& g);
 // TMA descriptor of one operand for tiles of `rows_per_tile` rows.
 int make_operand_map(CUtensorMap* map, const Fp64Operand& op, int64_t K, int rows_per_tile);
 
