@@ -334,12 +334,12 @@ int configure(BatchPlan* P, Config c) {
     if ((st = P->d_probs.ensure(hp.size() * sizeof(Fp64Params)))) return st;
     if ((st = P->d_maps.ensure(hm.size() * sizeof(CUtensorMap)))) return st;
     if ((st = P->d_iters.ensure(hb.size() * sizeof(int64_t)))) return st;
-    const size_t slots = (size_t)fixup_slots(grid, 1);
+    const size_t slots = (size_t)fixup_slots(grid, fp64_group_spread(G) ? 1 : 0);
     if ((st = P->d_part.ensure(slots * BM * BN * sizeof(double)))) return st;
-    if ((st = P->d_flags.ensure(slots * sizeof(uint32_t)))) return st;
-    if ((st = upload_table(P->d_probs.ptr, hp.data(), hp.size() * sizeof(Fp64Params))) ||
-        (st = upload_table(P->d_maps.ptr, hm.data(), hm.size() * sizeof(CUtensorMap))) ||
-        (st = upload_table(P->d_iters.ptr, hb.data(), hb.size() * sizeof(int64_t))))
+    if ((st = P->d_flags.ensure((size_t)fixup_slots(grid, 1) * sizeof(uint32_t)))) return st;
+    if ((st = upload_tables({{P->d_probs.ptr, hp.data(), hp.size() * sizeof(Fp64Params)},
+                             {P->d_maps.ptr, hm.data(), hm.size() * sizeof(CUtensorMap)},
+                             {P->d_iters.ptr, hb.data(), hb.size() * sizeof(int64_t)}})))
       return st;
   }
   if (!P->d_err.ptr) {

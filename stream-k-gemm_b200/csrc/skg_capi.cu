@@ -63,12 +63,20 @@ static int table_stream(cudaStream_t* s) {
   return SKGEMM_OK;
 }
 
-int upload_table(void* dst, const void* src, size_t bytes) {
+int upload_tables(const std::vector<TableCopy>& copies) {
   cudaStream_t s = nullptr;
   if (int st = table_stream(&s)) return st;
-  SKG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
-  SKG_CUDA(cudaStreamSynchronize(s));
-  return SKGEMM_OK;
+  cudaError_t e = cudaSuccess;
+  for (const TableCopy& c : copies)
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, s);
+  // Also after a failure: the sources may be gone when this returns.
+  const cudaError_t w = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = w;
+  return e == cudaSuccess ? SKGEMM_OK : cuda_fail(e, "table upload");
+}
+
+int upload_table(void* dst, const void* src, size_t bytes) {
+  return upload_tables({{dst, src, bytes}});
 }
 
 int fill_table(void* dst, int byte, size_t bytes) {

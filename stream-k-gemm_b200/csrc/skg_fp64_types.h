@@ -142,7 +142,7 @@ struct Fp64Group {
   int grid;
   int max_tile_iters;  // the longest tile's iterations
   IterSplit split;    // make_split(total_iters, grid)
-  double* workspace;  // 2 * grid slots of BM*BN doubles (shared fix-up)
+  double* workspace;  // grid slots of BM*BN doubles, 2 * grid with the shared fix-up
   uint32_t* flags;    // 2 * grid flags, zero at launch
   uint32_t* err;
 };

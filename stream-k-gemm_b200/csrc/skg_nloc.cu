@@ -361,19 +361,20 @@ __global__ void __launch_bounds__(256) nloc_backward_kernel(
   if (two) o[1] = v1;
 }
 
+// Allocates *dst for v and adds its upload to `copies`.
 template <typename T>
-int upload(T** dst, const std::vector<T>& v) {
+int stage(T** dst, const std::vector<T>& v, std::vector<TableCopy>& copies) {
   if (v.empty()) return SKGEMM_OK;
   SKG_CUDA(cudaMalloc(dst, v.size() * sizeof(T)));
-  return upload_table(*dst, v.data(), v.size() * sizeof(T));
+  copies.push_back({*dst, v.data(), v.size() * sizeof(T)});
+  return SKGEMM_OK;
 }
 
-// chi (projector p's columns one after the other from in_off[p]) into d_chi (total
-// doubles) in the kernels' layout, row by row: the reads are as many streams as the
-// group has columns, the writes one.
+// Uploads `copies` and chi (projector p's columns one after the other from in_off[p])
+// into d_chi (total doubles) in the kernels' layout, row by row: the reads are as many
+// streams as the group has columns, the writes one.
 int upload_chi(skgemm_nloc* h, const double* chi, const uint32_t* nrow, const uint32_t* ncol,
-               const std::vector<int64_t>& in_off, int64_t total) {
-  if (total == 0) return SKGEMM_OK;
+               const std::vector<int64_t>& in_off, int64_t total, std::vector<TableCopy>& copies) {
   std::unique_ptr<double[]> buf(new double[total]);
   double* out = buf.get();
   for (int64_t p = 0; p < (int64_t)in_off.size(); ++p) {
@@ -388,8 +389,11 @@ int upload_chi(skgemm_nloc* h, const double* chi, const uint32_t* nrow, const ui
       }
     }
   }
-  SKG_CUDA(cudaMalloc(&h->d_chi, (size_t)total * sizeof(double)));
-  return upload_table(h->d_chi, buf.get(), (size_t)total * sizeof(double));
+  if (total > 0) {
+    SKG_CUDA(cudaMalloc(&h->d_chi, (size_t)total * sizeof(double)));
+    copies.push_back({h->d_chi, buf.get(), (size_t)total * sizeof(double)});
+  }
+  return upload_tables(copies);
 }
 
 // Sorts `rows` (ascending) by their index, rows of one index in their order: two stable
@@ -541,16 +545,24 @@ int nloc_create(int64_t P, const uint32_t* nrow, const uint32_t* ncol, const int
   std::vector<uint32_t> vnrow(nrow, nrow + P), vncol(ncol, ncol + P);
   std::vector<uint32_t> vindex(index, index + rows);
   std::vector<double> vgam(gamma, gamma + gams);
-  if ((st = upload(&h->d_nrow, vnrow)) || (st = upload(&h->d_ncol, vncol)) ||
-      (st = upload(&h->d_index, vindex)) || (st = upload(&h->d_row_off, row_off)) ||
-      (st = upload(&h->d_chi_off, chi_off)) || 
-      (st = upload(&h->d_gamma, vgam)) || (st = upload(&h->d_blk, blk)) ||
-      (st = upload(&h->d_blk_end, blk_end)) || (st = upload(&h->d_blk_proj, blk_proj)) ||
-      (st = upload(&h->d_blk_scale, blk_scale)) || (st = upload(&h->d_proj_blk_col, proj_col)) ||
-      (st = upload(&h->d_touch, touch)) || (st = upload(&h->d_touch_off, touch_off)) ||
-      (st = upload(&h->d_ent_off, ent_off)) ||
-      (st = upload(&h->d_tile_proj, tile_proj)) || (st = upload(&h->d_tile_r0, tile_r0)) ||
-      (st = upload_chi(h, chi, nrow, ncol, in_off, chis))) {
+  std::vector<TableCopy> up;
+  if ((st = stage(&h->d_nrow, vnrow, up)) ||
+      (st = stage(&h->d_ncol, vncol, up)) ||
+      (st = stage(&h->d_index, vindex, up)) ||
+      (st = stage(&h->d_row_off, row_off, up)) ||
+      (st = stage(&h->d_chi_off, chi_off, up)) ||
+      (st = stage(&h->d_gamma, vgam, up)) ||
+      (st = stage(&h->d_blk, blk, up)) ||
+      (st = stage(&h->d_blk_end, blk_end, up)) ||
+      (st = stage(&h->d_blk_proj, blk_proj, up)) ||
+      (st = stage(&h->d_blk_scale, blk_scale, up)) ||
+      (st = stage(&h->d_proj_blk_col, proj_col, up)) ||
+      (st = stage(&h->d_touch, touch, up)) ||
+      (st = stage(&h->d_touch_off, touch_off, up)) ||
+      (st = stage(&h->d_ent_off, ent_off, up)) ||
+      (st = stage(&h->d_tile_proj, tile_proj, up)) ||
+      (st = stage(&h->d_tile_r0, tile_r0, up)) ||
+      (st = upload_chi(h, chi, nrow, ncol, in_off, chis, up))) {
     release(h);
     delete h;
     return st;

@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -53,6 +54,12 @@ int debug_poison(void* p, size_t bytes, cudaStream_t s);
 // cudaMemset does; both run on the default stream, which non-blocking streams do
 // not wait for.
 int upload_table(void* dst, const void* src, size_t bytes);
+struct TableCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+int upload_tables(const std::vector<TableCopy>& copies);  // several, one wait
 int fill_table(void* dst, int byte, size_t bytes);
 
 struct DeviceBuffer {
