@@ -418,7 +418,7 @@ int launch_stencil_ext(int64_t ni, int64_t nj, int64_t nk, int64_t nb, int FDn,
   const int64_t work = cols * ((nb + kSlab - 1) / kSlab);
   if (work > INT32_MAX) return fail(SKGEMM_ERR_INVALID_ARG, "grid too large");
   // A CTA per tile at least, where tiles have fewer planes than that (6^3 x 512: 12.8
-  // -> 11 us).
+  // -> 12.2 us).
   const int grid = (int)std::min<int64_t>(num_sms, std::max<int64_t>(work, work * nk / kStMinSteps));
   if (out_tile == 32)
     return launch_staged<32>(mapP, mapC, mapF, (int)ni, (int)nj, (int)nk, (int)nb, (int)work, grid, A,
