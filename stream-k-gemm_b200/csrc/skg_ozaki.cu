@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
   // and the loads stream one contiguous span.
   const int64_t gw = (int64_t)blockIdx.x * kConvWarps + warp, nw = (int64_t)gridDim.x * kConvWarps;
   if (gw >= ntiles) return;
-  const int64_t nmine = (ntiles - gw + nw - 1) / nw;  // tiles of this warp
+  int64_t nmine = (ntiles - gw + nw - 1) / nw;  // tiles of this warp
   const int64_t dq = nw / KB, dr = nw % KB;           // stride nw as (groups, k-blocks)
   if (lane == 0) {
     for (int st = 0; st < kConvStages; ++st) mbar_init(&bar[st], 1);
@@ -488,24 +488,20 @@ __global__ void __launch_bounds__(256, 2) convert_tma_kernel(
       pow2_pair(mu[g * 16 + r], s1, s2);
       cur_g = g;
     }
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], (phase >> s) & 1u, err, kDevErrConvert))) {
-      // A lost load: the warp stops at its first wait that runs out, stores nothing
-      // more and leaves when the loads behind it have landed.
-      for (int j = 1; j < kConvStages && n + j < nmine; ++j) {
-        const int sj = (s + j) % kConvStages;
-        mbar_wait(&bar[sj], (phase >> sj) & 1u, err, kDevErrConvert);
-      }
-      return;
-    }
+    const bool ok = mbar_wait(&bar[s], (phase >> s) & 1u, err, kDevErrConvert);
     phase ^= 1u << s;
     constexpr int ES = BF ? 2 : 1;  // bytes per residue
     uint8_t* dst = res + ((g * 16 + r) * KP + kb * 32 + 16 * h) * ES;
     const int64_t lstride = Rpad * KP * ES;
-    if (BF) {
+    if (ok && BF) {
       uint8_t* row = res + ((g * 16 + r) * KP + kb * 32) * 2;
       convert_stage_bf16<L, KM>(buf + s * kConvTile, r, h, s1, s2, row, lstride);
-    } else {
+    } else if (ok) {
       convert_stage_i8<L, KM>(buf + s * kConvTile, r, h, s1, s2, dst, lstride);
+    } else {
+      // A lost load: no tile is issued after those in flight, which the loop still
+      // waits for, and the warp leaves (a vote and a return cost the loop 1%).
+      nmine = n + kConvStages < nmine ? n + kConvStages : nmine;
     }
     __syncwarp();  // stage s consumed by every lane before it is refilled
     s = (s + 1) % kConvStages;
