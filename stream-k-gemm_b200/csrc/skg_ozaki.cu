@@ -1741,9 +1741,6 @@ struct OzakiNeed {
     partials = std::max(partials, o.partials);
     rbytes = std::max(rbytes, o.rbytes);
   }
-  size_t total() const {
-    return res_a + res_b + part_a + part_b + mu_a + mu_b + partials + rbytes;
-  }
 };
 
 // Norm partials of any operand of at most R rows: ceil(R'/T) panels of C chunks, C =
