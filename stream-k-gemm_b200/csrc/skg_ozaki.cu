@@ -1698,8 +1698,8 @@ int subspace_impl(int64_t K, int64_t M, const double* Psi, const double* HPsi, d
     SKG_CUDA(cudaEventCreateWithFlags(&os->fork2, cudaEventDisableTiming));
     SKG_CUDA(cudaEventCreateWithFlags(&os->join2, cudaEventDisableTiming));
   }
-  // Two streams (none of these kernels waits on another CTA, so they may
-  // share the machine in any proportion):
+  // Two streams (these kernels wait on no CTA but the other one of a pair, so they
+  // may share the machine in any proportion):
   //   s:   norms(Psi) -> convert(Psi) -- wait(join) -> products(S, Hs) -> CRT(Hs)
   //   aux: norms(HPsi) -> convert(HPsi) -> [join] -- wait(fork2) -> CRT(S) -> [join2]
   // HPsi's norm pass and conversion overlap Psi's; one INT8 launch computes

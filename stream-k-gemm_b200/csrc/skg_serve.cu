@@ -11,7 +11,7 @@
 // each other, so their CTAs never wait on CTAs that cannot become resident;
 // input generation and layout conversion overlap them on a second stream.
 // The Ozaki path runs each admitted request's whole sequence on one of a few
-// slot streams (its kernels have no inter-CTA waits), with the slots'
+// slot streams (its kernels wait on no CTA but a pair's other one), with the slots'
 // scratch reserved up front for the largest request of the trace.
 //
 // Memory: request data lives in one device arena of the admission budget
